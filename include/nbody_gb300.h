@@ -85,7 +85,9 @@ NBGB_API size_t nbgb_force_workspace_bytes(size_t N);
  * every fourth source pair's m r^-3 as 2^(log2 m - 1.5 log2 r^2), which needs
  * m >= 0.  A negative (or NaN) mass gives NaN forces and sets
  * NBGB_STATUS_NEGATIVE_MASS; for signed masses force an rsqrt-only
- * configuration through nbgb_force_ex.
+ * configuration through nbgb_force_ex.  Larger N (nbgb_force_kind) evaluate
+ * each pair once instead, with the same rule for the masses.  Results are
+ * deterministic in both forms.
  */
 NBGB_API int nbgb_force(float *force, const float *posMass, float softeningSquared, size_t N,
                         void *workspace, size_t workspace_bytes, void *stream);
@@ -103,9 +105,10 @@ NBGB_API int nbgb_force_ex(float *force, const float *posMass, float softeningSq
 /*
  * Newton's-third-law variant (the reference's unregistered tiled kernels,
  * src/nbody_GPU_AOS_tiled.cu:93-179, compute each pair once too): each pair
- * is evaluated once and applied to both bodies; per-block-pair sums are
- * accumulated in FP64 and rounded to FP32 at the end.  Same arguments and
- * conventions as nbgb_force; workspace >= nbgb_force_newton3_workspace_bytes.
+ * is evaluated once and applied to both bodies, at every N and for masses of
+ * any sign; partial sums are added in a fixed order (deterministic).  Same
+ * arguments and conventions as nbgb_force; workspace >=
+ * nbgb_force_newton3_workspace_bytes.
  */
 /*
  * Replaces: one GPU's share of the reference's multi-GPU algorithm
@@ -127,8 +130,13 @@ NBGB_API size_t nbgb_force_newton3_workspace_bytes(size_t N);
 NBGB_API int nbgb_force_newton3(float *force, const float *posMass, float softeningSquared,
                                 size_t N, void *workspace, size_t workspace_bytes, void *stream);
 
-/* The planner's decision for N (config forced when >= 0, nsplit as for
-   nbgb_force_ex). */
+/* How nbgb_force evaluates N bodies on the current device: *pairs (may be
+   NULL) 1 when it evaluates each pair once rather than run the one-sided plan
+   below, *launches (may be NULL) the kernels one call launches. */
+NBGB_API int nbgb_force_kind(size_t N, int *pairs, int *launches);
+/* The one-sided kernel's plan for N (config forced when >= 0, nsplit as for
+   nbgb_force_ex); the workspace is what nbgb_force_ex needs for the same
+   arguments. */
 NBGB_API int nbgb_force_plan(size_t N, int config, int nsplit, int *out_config, int *out_nsplit,
                              size_t *out_workspace_bytes);
 /* The same decision without a GPU, for a device with `sms` SMs and
@@ -223,24 +231,26 @@ NBGB_API int nbgb_system_set_state64(nbgb_system *sys, const double *pos3, const
                                      const float *mass);
 /* Advance nsteps (asynchronous; whole groups of 8 steps replay a captured
    CUDA graph, the rest launch directly).  Reference integrators with the
-   one-sided kernel: each step is one launch (the force kernel integrates
-   each body in its epilogue).  KDK: each step is one kick+drift launch and
-   one force launch; the call's closing half kick is applied when the
+   default force: the force pass's last kernel integrates each body once its
+   force is final (one launch a step with the one-sided kernel, two or more
+   when pairs are evaluated once).  KDK: each step is one kick+drift launch and
+   one force pass; the call's closing half kick is applied when the
    velocities are next read (getters, diagnostics) or merged into the next
    call's opening kick. */
 NBGB_API int nbgb_system_step(nbgb_system *sys, int nsteps);
 /* KDK: apply a pending closing half kick now (asynchronous). */
 NBGB_API int nbgb_system_sync_velocities(nbgb_system *sys);
 NBGB_API int nbgb_system_set_graph(nbgb_system *sys, int enable);
-/* 0: one-sided force kernel (default); 1: Newton's-third-law variant. */
+/* 0: nbgb_force's choice for N (default); 1: the Newton's-third-law variant
+   at every N, with the integrate as its own launch. */
 NBGB_API int nbgb_system_set_force_algorithm(nbgb_system *sys, int algorithm);
 /* Bracket every force launch and every integrate launch with CUDA events on
    the system's stream (steps then run eagerly); nbgb_system_last_force_ms
    reads the latest force launch, nbgb_system_last_integrate_ms the latest
    integrate launches: step_ms the reference integrate or the FP64
    kick+drift, half_kick_ms the closing FP64 half kick (0 if none ran).  With
-   a reference integrator and the one-sided kernel the integrate runs inside
-   the force launch (its epilogue), so the force time covers both and
+   a reference integrator and the default force the integrate runs inside the
+   force pass (its last kernel's epilogue), so the force time covers both and
    nbgb_system_last_integrate_ms has nothing to report (-1). */
 NBGB_API int nbgb_system_set_timing(nbgb_system *sys, int enable);
 NBGB_API int nbgb_system_last_force_ms(nbgb_system *sys, float *ms);
@@ -261,8 +271,8 @@ NBGB_API void *nbgb_system_device_posmass(nbgb_system *sys);
 NBGB_API void *nbgb_system_device_force(nbgb_system *sys);
 NBGB_API void *nbgb_system_stream(nbgb_system *sys);
 NBGB_API int nbgb_system_plan(nbgb_system *sys, int *config, int *nsplit);
-/* Force the one-sided kernel's plan (config / nsplit as for nbgb_force_ex;
-   -1, -1 restores the planner's choice).  For tuning and tests; the
+/* Force the one-sided kernel and its plan (config / nsplit as for
+   nbgb_force_ex; -1, -1 restores nbgb_force's choice for N).  For tuning and tests; the
    potential configuration is refused, log-domain configurations need
    masses >= 0.  Synchronises the system's stream. */
 NBGB_API int nbgb_system_set_plan(nbgb_system *sys, int config, int nsplit);

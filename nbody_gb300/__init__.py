@@ -97,12 +97,21 @@ def release_workspace() -> None:
 # Stream-ordered force
 # ---------------------------------------------------------------------------
 def force_plan(N: int, config: int = -1, nsplit: int = -1):
-    """(configuration, slice count, workspace bytes) of the plan nbgb_force
-    runs for N (config / nsplit as for force())."""
+    """(configuration, slice count, workspace bytes) of the one-sided plan
+    for N (config / nsplit as for force()); force_kind tells whether force()
+    runs it unforced."""
     c, s, w = ctypes.c_int(), ctypes.c_int(), ctypes.c_size_t()
     check(load().nbgb_force_plan(N, config, nsplit, ctypes.byref(c), ctypes.byref(s),
                                  ctypes.byref(w)), "nbgb_force_plan")
     return c.value, s.value, w.value
+
+
+def force_kind(N: int):
+    """("pairs" or "onesided", kernel launches) of force() for N bodies:
+    whether it evaluates each pair once or runs the one-sided plan."""
+    p, k = ctypes.c_int(), ctypes.c_int()
+    check(load().nbgb_force_kind(N, ctypes.byref(p), ctypes.byref(k)), "nbgb_force_kind")
+    return ("pairs" if p.value else "onesided"), k.value
 
 
 def force_plan_on(N: int, sms: int, occupancy, config: int = -1, nsplit: int = -1):
@@ -154,7 +163,8 @@ def force(posMass, softeningSquared: float, out=None, stream=None, workspace: Wo
           config: int = -1, nsplit: int = -1):
     """F_i = sum_j m_j d_ij / (|d_ij|^2 + eps2)^1.5 for a (N,4) float32 CUDA
     tensor {x,y,z,m}; returns (N,4) {fx,fy,fz,0}.  config / nsplit force a
-    plan (-1: the planner's choice; nsplit > 0 splits every i-block's
+    one-sided plan (-1, -1: the library's choice, which evaluates each pair
+    once at larger N; -1: the planner's choice; nsplit > 0 splits every i-block's
     sources nsplit ways, nsplit <= -2 only the i-blocks left over after
     whole rounds of CTA slots, -nsplit ways)."""
     torch = _torch()
@@ -256,8 +266,8 @@ def last_status() -> int:
 # ---------------------------------------------------------------------------
 class System:
     """State resident in HBM; step() = force + integrate per step (reference
-    integrators on the one-sided kernel: one launch, the integrate in the
-    force kernel's epilogue; groups of 8 steps replay a CUDA graph), no host
+    integrators with the default force: the integrate runs in the force
+    pass's last kernel; groups of 8 steps replay a CUDA graph), no host
     round trip."""
 
     def __init__(self, N: int, integrator: int = INTEGRATOR_REFERENCE,
@@ -300,7 +310,8 @@ class System:
         check(self.lib.nbgb_system_set_graph(self.h, int(enable)), "set_graph")
 
     def set_force_algorithm(self, name: str):
-        """'onesided' (default) or 'newton3'."""
+        """'onesided' (default: force()'s choice for N) or 'newton3' (each
+        pair once at every N)."""
         code = {"onesided": 0, "newton3": 1}[name]
         check(self.lib.nbgb_system_set_force_algorithm(self.h, code), "set_force_algorithm")
 
@@ -354,8 +365,8 @@ class System:
                 "momentum": out[2:5].copy(), "angular_momentum": out[5:8].copy()}
 
     def set_plan(self, config: int = -1, nsplit: int = -1):
-        """Force the one-sided kernel's plan (as for force(); -1, -1: the
-        planner's choice)."""
+        """Force the one-sided kernel and its plan (as for force(); -1, -1:
+        force()'s choice)."""
         check(self.lib.nbgb_system_set_plan(self.h, config, nsplit), "set_plan")
 
     def plan(self):

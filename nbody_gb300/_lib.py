@@ -29,6 +29,8 @@ SIGNATURES = {
     "nbgb_force": (ctypes.c_int, [c_vp, c_vp, ctypes.c_float, c_size, c_vp, c_size, c_vp]),
     "nbgb_force_ex": (ctypes.c_int, [c_vp, c_vp, ctypes.c_float, c_size, c_vp, c_size,
                                      ctypes.c_int, ctypes.c_int, c_vp]),
+    "nbgb_force_kind": (ctypes.c_int, [c_size, ctypes.POINTER(ctypes.c_int),
+                                       ctypes.POINTER(ctypes.c_int)]),
     "nbgb_force_newton3_workspace_bytes": (c_size, [c_size]),
     "nbgb_force_newton3": (ctypes.c_int, [c_vp, c_vp, ctypes.c_float, c_size, c_vp, c_size,
                                           c_vp]),

@@ -12,7 +12,7 @@ are the reference driver's own initial conditions (randomUnitBodies, scale
 0.9, velocity scale 8, src/nbody.cu:996), N = --bodies x 1024, softening 0.1
 (eps2 0.01), timestep 0.016, damping 0.95 (src/nbody.cu:151-156) unless
 overridden.  Two algorithm rows run the device-resident step loop:
-GPU_GB300 (the one-sided force kernel) and GPU_GB300_Newton3 (each pair
+GPU_GB300 (the default force) and GPU_GB300_Newton3 (each pair
 once); --cycle-after moves to the next row every N steps and an iteration
 is one pass through the rows, as in the reference (src/nbody.cu:1055-1068).
 The printed milliseconds are the force launch's CUDA-event time, as the

@@ -52,6 +52,7 @@
 #include <vector>
 
 #include "nbgb_device.cuh"
+#include "nbgb_integrate.cuh"
 #include "nbgb_internal.h"
 #include "nbody_gb300.h"
 
@@ -88,49 +89,6 @@ __global__ void pack_jstream_kernel(const float4 *__restrict__ pm, float4 *__res
         counters[i] = 0u;
     const float4 b = (i < n) ? pm[i] : make_float4(0.f, 0.f, 0.f, 0.f);
     store_jstream_body(js, vpb, logm, i, b, i < npad);
-}
-
-// The reference integrator (integrateOne, src/nbody.cu:158-182) applied to
-// target i by the unit that produced its final force F: v += (F invMass) dt;
-// v *= damping; x += v dt, each operation rounded separately or, fused drift,
-// x = fma(v, dt, x) -- the same arithmetic as integrate_reference_kernel, so
-// the results are identical.  Writes posMass (mass kept), velInvMass and body
-// i's entry of the next step's j-stream (fi.js, the other buffer: the current
-// one is still being read by other units).  Only the last unit of an
-// i-block writes its targets, after every unit of that i-block has loaded
-// them, so no unit reads a target this launch has moved.
-__device__ __forceinline__ void fused_integrate(const FusedIntegrate &fi, int i, float x, float y,
-                                                float z, float m, float fx, float fy, float fz) {
-    float4 v = fi.vel[i];
-    const float im = v.w, dt = fi.dt;
-    v.x = __fmul_rn(__fadd_rn(v.x, __fmul_rn(__fmul_rn(fx, im), dt)), fi.damping);
-    v.y = __fmul_rn(__fadd_rn(v.y, __fmul_rn(__fmul_rn(fy, im), dt)), fi.damping);
-    v.z = __fmul_rn(__fadd_rn(v.z, __fmul_rn(__fmul_rn(fz, im), dt)), fi.damping);
-    if (fi.fused_drift) {
-        x = __fmaf_rn(v.x, dt, x);
-        y = __fmaf_rn(v.y, dt, y);
-        z = __fmaf_rn(v.z, dt, z);
-    } else {
-        x = __fadd_rn(x, __fmul_rn(v.x, dt));
-        y = __fadd_rn(y, __fmul_rn(v.y, dt));
-        z = __fadd_rn(z, __fmul_rn(v.z, dt));
-    }
-    fi.pm[i] = make_float4(x, y, z, m);
-    fi.vel[i] = v;
-    const int q = i >> 1, h = i & 1;
-    float w = m;
-    if (fi.js_log && jstream_log_slot(q))
-        w = jstream_log_mass(w);
-    if (fi.js_vpb == 2) {
-        fi.js[2 * i] = make_float4(x, x, y, y);
-        fi.js[2 * i + 1] = make_float4(z, z, w, w);
-    } else {
-        float *a = reinterpret_cast<float *>(fi.js + 2 * q);
-        a[h] = x;
-        a[2 + h] = y;
-        a[4 + h] = z;
-        a[6 + h] = w;
-    }
 }
 
 // ---------------------------------------------------------------------------
@@ -655,6 +613,7 @@ static_assert(sizeof(kConfigs) / sizeof(kConfigs[0]) <= (size_t)kMaxConfigs,
 struct DeviceInfo {
     int sms = 0;
     int occ[kMaxConfigs] = {0};
+    unsigned *status = nullptr;  // this translation unit's device status word
     bool ok = false;
     unsigned long long ctx = 0;
 };
@@ -689,6 +648,10 @@ static const DeviceInfo *device_info() {
             return nullptr;
         d.occ[c] = occ;
     }
+    void *status = nullptr;
+    if (pair_prepare() != NBGB_OK || cudaGetSymbolAddress(&status, g_status) != cudaSuccess)
+        return nullptr;
+    d.status = (unsigned *)status;
     d.ok = true;
     return &d;
 }
@@ -887,6 +850,27 @@ static int plan_force_among(size_t n, const std::vector<int> &cands, int force_n
         [](const ForcePlan &) { return true; }, d);
 }
 
+// Evaluate pairs once (force_pair.cu) from kMinPairForce bodies on: 14-16
+// FP32 operations for two interactions against 23.  Microseconds a call,
+// pairs against the one-sided plan (back to back in a graph, GB300, uniform
+// ball): N = 4,096 16 / 15, 6,000 24 / 23, 8,192 31 / 37, 10,007 40 / 53,
+// 16,384 85 / 110, 131,072 4,415 / 5,820; equal masses (Plummer) 100,003
+// 2,390 / 3,480, 131,072 4,065 / 5,820, 2^20 253,200 / 369,100.  Below the line the one-sided kernel's finer split wins; above
+// kMaxPairForce a phase's pieces (12 N bytes a row) take too much workspace.
+// Results of pair plans are closer to 64 bits at every size (3.7e-8 against
+// 8.5e-8 at 100,003).  A plan that would take log-domain pairs refuses
+// negative masses as that plan does.
+static void use_pair_plan(ForcePlan &pl, const DeviceInfo *d, size_t max_bytes = 0) {
+    if (!d)
+        d = device_info();
+    if (!d || pl.n < kMinPairForce || pl.n > kMaxPairForce ||
+        !plan_pair(pl.n, d->sms, max_bytes, pl.pair))
+        return;
+    pl.use_pair = 1;
+    pl.pair.status = pl.js_log ? d->status : nullptr;
+    pl.workspace_bytes = std::max(pl.workspace_bytes, pl.pair.workspace_bytes);
+}
+
 static int plan_force_on(size_t n, int force_config, int force_nsplit, ForcePlan &pl,
                          const DeviceInfo *d) {
     if (n == 0 || n > kMaxBodies)
@@ -899,7 +883,10 @@ static int plan_force_on(size_t n, int force_config, int force_nsplit, ForcePlan
     } else {
         cands.assign(std::begin(kDefaultCandidates), std::end(kDefaultCandidates));
     }
-    return plan_force_among(n, cands, force_nsplit, pl, 0, d);
+    const int rc = plan_force_among(n, cands, force_nsplit, pl, 0, d);
+    if (rc == NBGB_OK && force_config < 0 && force_nsplit == -1)
+        use_pair_plan(pl, d);
+    return rc;
 }
 
 int plan_force(size_t n, int force_config, int force_nsplit, ForcePlan &pl) {
@@ -909,6 +896,8 @@ int plan_force(size_t n, int force_config, int force_nsplit, ForcePlan &pl) {
 int plan_force_rows(size_t n, size_t rows, ForcePlan &pl) {
     if (n == 0 || n > kMaxBodies || rows == 0 || rows > n)
         return NBGB_ERR_INVALID_ARGUMENT;
+    if (rows == n)  // the whole force
+        return plan_force(n, -1, -1, pl);
     return plan_force_among(n,
                             std::vector<int>(std::begin(kDefaultCandidates),
                                              std::end(kDefaultCandidates)),
@@ -918,9 +907,12 @@ int plan_force_rows(size_t n, size_t rows, ForcePlan &pl) {
 int plan_force_rsqrt(size_t n, ForcePlan &pl) {
     if (n == 0 || n > kMaxBodies)
         return NBGB_ERR_INVALID_ARGUMENT;
-    return plan_force_among(n, std::vector<int>(std::begin(kRsqrtCandidates),
-                                                std::end(kRsqrtCandidates)),
-                            -1, pl);
+    const int rc = plan_force_among(n, std::vector<int>(std::begin(kRsqrtCandidates),
+                                                        std::end(kRsqrtCandidates)),
+                                    -1, pl);
+    if (rc == NBGB_OK)
+        use_pair_plan(pl, nullptr);
+    return rc;
 }
 
 // The best plan (same cost model as plan_force) whose workspace fits in
@@ -932,11 +924,15 @@ int plan_force_within(size_t n, size_t max_bytes, ForcePlan &pl) {
     const int rc = plan_enumerate(
         n, 0, kDefaultCandidates, (int)(sizeof(kDefaultCandidates) / sizeof(int)), -1, pl,
         [max_bytes](const ForcePlan &c) { return c.workspace_bytes <= max_bytes; });
+    if (rc == NBGB_OK)
+        use_pair_plan(pl, nullptr, max_bytes);
     return rc == NBGB_ERR_UNSUPPORTED ? NBGB_ERR_TOO_LARGE : rc;
 }
 
 int launch_force(const ForcePlan &pl, float4 *force, const float4 *posMass, const float4 *jstream,
                  float eps2, void *workspace, cudaStream_t stream, const FusedIntegrate *fi) {
+    if (pl.use_pair)
+        return launch_pair(pl.pair, force, posMass, eps2, workspace, stream, fi);
     const ForceConfig &cf = kConfigs[pl.config];
     char *ws = (char *)workspace;
     ForceParams p;
@@ -971,6 +967,8 @@ int launch_force(const ForcePlan &pl, float4 *force, const float4 *posMass, cons
 
 int launch_pack(const ForcePlan &pl, const float4 *posMass, void *workspace, cudaStream_t stream,
                 float4 *js_out) {
+    if (pl.use_pair)
+        return NBGB_OK;  // reads posMass
     char *ws = (char *)workspace;
     float4 *js = js_out ? js_out : (float4 *)(ws + pl.off_js);
     unsigned *cnt = (!js_out && split_blocks(pl)) ? (unsigned *)(ws + pl.off_cnt) : nullptr;
@@ -1144,6 +1142,20 @@ NBGB_API int nbgb_force_plan(size_t N, int config, int nsplit, int *out_config, 
         *out_nsplit = pl.nsplit;
     if (out_workspace_bytes)
         *out_workspace_bytes = pl.workspace_bytes;
+    return NBGB_OK;
+}
+
+// How nbgb_force evaluates N bodies on the current device: *pairs 1 when it
+// evaluates each pair once, *launches the kernels of one call.
+NBGB_API int nbgb_force_kind(size_t N, int *pairs, int *launches) {
+    ForcePlan pl;
+    int rc = plan_force(N, -1, -1, pl);
+    if (rc != NBGB_OK)
+        return rc;
+    if (pairs)
+        *pairs = pl.use_pair;
+    if (launches)
+        *launches = pl.use_pair ? pair_launches(pl.pair) : 2;
     return NBGB_OK;
 }
 

@@ -1,0 +1,718 @@
+// force_pair.cu -- the all-pairs force with every pair of bodies evaluated
+// once and applied to both (Newton's third law), deterministic: no atomics,
+// every partial sum is written once and added in a fixed order.
+//
+// What bounds it: the FP32 (FMA) pipe and the registers that feed it.  A pair
+// costs 16 packed FP32 operations for two interactions (14 when the masses
+// involved are equal), against 11.5-12 for each interaction of the one-sided
+// kernel.  ncu: FMA pipe 82 % busy; the rest are dispatch stalls of
+// three-operand instructions (six of the 16) and the other instructions' issue.
+// GB300, N = 131,072: 4,415 us with mixed masses (3.89e12 interactions/s),
+// 4,065 us with equal ones (4.23e12), against 4,830 us for 8 sources and 8
+// targets a lane with all source registers shuffled and FP64 atomics, and
+// 5,820 us one-sided.
+//
+// Work.  Targets are taken in rows of kRow bodies (one CTA: W warps x 32
+// lanes x KI bodies held in registers), sources in sets of kSet = 64 NC
+// bodies.  Row b meets its own sets one-sided (every ordered pair, the self
+// pair contributing 0) and every later set both ways.  A warp meets a set in
+// 32 steps: at step t lane L evaluates its KI targets against the NC source
+// pairs (L + t) & 31 (f32x2: two sources an instruction), whose reaction sums
+// then move to the next lane by shuffle; positions and masses are not
+// shuffled but read from shared memory (two 128-bit loads instead of eight
+// shuffles a source pair; each set is stored twice in a row, so lane L + t
+// needs no wrap).  Every instruction beside the FMA-pipe ones costs about as
+// much issue time as one of them, so the tile is as wide in targets as the
+// registers allow (12 targets a lane 4,400 / 4,120 us, 11 4,415 / 4,065, 10
+// 4,515 / 4,040, 8 4,550 / 4,005 at N = 131,072, mixed / equal masses; 3 warps
+// a scheduler with 8 targets were 2 % slower than 2 with 12).  The next set
+// comes by cp.async, which holds no registers.
+//
+// Split.  The steps of all (row, set) meetings form one line, and the host
+// cuts it into equal stretches of cost, one per resident CTA: one wave without
+// a tail at every N.  A stretch may begin and end inside a set or a row.
+// Pieces: the reactions of one stretch's part of one (row, set) meeting
+// (kSet x 3 floats, slot = meeting index + CTA index) and the targets' sums
+// of its part of one row (kRow x 3 floats, slot = row + CTA index); both
+// numberings grow strictly along the line, so no two pieces share a slot.
+// The reduce kernel adds each body's pieces in a fixed order with compensated
+// FP32 sums and writes the force (and integrates, when asked).  Both kernels
+// are launched with programmatic dependence: their CTAs start as the previous
+// kernel's leave and wait for it only before they touch its results.
+//
+// Phases.  The reaction pieces of all rows take N^2/(2 kRow) x 12 B; rows are
+// processed in as many phases as the workspace needs.  Bodies of the rows
+// done are final after their phase and no later phase reads them; the sums
+// of later bodies are carried over in the workspace.
+//
+// Ranges.  (|d|^2 + eps2)^-3/2 alone leaves the binary32 range beyond
+// distances of 2^42 although m times it may not.  Warps whose targets and set
+// lie within 2^40 of the origin (eps2 within 2^+-80) take the short forms;
+// others multiply by the mass first, as the one-sided kernel does.
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <cmath>
+#include <cstdint>
+
+#include "nbgb_device.cuh"
+#include "nbgb_integrate.cuh"
+#include "nbgb_internal.h"
+#include "nbody_gb300.h"
+
+namespace nbgb {
+namespace pair {
+
+template <int W_, int KI_, int NC_, int CTAS_>
+struct Geo {
+    static constexpr int W = W_, KI = KI_, NC = NC_;
+    static constexpr int kThreads = 32 * W;
+    static constexpr int kCtas = CTAS_;           // resident CTAs per SM
+    static constexpr int kRow = 32 * W * KI;      // targets per row
+    static constexpr int kSet = 64 * NC;          // sources per set
+    static constexpr int kRowSets = kRow / kSet;
+    static_assert(kRow % kSet == 0, "a row is whole sets");
+    // steps between folds of the targets' sums: 256 sources
+    static constexpr int kFoldSteps = 128 / NC;
+    static constexpr int kHop = 16;  // steps a reaction travels between adds
+    // dynamic shared memory: hi/lo sums, reactions of two pieces, two
+    // sets in pairs, the next set as it comes from memory
+    static constexpr int kHl = 6 * KI * kThreads;             // floats
+    static constexpr int kRed = 2 * W * 3 * kSet;             // floats
+    static constexpr int kSrc = 2 * (2 * NC) * 64 * 4;        // floats
+    static constexpr int kRaw = kSet * 4;                     // floats
+    static constexpr size_t kSmem = (size_t)(kHl + kRed + kSrc + kRaw) * 4;
+};
+typedef Geo<4, 11, 2, 2> G;
+
+constexpr float kRange = 1.0995116e12f;  // 2^40
+
+enum : int { kFar = 1, kMixed = 2 };  // set flags: out of range, masses differ
+
+struct Params {
+    const float4 *__restrict__ pm;
+    float *__restrict__ react;  // [slot][3][kSet]
+    float *__restrict__ tsum;   // [slot][3][kRow]
+    int n, nsets, row0, row1;   // rows of this phase
+    float eps2;
+    int short_ok;               // eps2 in the short forms' range
+    unsigned *__restrict__ status;  // not null: refuse masses < 0
+    int ncta;
+    unsigned step[kMaxPairCtas + 1];  // first step of each CTA's stretch
+};
+
+// (row, set) meetings of the rows before b, counted from row 0.
+__host__ __device__ inline long long meetings_before(int b, int nsets) {
+    return (long long)b * nsets - (long long)G::kRowSets * b * (b - 1) / 2;
+}
+
+enum : int { kEqual = 0, kShort = 1, kWide = 2, kOneSided = 3 };
+
+// Steps t0 .. t1-1 of one meeting.  src: this lane's first source pair; rw:
+// the warp's reaction sums [3][kSet] (overwritten), times rs.  The travelling
+// reactions are added to them every kHop steps: chains of kHop KI terms
+// instead of 32 KI, so that they are no longer than the targets' chains.
+template <int MODE>
+__device__ __forceinline__ void
+meet(const ulonglong2 *src, int t0, int t1, const f2 (&nx)[G::KI], const f2 (&ny)[G::KI],
+     const f2 (&nz)[G::KI], const f2 (&nm)[G::KI], f2 (&ax)[G::KI], f2 (&ay)[G::KI],
+     f2 (&az)[G::KI], f2 eps2p, int lane, float *rw, float rs) {
+    constexpr int KI = G::KI, NC = G::NC;
+    const int from = (lane + 1) & 31;
+    f2 sx[NC], sy[NC], sz[NC], sm[NC];
+    src += t0;
+#pragma unroll
+    for (int c = 0; c < NC; c++) {
+        const ulonglong2 a = src[128 * c], b = src[128 * c + 64];
+        sx[c] = a.x;
+        sy[c] = a.y;
+        sz[c] = b.x;
+        sm[c] = b.y;
+    }
+#pragma unroll 1
+    for (int ta = t0; ta < t1; ta += G::kHop) {
+        const int tb = min(ta + G::kHop, t1);
+        f2 rx[NC], ry[NC], rz[NC];
+#pragma unroll
+        for (int c = 0; c < NC; c++)
+            rx[c] = ry[c] = rz[c] = 0;
+#pragma unroll 2
+        for (int t = ta; t < tb; t++) {
+            src++;
+#pragma unroll
+            for (int c = 0; c < NC; c++) {
+#pragma unroll
+                for (int k = 0; k < KI; k++) {
+                    const f2 dx = f2_add(sx[c], nx[k]);
+                    const f2 dy = f2_add(sy[c], ny[k]);
+                    const f2 dz = f2_add(sz[c], nz[k]);
+                    f2 d2 = f2_fma(dx, dx, eps2p);
+                    d2 = f2_fma(dy, dy, d2);
+                    d2 = f2_fma(dz, dz, d2);
+                    float l, h;
+                    f2_unpack(d2, l, h);
+                    const f2 inv = f2_pack(rsqrt_mufu(l), rsqrt_mufu(h));
+                    const f2 inv2 = f2_mul(inv, inv);
+                    f2 wi, wj;
+                    if constexpr (MODE == kEqual) {
+                        wi = wj = f2_mul(inv, inv2);
+                    } else if constexpr (MODE == kShort) {
+                        const f2 s = f2_mul(inv, inv2);
+                        wi = f2_mul(sm[c], s);
+                        wj = f2_mul(nm[k], s);
+                    } else {
+                        wi = f2_mul(f2_mul(sm[c], inv), inv2);
+                        if constexpr (MODE == kWide)
+                            wj = f2_mul(f2_mul(nm[k], inv), inv2);
+                    }
+                    ax[k] = f2_fma(dx, wi, ax[k]);
+                    ay[k] = f2_fma(dy, wi, ay[k]);
+                    az[k] = f2_fma(dz, wi, az[k]);
+                    if constexpr (MODE != kOneSided) {
+                        rx[c] = f2_fma(dx, wj, rx[c]);
+                        ry[c] = f2_fma(dy, wj, ry[c]);
+                        rz[c] = f2_fma(dz, wj, rz[c]);
+                    }
+                }
+                const ulonglong2 a = src[128 * c], b = src[128 * c + 64];
+                sx[c] = a.x;
+                sy[c] = a.y;
+                sz[c] = b.x;
+                sm[c] = b.y;
+                if constexpr (MODE != kOneSided) {
+                    rx[c] = __shfl_sync(0xffffffffu, rx[c], from);
+                    ry[c] = __shfl_sync(0xffffffffu, ry[c], from);
+                    rz[c] = __shfl_sync(0xffffffffu, rz[c], from);
+                }
+            }
+        }
+        if constexpr (MODE != kOneSided) {
+#pragma unroll
+            for (int c = 0; c < NC; c++) {
+                const int p = 32 * c + ((lane + tb) & 31);
+                const f2 r[3] = {rx[c], ry[c], rz[c]};
+#pragma unroll
+                for (int q = 0; q < 3; q++) {
+                    float2 *d = reinterpret_cast<float2 *>(rw + q * G::kSet + 2 * p);
+                    float l, h;
+                    f2_unpack(r[q], l, h);
+                    float2 v = make_float2(l * rs, h * rs);
+                    if (ta > t0) {
+                        v.x += d->x;
+                        v.y += d->y;
+                    }
+                    *d = v;
+                }
+            }
+            __syncwarp();
+        }
+    }
+}
+
+__global__ void __launch_bounds__(G::kThreads, G::kCtas)
+    pair_kernel(const __grid_constant__ Params P) {
+    constexpr int KI = G::KI, NC = G::NC, NT = G::kThreads, kSet = G::kSet;
+    extern __shared__ __align__(128) float smem[];
+    float *src_buf = smem;                     // [2][2 NC][64] float4
+    float *red = smem + G::kSrc;               // [2][W][3][kSet]
+    float *hl = smem + G::kSrc + G::kRed;      // [6 KI][NT]
+    float4 *raw = reinterpret_cast<float4 *>(smem + G::kSrc + G::kRed + G::kHl);  // [kSet]
+    __shared__ int flags[2][G::W];
+    __shared__ float mass[2][G::W];            // a warp's (first) mass of each set
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int cta = blockIdx.x;
+    unsigned s = P.step[cta];
+    const unsigned s_end = P.step[cta + 1];
+    const long long g0 = meetings_before(P.row0, P.nsets);
+    int b;
+    {  // the row that holds meeting s / 32
+        const long long g = g0 + (s >> 5);
+        int lo = P.row0, hi = P.row1 - 1;
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (meetings_before(mid, P.nsets) <= g)
+                lo = mid;
+            else
+                hi = mid - 1;
+        }
+        b = lo;
+    }
+    const f2 eps2p = f2_pack(P.eps2, P.eps2);
+    const f2 zero2 = f2_pack(0.f, 0.f);
+    grid_dependents_launch();
+    grid_dependency_wait();
+
+    // a plan that refuses negative masses turns them into NaN, which every
+    // body's sum then meets
+    auto checked = [&](float4 v) {
+        if (P.status && !(v.w >= 0.f)) {
+            atomicOr(P.status, NBGB_STATUS_NEGATIVE_MASS);
+            v.w = __int_as_float(0x7fc00000);
+        }
+        return v;
+    };
+    // one set: kSet bodies in pairs {x0,x1,y0,y1}, {z0,z1,m0,m1}, each list
+    // stored twice in a row; the flags say which forms it allows.  The bodies
+    // come asynchronously (no registers held), each read by the thread that
+    // asked for it; bodies beyond n are zeros.
+    auto fetch = [&](int set) {
+        const int j = set * kSet + tid;
+        if (tid < kSet)
+            async_g2s_16(raw + tid, P.pm + (j < P.n ? j : 0), j < P.n ? 16u : 0u);
+    };
+    auto stage = [&](int buf) {
+        async_wait_all();
+        if (tid >= kSet)
+            return;
+        const float4 v = checked(raw[tid]);
+        const float m0 = __shfl_sync(0xffffffffu, v.w, 0);
+        const bool far = !(fabsf(v.x) < kRange && fabsf(v.y) < kRange && fabsf(v.z) < kRange);
+        const bool mixed = !(v.w == m0 && fabsf(m0) < 1e30f);
+        const int pr = tid >> 1, h = tid & 1, c = pr >> 5;
+        float *p = src_buf + ((size_t)(buf * 2 * NC + 2 * c) * 64 + (pr & 31)) * 4 + h;
+        p[0] = p[128] = v.x;
+        p[2] = p[130] = v.y;
+        p[256] = p[384] = v.z;
+        p[258] = p[386] = v.w;
+        const bool any_far = __any_sync(0xffffffffu, far);
+        const bool any_mixed = __any_sync(0xffffffffu, mixed);
+        if (lane == 0) {
+            flags[buf][warp] = (any_far ? kFar : 0) | (any_mixed ? kMixed : 0);
+            mass[buf][warp] = m0;
+        }
+    };
+    static_assert(kSet % 32 == 0, "whole warps stage");
+    static_assert(NT >= kSet, "one thread stages one source");
+
+    int buf = 0;
+    while (s < s_end) {
+        const long long gb = meetings_before(b, P.nsets) - g0;  // row b's first meeting
+        const int row_set = b * G::kRowSets;
+        const unsigned seg_end =
+            min(s_end, (unsigned)((gb + (P.nsets - row_set)) << 5));
+        f2 nx[KI], ny[KI], nz[KI], nm[KI], ax[KI], ay[KI], az[KI];
+        bool tfar = false, tmixed = false;
+        float tm0 = 0.f;
+#pragma unroll
+        for (int k = 0; k < KI; k++) {
+            const int i = b * G::kRow + warp * 32 * KI + lane + 32 * k;
+            const float4 v =
+                i < P.n ? checked(P.pm[i]) : make_float4(0.f, 0.f, 0.f, 0.f);
+            if (k == 0)
+                tm0 = __shfl_sync(0xffffffffu, v.w, 0);
+            tfar |= !(fabsf(v.x) < kRange && fabsf(v.y) < kRange && fabsf(v.z) < kRange);
+            tmixed |= !(v.w == tm0 && fabsf(tm0) < 1e30f);
+            nx[k] = f2_pack(-v.x, -v.x);
+            ny[k] = f2_pack(-v.y, -v.y);
+            nz[k] = f2_pack(-v.z, -v.z);
+            nm[k] = f2_pack(-v.w, -v.w);
+            ax[k] = ay[k] = az[k] = zero2;
+#pragma unroll
+            for (int c = 0; c < 6; c++)
+                hl[(6 * k + c) * NT + tid] = 0.f;
+        }
+        const bool short_ok = P.short_ok && !__any_sync(0xffffffffu, tfar);
+        const bool tequal = !__any_sync(0xffffffffu, tmixed);
+        int folded_steps = 0;
+        float scale = 1.f;
+        // the targets' sums since the last fold -> compensated sums
+        auto fold = [&]() {
+#pragma unroll
+            for (int k = 0; k < KI; k++) {
+                f2 *a[3] = {&ax[k], &ay[k], &az[k]};
+#pragma unroll
+                for (int c = 0; c < 3; c++) {
+                    float l, h;
+                    f2_unpack(*a[c], l, h);
+                    float hi = hl[(6 * k + c) * NT + tid], lo = hl[(6 * k + 3 + c) * NT + tid];
+                    comp_add(hi, lo, (l + h) * scale);
+                    hl[(6 * k + c) * NT + tid] = hi;
+                    hl[(6 * k + 3 + c) * NT + tid] = lo;
+                    *a[c] = zero2;
+                }
+            }
+            folded_steps = 0;
+        };
+
+        int set = row_set + (int)((s >> 5) - gb);
+        fetch(set);
+        stage(buf);
+        __syncthreads();
+        while (s < seg_end) {
+            const int t0 = (int)(s & 31u);
+            const int t1 = min(32, t0 + (int)(seg_end - s));
+            const unsigned s_next = s + (unsigned)(t1 - t0);
+            const bool more = s_next < seg_end;  // then t1 == 32
+            if (more)
+                fetch(set + 1);
+            const float sm0 = mass[buf][0];
+            int fl = 0;
+#pragma unroll
+            for (int w = 0; w < kSet / 32; w++)
+                fl |= flags[buf][w] | (mass[buf][w] == sm0 ? 0 : kMixed);
+            const bool one_sided = set < row_set + G::kRowSets;
+            const bool in_range = short_ok && !(fl & kFar);
+            const bool equal = in_range && tequal && !(fl & kMixed) && !one_sided;
+            const float new_scale = equal ? sm0 : 1.f;
+            if (new_scale != scale) {
+                if (folded_steps)
+                    fold();
+                scale = new_scale;
+            }
+            const ulonglong2 *src = reinterpret_cast<const ulonglong2 *>(src_buf) +
+                                    (size_t)buf * 2 * NC * 64 + lane;
+            float *rb = red + (size_t)(buf * G::W) * 3 * kSet;
+            float *rw = rb + (size_t)warp * 3 * kSet;
+            const float rs = equal ? -tm0 : 1.f;
+            if (equal)
+                meet<kEqual>(src, t0, t1, nx, ny, nz, nm, ax, ay, az, eps2p, lane, rw, rs);
+            else if (one_sided)
+                meet<kOneSided>(src, t0, t1, nx, ny, nz, nm, ax, ay, az, eps2p, lane, rw, rs);
+            else if (in_range)
+                meet<kShort>(src, t0, t1, nx, ny, nz, nm, ax, ay, az, eps2p, lane, rw, rs);
+            else
+                meet<kWide>(src, t0, t1, nx, ny, nz, nm, ax, ay, az, eps2p, lane, rw, rs);
+            folded_steps += t1 - t0;
+            if (folded_steps + 32 > G::kFoldSteps)
+                fold();
+            if (more)
+                stage(buf ^ 1);
+            __syncthreads();
+            if (!one_sided) {
+                float *out = P.react + ((size_t)(s >> 5) + cta) * 3 * kSet;
+#pragma unroll
+                for (int q = tid; q < 3 * kSet; q += NT) {
+                    float t = rb[q];
+#pragma unroll
+                    for (int w = 1; w < G::W; w++)
+                        t += rb[w * 3 * kSet + q];
+                    out[q] = t;
+                }
+            }
+            s = s_next;
+            set++;
+            buf ^= 1;
+        }
+        if (folded_steps)
+            fold();
+        float *out = P.tsum + ((size_t)(b - P.row0) + cta) * 3 * G::kRow;
+#pragma unroll
+        for (int k = 0; k < KI; k++)
+#pragma unroll
+            for (int c = 0; c < 3; c++)
+                out[c * G::kRow + warp * 32 * KI + lane + 32 * k] =
+                    hl[(6 * k + c) * NT + tid] + hl[(6 * k + 3 + c) * NT + tid];
+        b++;
+        // the next row's staging reuses buffers others may still be reading
+        __syncthreads();
+    }
+}
+
+struct ReduceParams {
+    Params p;
+    float *__restrict__ carry;  // [6][npad]: sums of bodies whose rows come later
+    size_t npad;
+    float4 *__restrict__ force;
+    FusedIntegrate fi;  // fi.vel == nullptr: forces only
+};
+
+// kReduceBodies bodies a block, kReduceGroups x 3 (components) threads a body:
+// the body's reaction pieces (one list for the block, from the phase's earlier
+// rows in row order) and then its row's target pieces form one sequence; each
+// group adds a contiguous part of it, eight loads in flight, and the parts
+// are added in order.  A latency problem, not a bandwidth one: at N = 16,384
+// there are about 35 pieces a body and 49,152 sums.
+constexpr int kReduceBodies = 32, kReduceGroups = 4;
+constexpr int kReduceThreads = 3 * kReduceBodies * kReduceGroups;
+
+__global__ void __launch_bounds__(kReduceThreads)
+    pair_reduce_kernel(const __grid_constant__ ReduceParams R) {
+    constexpr int kSet = G::kSet, kB = kReduceBodies, kPart = kSet / kB;
+    static_assert(kSet % kB == 0, "blocks are parts of a set");
+    __shared__ unsigned short first[kMaxPairRows], count[kMaxPairRows];
+    __shared__ int list[kMaxPairRows + kMaxPairCtas];
+    __shared__ int n_list;
+    __shared__ float part[kReduceGroups - 1][2][3][kB], out[3][kB];
+    const Params &P = R.p;
+    const int tid = threadIdx.x, group = tid / (3 * kB), comp = (tid / kB) % 3, j = tid % kB;
+    const int set = P.row0 * G::kRowSets + blockIdx.x / kPart;
+    const int sub = blockIdx.x % kPart;  // part of the set
+    const int b = set / G::kRowSets;
+    const long long g0 = meetings_before(P.row0, P.nsets);
+    // CTAs f..l (inclusive) whose stretches touch steps [a, e); no stretch is
+    // empty
+    auto ctas = [&](unsigned a, unsigned e, int &f, int &l) {
+        int lo = 0, hi = P.ncta - 1;  // last c with step[c] <= a
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (P.step[mid] <= a)
+                lo = mid;
+            else
+                hi = mid - 1;
+        }
+        f = lo;
+        while (lo + 1 < P.ncta && P.step[lo + 1] < e)
+            lo++;
+        l = lo;
+    };
+    const int nrow = min(b, P.row1) - P.row0;  // earlier rows of this phase
+    auto meeting = [&](int r) {  // of row row0 + r with the set, in the phase
+        const int row = P.row0 + r;
+        return (int)(meetings_before(row, P.nsets) - g0) + (set - row * G::kRowSets);
+    };
+    for (int r = tid; r < nrow; r += kReduceThreads) {
+        const unsigned g = (unsigned)meeting(r);
+        int f, l;
+        ctas(g << 5, (g << 5) + 32, f, l);
+        first[r] = (unsigned short)f;
+        count[r] = (unsigned short)(l - f + 1);
+    }
+    __syncthreads();
+    if (tid < 32) {  // list of slots, in row order
+        int base = 0;
+        for (int r0 = 0; r0 < nrow; r0 += 32) {
+            const int r = r0 + tid, c = r < nrow ? count[r] : 0;
+            int incl = c;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int v = __shfl_up_sync(0xffffffffu, incl, o);
+                if (tid >= o)
+                    incl += v;
+            }
+            if (c) {
+                const int slot = meeting(r) + first[r];
+                for (int q = 0; q < c; q++)
+                    list[base + incl - c + q] = slot + q;
+            }
+            base += __shfl_sync(0xffffffffu, incl, 31);
+        }
+        if (tid == 0)
+            n_list = base;
+    }
+    __syncthreads();
+    const bool final = b < P.row1;  // else rows to come add to these bodies
+    const int nr = n_list;
+    int tf = 0, tl = -1;
+    if (final)
+        ctas((unsigned)((meetings_before(b, P.nsets) - g0) << 5),
+             (unsigned)((meetings_before(b + 1, P.nsets) - g0) << 5), tf, tl);
+    const int total = nr + (tl - tf + 1);
+    const int q0 = total * group / kReduceGroups, q1 = total * (group + 1) / kReduceGroups;
+    const float *react = P.react + (size_t)comp * kSet + sub * kB + j;
+    const int i = set * kSet + sub * kB + j;
+    const float *tsum = P.tsum + (size_t)comp * G::kRow + (i - b * G::kRow) +
+                        (size_t)(b - P.row0 + tf) * 3 * G::kRow;
+    auto piece = [&](int q) {
+        return q < nr ? react + (size_t)list[q] * 3 * kSet
+                      : tsum + (size_t)(q - nr) * 3 * G::kRow;
+    };
+    grid_dependents_launch();
+    grid_dependency_wait();
+    float hi = 0.f, lo = 0.f;
+    if (P.row0 > 0 && group == 0) {
+        hi = R.carry[comp * R.npad + i];
+        lo = R.carry[(3 + comp) * R.npad + i];
+    }
+    int q = q0;
+    for (; q + 8 <= q1; q += 8) {
+        float v[8];
+#pragma unroll
+        for (int u = 0; u < 8; u++)
+            v[u] = __ldcs(piece(q + u));
+#pragma unroll
+        for (int u = 0; u < 8; u++)
+            comp_add(hi, lo, v[u]);
+    }
+    if (q < q1) {
+        float v[8];
+#pragma unroll
+        for (int u = 0; u < 8; u++)
+            v[u] = q + u < q1 ? __ldcs(piece(q + u)) : 0.f;
+#pragma unroll
+        for (int u = 0; u < 8; u++)
+            comp_add(hi, lo, v[u]);
+    }
+    if (group) {
+        part[group - 1][0][comp][j] = hi;
+        part[group - 1][1][comp][j] = lo;
+    }
+    __syncthreads();
+    if (group == 0) {
+#pragma unroll
+        for (int q = 0; q < kReduceGroups - 1; q++) {
+            comp_add(hi, lo, part[q][0][comp][j]);
+            lo += part[q][1][comp][j];
+        }
+        if (!final) {
+            R.carry[comp * R.npad + i] = hi;
+            R.carry[(3 + comp) * R.npad + i] = lo;
+        }
+        out[comp][j] = hi + lo;
+    }
+    if (!final)
+        return;
+    __syncthreads();
+    const int ib = set * kSet + sub * kB + tid;
+    if (tid < kB && ib < P.n) {
+        const float fx = out[0][tid], fy = out[1][tid], fz = out[2][tid];
+        R.force[ib] = make_float4(fx, fy, fz, 0.f);
+        if (R.fi.vel) {
+            const float4 v = P.pm[ib];
+            fused_integrate(R.fi, ib, v.x, v.y, v.z, v.w, fx, fy, fz);
+        }
+    }
+}
+
+// Cost of a step: both ways against one-sided (measured 4 : 3); a stretch has
+// at least kMinCost (no stretch is empty, and few pieces at small N).
+constexpr int kCostBoth = 4, kCostOne = 3, kMinCost = 32;
+
+static int sets_of(size_t n) { return (int)((n + G::kSet - 1) / G::kSet); }
+static int rows_of(size_t n) { return (int)((n + G::kRow - 1) / G::kRow); }
+
+// Cost of the rows before b, from row 0 (meetings x 32 steps).
+static long long cost_before(int b, int nsets) {
+    return 32 * (kCostBoth * meetings_before(b, nsets) -
+                 (long long)(kCostBoth - kCostOne) * std::min((long long)G::kRowSets * b,
+                                                              (long long)nsets));
+}
+
+// The step at cost offset `at` from row0 (rows row0..row1-1), rounded up to
+// a whole step.
+static unsigned step_at(long long at, int row0, int row1, int nsets) {
+    const long long c0 = cost_before(row0, nsets), g0 = meetings_before(row0, nsets);
+    int lo = row0, hi = row1 - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (cost_before(mid, nsets) - c0 <= at)
+            lo = mid;
+        else
+            hi = mid - 1;
+    }
+    long long off = at - (cost_before(lo, nsets) - c0);
+    const long long own = 32LL * kCostOne * std::min(G::kRowSets, nsets - lo * G::kRowSets);
+    long long steps = 32 * (meetings_before(lo, nsets) - g0);
+    if (off <= own)
+        steps += (off + kCostOne - 1) / kCostOne;
+    else
+        steps += own / kCostOne + (off - own + kCostBoth - 1) / kCostBoth;
+    return (unsigned)steps;
+}
+
+}  // namespace pair
+
+using pair::G;
+
+static size_t align256(size_t x) { return (x + 255) / 256 * 256; }
+
+// Reaction pieces of one phase of rows [row0, row1).
+static size_t react_bytes(int row0, int row1, int nsets, int ncta) {
+    const long long g = pair::meetings_before(row1, nsets) - pair::meetings_before(row0, nsets);
+    return (size_t)(g + ncta) * 3 * G::kSet * 4;
+}
+
+// Rows of the phase that starts at `row`: as many as fit (0: not even one).
+static int phase_end(int row, int rows, int nsets, int ncta, size_t room) {
+    int end = row;
+    while (end < rows && end - row < kMaxPairRows &&
+           react_bytes(row, end + 1, nsets, ncta) <= room)
+        end++;
+    return end;
+}
+
+bool plan_pair(size_t n, int sms, size_t max_bytes, PairPlan &pl) {
+    if (n == 0 || n > kMaxBodies || sms <= 0)
+        return false;
+    pl = PairPlan{};
+    pl.n = n;
+    const int nsets = pair::sets_of(n), rows = pair::rows_of(n);
+    pl.ncta = (int)std::min<long long>(std::min(sms * G::kCtas, kMaxPairCtas),
+                                       pair::cost_before(rows, nsets) / pair::kMinCost);
+    const size_t tsum =
+        align256((size_t)(std::min(rows, kMaxPairRows) + pl.ncta) * 3 * G::kRow * 4);
+    const size_t carry = align256((size_t)nsets * G::kSet * 6 * 4);
+    const size_t all = align256(react_bytes(0, rows, nsets, pl.ncta));
+    // a phase of 256 MiB of pieces is about 16 ms of work; always at least
+    // four rows
+    size_t room = std::max((size_t)256 << 20, (size_t)4 * (nsets + pl.ncta) * 3 * G::kSet * 4);
+    if (max_bytes) {
+        if (rows <= kMaxPairRows && all + tsum <= max_bytes)
+            room = std::min(room, max_bytes - tsum);
+        else if (max_bytes > tsum + carry)
+            room = std::min(room, (max_bytes - tsum - carry) & ~(size_t)255);
+        else
+            return false;
+    }
+    const bool one = rows <= kMaxPairRows && all <= room;
+    if (!one && phase_end(0, rows, nsets, pl.ncta, room) == 0)
+        return false;
+    pl.react_bytes = one ? all : room;
+    pl.off_react = 0;
+    pl.off_tsum = align256(pl.react_bytes);
+    pl.off_carry = pl.off_tsum + tsum;
+    pl.workspace_bytes = pl.off_carry + (one ? 0 : carry);
+    return !max_bytes || pl.workspace_bytes <= max_bytes;
+}
+
+int launch_pair(const PairPlan &pl, float4 *force, const float4 *posMass, float eps2,
+                void *workspace, cudaStream_t st, const FusedIntegrate *fi) {
+    static_assert(sizeof(pair::ReduceParams) <= 4096, "kernel parameters");
+    const int nsets = pair::sets_of(pl.n), rows = pair::rows_of(pl.n);
+    char *ws = (char *)workspace;
+    pair::ReduceParams R;
+    pair::Params &P = R.p;
+    P.pm = posMass;
+    P.react = (float *)(ws + pl.off_react);
+    P.tsum = (float *)(ws + pl.off_tsum);
+    P.n = (int)pl.n;
+    P.nsets = nsets;
+    P.eps2 = eps2;
+    P.status = pl.status;
+    P.short_ok = eps2 >= 8.3e-25f && eps2 <= 1.2e24f;  // 2^-80 .. 2^80
+    R.carry = (float *)(ws + pl.off_carry);
+    R.npad = (size_t)nsets * G::kSet;
+    R.force = force;
+    R.fi = fi ? *fi : FusedIntegrate{};
+    R.fi.js = nullptr;
+    for (P.row0 = 0; P.row0 < rows; P.row0 = P.row1) {
+        P.row1 = phase_end(P.row0, rows, nsets, pl.ncta, pl.react_bytes);
+        if (P.row1 == P.row0)
+            return NBGB_ERR_WORKSPACE;
+        const long long total =
+            pair::cost_before(P.row1, nsets) - pair::cost_before(P.row0, nsets);
+        P.ncta = (int)std::min<long long>(pl.ncta, total / pair::kMinCost);
+        for (int c = 0; c < P.ncta; c++)
+            P.step[c] = pair::step_at(total * c / P.ncta, P.row0, P.row1, nsets);
+        P.step[P.ncta] = (unsigned)((pair::meetings_before(P.row1, nsets) -
+                                     pair::meetings_before(P.row0, nsets))
+                                    << 5);
+        if (launch_dependent(pair::pair_kernel, P.ncta, G::kThreads, G::kSmem, st, P) !=
+                cudaSuccess ||
+            launch_dependent(pair::pair_reduce_kernel,
+                             (nsets - P.row0 * G::kRowSets) * (G::kSet / pair::kReduceBodies),
+                             pair::kReduceThreads, 0, st, R) != cudaSuccess)
+            return NBGB_ERR_CUDA;
+    }
+    return NBGB_OK;
+}
+
+int pair_launches(const PairPlan &pl) {
+    const int nsets = pair::sets_of(pl.n), rows = pair::rows_of(pl.n);
+    int k = 0;
+    for (int row = 0; row < rows; k++) {
+        const int end = phase_end(row, rows, nsets, pl.ncta, pl.react_bytes);
+        if (end == row)
+            break;
+        row = end;
+    }
+    return 2 * k;
+}
+
+int pair_prepare() {
+    return cudaFuncSetAttribute(pair::pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)G::kSmem) == cudaSuccess
+               ? NBGB_OK
+               : NBGB_ERR_CUDA;
+}
+
+}  // namespace nbgb

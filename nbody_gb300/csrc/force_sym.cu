@@ -253,13 +253,6 @@ __device__ __forceinline__ void sym_block_pair(const Params &P, int bi, int bj) 
     }
 }
 
-template <int KI_>
-__global__ void __launch_bounds__(kThreads, Geo<KI_>::kMinBlocks) sym_kernel(Params P) {
-    int bi, bj;
-    pair_of(blockIdx.x, P.nblocks, bi, bj);
-    sym_block_pair<KI_>(P, bi, bj);
-}
-
 // Many systems in one launch (the ensemble's Newton-3 systems): CTA b takes
 // block pair b - pair_begin[s] of the system s whose range holds b (binary
 // search over the systems' prefix counts).
@@ -300,14 +293,6 @@ __global__ void sym_finish_zero_kernel(double *__restrict__ acc, int n, int npad
     }
 }
 
-__global__ void sym_finish_kernel(const double *__restrict__ acc, int n, int npad,
-                                  float4 *__restrict__ force) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n)
-        force[i] = make_float4((float)acc[i], (float)acc[(size_t)npad + i],
-                               (float)acc[2 * (size_t)npad + i], 0.f);
-}
-
 }  // namespace sym
 
 int launch_sym_systems(const SymSystem *d_tab, const SymSystem *h_tab, int nsys,
@@ -331,12 +316,6 @@ int sym_block_bodies() { return sym::Geo<sym::kWideKI>::kBlock; }
 
 namespace {
 
-struct SymLayout {
-    int ki, block;  // geometry: targets per lane, bodies per block
-    int nblocks, npad;
-    size_t off_js, off_acc, bytes;
-};
-
 int device_sms() {
     int dev = 0, sms = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
@@ -348,25 +327,6 @@ int device_sms() {
     return sms;
 }
 
-// The wide geometry (2048-body blocks, one CTA per SM) when its block pairs
-// give every SM at least two; the narrow one (1024-body blocks, four times
-// the pairs) below that.
-SymLayout sym_layout(size_t n) {
-    using Wide = nbgb::sym::Geo<nbgb::sym::kWideKI>;
-    using Narrow = nbgb::sym::Geo<nbgb::sym::kNarrowKI>;
-    SymLayout L;
-    const long long nbw = (long long)((n + Wide::kBlock - 1) / Wide::kBlock);
-    const bool wide = nbw * (nbw + 1) / 2 >= 2LL * device_sms();
-    L.ki = wide ? Wide::KI : Narrow::KI;
-    L.block = wide ? Wide::kBlock : Narrow::kBlock;
-    L.nblocks = (int)((n + L.block - 1) / L.block);
-    L.npad = L.nblocks * L.block;
-    L.off_js = 0;
-    L.off_acc = ((size_t)L.npad * 16 + 255) / 256 * 256;
-    L.bytes = L.off_acc + (size_t)3 * L.npad * sizeof(double);
-    return L;
-}
-
 }  // namespace
 
 extern "C" {
@@ -374,7 +334,8 @@ extern "C" {
 NBGB_API size_t nbgb_force_newton3_workspace_bytes(size_t N) {
     if (N == 0 || N > nbgb::kMaxBodies)
         return 0;
-    return sym_layout(N).bytes;
+    nbgb::PairPlan pl;
+    return nbgb::plan_pair(N, device_sms(), 0, pl) ? pl.workspace_bytes : 0;
 }
 
 NBGB_API int nbgb_force_newton3(float *force, const float *posMass, float softeningSquared,
@@ -385,44 +346,13 @@ NBGB_API int nbgb_force_newton3(float *force, const float *posMass, float soften
         return NBGB_ERR_INVALID_ARGUMENT;
     if (((uintptr_t)force | (uintptr_t)posMass) & 15u)
         return NBGB_ERR_INVALID_ARGUMENT;
-    const SymLayout L = sym_layout(N);
-    if (!workspace || workspace_bytes < L.bytes || ((uintptr_t)workspace & 255u))
-        return NBGB_ERR_WORKSPACE;
-    cudaStream_t st = (cudaStream_t)stream;
-    char *ws = (char *)workspace;
-    // the j-stream (paired layout, zero-mass padding to whole blocks)
-    nbgb::ForcePlan pl;
-    pl.n = N;
-    pl.ntiles = L.nblocks;
-    pl.tile_bodies = L.block;
-    pl.js_vpb = 1;
-    pl.nsplit = 1;
-    pl.off_js = L.off_js;
-    int rc = nbgb::launch_pack(pl, (const float4 *)posMass, ws, st);
-    if (rc != NBGB_OK)
-        return rc;
-    double *acc = (double *)(ws + L.off_acc);
-    if (cudaMemsetAsync(acc, 0, (size_t)3 * L.npad * sizeof(double), st) != cudaSuccess)
+    nbgb::PairPlan pl;
+    if (!nbgb::plan_pair(N, device_sms(), 0, pl) || nbgb::pair_prepare() != NBGB_OK)
         return NBGB_ERR_CUDA;
-    nbgb::sym::Params P;
-    P.pm = (const float4 *)posMass;
-    P.js = (const float4 *)(ws + L.off_js);
-    P.acc = acc;
-    P.n = (int)N;
-    P.npad = L.npad;
-    P.nblocks = L.nblocks;
-    P.eps2 = softeningSquared;
-    const long long pairs = (long long)L.nblocks * (L.nblocks + 1) / 2;
-    if (pairs > (1ll << 31) - 1)
-        return NBGB_ERR_TOO_LARGE;
-    if (L.ki == nbgb::sym::kWideKI)
-        nbgb::sym::sym_kernel<nbgb::sym::kWideKI><<<(unsigned)pairs, nbgb::sym::kThreads, 0, st>>>(P);
-    else
-        nbgb::sym::sym_kernel<nbgb::sym::kNarrowKI>
-            <<<(unsigned)pairs, nbgb::sym::kThreads, 0, st>>>(P);
-    nbgb::sym::sym_finish_kernel<<<(unsigned)((N + 255) / 256), 256, 0, st>>>(
-        acc, (int)N, L.npad, (float4 *)force);
-    return cudaGetLastError() == cudaSuccess ? NBGB_OK : NBGB_ERR_CUDA;
+    if (!workspace || workspace_bytes < pl.workspace_bytes || ((uintptr_t)workspace & 255u))
+        return NBGB_ERR_WORKSPACE;
+    return nbgb::launch_pair(pl, (float4 *)force, (const float4 *)posMass, softeningSquared,
+                             workspace, (cudaStream_t)stream);
 }
 
 }  // extern "C"

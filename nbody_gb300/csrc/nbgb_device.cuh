@@ -367,6 +367,27 @@ __device__ __forceinline__ void fence_proxy_async_shared() {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
 
+// Per-thread asynchronous copy of 16 bytes (bytes of them from src, the rest
+// zeros) and the wait for all of this thread's copies.
+__device__ __forceinline__ void async_g2s_16(void *dst, const void *src, uint32_t bytes) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_addr(dst)), "l"(src),
+                 "r"(bytes)
+                 : "memory");
+}
+__device__ __forceinline__ void async_wait_all() {
+    asm volatile("cp.async.wait_all;" ::: "memory");
+}
+
+// Programmatic dependent launch: let the next kernel's CTAs start when this
+// kernel's have all come here or left; wait until the previous kernel is
+// complete and its writes are visible (at once for an ordinary launch).
+__device__ __forceinline__ void grid_dependents_launch() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void grid_dependency_wait() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 __device__ __forceinline__ uint64_t global_ns() {
     uint64_t t;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));

@@ -17,6 +17,37 @@ constexpr size_t kMaxBodies = (size_t)1 << 30;
 // NBGB_ERR_CUDA.
 int current_context(int *device, unsigned long long *ctx_id);
 
+// The pair kernel's decomposition and workspace layout (force_pair.cu).
+struct PairPlan {
+    size_t n = 0;
+    int ncta = 0;             // stretches (resident CTAs)
+    size_t react_bytes = 0;   // reaction pieces of one phase, at most
+    size_t off_react = 0, off_tsum = 0, off_carry = 0;
+    size_t workspace_bytes = 0;
+    // not null: masses < 0 (or NaN) are refused, as by log-domain plans (NaN
+    // forces, NBGB_STATUS_NEGATIVE_MASS set in this device word)
+    unsigned *status = nullptr;
+};
+
+// Launches a kernel with programmatic dependence on the stream's previous
+// kernel: its CTAs may start early, so the kernel must call
+// grid_dependency_wait() before it touches global memory.
+template <typename Args>
+cudaError_t launch_dependent(void (*kernel)(Args), unsigned grid, unsigned block, size_t smem,
+                             cudaStream_t st, const Args &args) {
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, args);
+}
+
 // One force evaluation's decomposition and workspace layout.
 struct ForcePlan {
     int config = 0;       // index into the kernel configuration table
@@ -34,6 +65,10 @@ struct ForcePlan {
     size_t ni_pad = 0;    // nblocks * BI
     size_t off_js = 0, off_hi = 0, off_lo = 0, off_cnt = 0;
     size_t workspace_bytes = 0;
+    // evaluate pairs once (pair) instead of the one-sided decomposition above,
+    // which describes what a forced plan of the same size would run
+    int use_pair = 0;
+    PairPlan pair;
 };
 
 int plan_force(size_t n, int force_config, int force_nsplit, ForcePlan &pl);
@@ -72,6 +107,18 @@ struct FusedIntegrate {
 int launch_force(const ForcePlan &pl, float4 *force, const float4 *posMass, const float4 *jstream,
                  float eps2, void *workspace, cudaStream_t stream,
                  const FusedIntegrate *fi = nullptr);
+// Pairs evaluated once (force_pair.cu): plan for n bodies on a device with
+// `sms` SMs (max_bytes > 0: within that workspace; false when it cannot),
+// and the launches (no j-stream; fi as for launch_force, fi->js ignored).
+constexpr int kMaxPairCtas = 512;          // step table in the kernel parameters
+constexpr int kMaxPairRows = 1024;         // rows of a phase
+constexpr size_t kMinPairForce = 6144;     // force(): sizes that take the pair kernel
+constexpr size_t kMaxPairForce = (size_t)1 << 23;
+bool plan_pair(size_t n, int sms, size_t max_bytes, PairPlan &pl);
+int launch_pair(const PairPlan &pl, float4 *force, const float4 *posMass, float eps2,
+                void *workspace, cudaStream_t st, const FusedIntegrate *fi = nullptr);
+int pair_launches(const PairPlan &pl);
+int pair_prepare();  // kernel attributes of the current context
 int read_and_clear_status(unsigned *bits);
 int read_status_ensemble(unsigned *bits);
 int read_status_integrate(unsigned *bits);

@@ -84,7 +84,8 @@ struct nbgb_system {
 
 namespace {
 
-float4 *js_of(nbgb_system *s) { return (float4 *)((char *)s->ws + s->plan.off_js); }
+// (a plan that evaluates pairs once reads posMass and keeps no j-stream)
+float4 *js_of(nbgb_system *s) { return s->plan.use_pair ? nullptr : (float4 *)((char *)s->ws + s->plan.off_js); }
 float4 *js_cur_ptr(nbgb_system *s) { return s->js_cur ? s->js2 : js_of(s); }
 float4 *js_next_ptr(nbgb_system *s) { return s->js_cur ? js_of(s) : s->js2; }
 
@@ -96,9 +97,9 @@ void drop_graphs(nbgb_system *s) {
     s->graph = s->graph2 = nullptr;
 }
 unsigned *cnt_of(nbgb_system *s) {
-    return nbgb::split_blocks(s->plan) ? (unsigned *)((char *)s->ws + s->plan.off_cnt) : nullptr;
+    return !s->plan.use_pair && nbgb::split_blocks(s->plan) ? (unsigned *)((char *)s->ws + s->plan.off_cnt) : nullptr;
 }
-int ncnt_of(nbgb_system *s) { return nbgb::split_blocks(s->plan); }
+int ncnt_of(nbgb_system *s) { return s->plan.use_pair ? 0 : nbgb::split_blocks(s->plan); }
 int npad_of(nbgb_system *s) { return s->plan.ntiles * s->plan.tile_bodies; }
 
 double *comp(nbgb_system *s, int c) { return s->x64 + (size_t)c * s->ld; }
@@ -132,6 +133,8 @@ size_t js_bytes(const nbgb::ForcePlan &pl) {
 // system and whenever the plan changes (never inside a step, so steps can be
 // captured by the caller), large enough for the plan.
 int alloc_js2(nbgb_system *s) {
+    if (s->plan.use_pair)
+        return NBGB_OK;
     const size_t bytes = js_bytes(s->plan);
     s->js2_ready = false;
     if (s->js2 && s->js2_bytes >= bytes)
@@ -204,7 +207,7 @@ int ref_step_body(nbgb_system *s) {
         fi.damping = s->damping;
         fi.fused_drift = fused_drift;
         int rc = timed_force(s, &fi);
-        if (rc == NBGB_OK)
+        if (rc == NBGB_OK && !s->plan.use_pair)
             s->js_cur ^= 1;
         return rc;
     }
@@ -329,7 +332,7 @@ void free_all(nbgb_system *s) {
 // The reference step with the integrate fused into the force launch, which
 // alternates between the two j-stream buffers.
 bool alternates(const nbgb_system *s) {
-    return reference_integrator(s->integrator) && s->algorithm == 0;
+    return reference_integrator(s->integrator) && s->algorithm == 0 && !s->plan.use_pair;
 }
 
 // Steps per captured graph.  Kernels inside one graph start back to back;

@@ -1,0 +1,152 @@
+"""Forces with each pair evaluated once (nbgb_force_newton3 at every N, the
+default force at larger N) at the edges of its tiles, against FP64 and the
+one-sided kernel: sets of 128 sources, rows of 1,408 targets, the sizes where
+the default force changes kernels, phases, and the forms for equal masses and
+for positions far from the origin."""
+import numpy as np
+import pytest
+
+from oracle import oracle as O
+
+import nbody_gb300 as nb
+
+pytestmark = pytest.mark.gpu
+
+TOL_VS_FP64 = 5e-6   # the force gate of the other tests
+ONE_SIDED = 25       # a one-sided configuration that takes masses of any sign
+
+
+def _run(fn, pm, *args, **kw):
+    import torch
+    t = torch.from_numpy(np.ascontiguousarray(pm, np.float32)).cuda()
+    out = fn(t, *args, **kw)
+    torch.cuda.synchronize()
+    return out.cpu().numpy()
+
+
+def _err(out, pm, eps2, idx=None):
+    f = O.ieee().forces_f64(pm, float(np.float32(eps2)), idx)
+    o = out if idx is None else out[idx]
+    assert np.all(o[:, 3] == 0)
+    return (np.linalg.norm(o[:, :3] - f, axis=1) / np.linalg.norm(f, axis=1)).max()
+
+
+@pytest.mark.parametrize("n", [2, 63, 64, 65, 127, 128, 129, 1407, 1408, 1409, 1535, 1537, 2817,
+                               6143, 6144, 6145, 7681])
+def test_edges_of_sets_and_rows(cuda, n):
+    pm, _ = nb.ic_uniform_ball(n, 40 + n, 1.0, 0.5, 1.5)
+    out = _run(nb.force_newton3, pm, 1e-4)
+    assert nb.last_status() == 0
+    assert _err(out, pm, 1e-4) <= TOL_VS_FP64
+    assert np.array_equal(out, _run(nb.force_newton3, pm, 1e-4))  # deterministic
+    if nb.force_kind(n)[0] == "pairs":
+        assert np.array_equal(_run(nb.force, pm, 1e-4), out)
+
+
+def test_kinds_and_launches(cuda):
+    assert nb.force_kind(1000) == ("onesided", 2)
+    assert nb.force_kind(16384) == ("pairs", 2)
+    kind, launches = nb.force_kind(400000)  # several phases
+    assert kind == "pairs" and launches > 2 and launches % 2 == 0
+
+
+def test_phases_against_the_one_sided_kernel(cuda):
+    """N = 400,001: reaction pieces beyond one phase's workspace, carried
+    sums, a ragged last row and set."""
+    n = 400001
+    _, _, pm, _ = nb.ic_plummer(n, 12)
+    out = _run(nb.force, pm, 1e-4)
+    assert nb.last_status() == 0
+    idx = np.unique(np.concatenate([np.random.default_rng(2).choice(n, 200, replace=False),
+                                    [0, 1407, 1408, n - 130, n - 1]]))
+    assert _err(out, pm, 1e-4, idx) <= TOL_VS_FP64
+    one = _run(nb.force, pm, 1e-4, config=ONE_SIDED)
+    d = np.linalg.norm(out - one, axis=1) / np.linalg.norm(one, axis=1)
+    assert d.max() <= TOL_VS_FP64
+
+
+def _mass_case(case, n):
+    pm, _ = nb.ic_uniform_ball(n, 5, 1.0, 0.5, 1.5)
+    pm = pm.copy()
+    if case == "equal":
+        pm[:, 3] = np.float32(1.0 / n)
+    elif case == "equal but one":  # one warp's targets and one set stay mixed
+        pm[:, 3] = np.float32(1.0 / n)
+        pm[2000, 3] *= 3
+    elif case == "zeros":
+        pm[::3, 3] = 0
+    elif case == "equal in sets":  # each set of 128 equal, sets differ
+        pm[:, 3] = (np.float32(1.0 / n) *
+                    (1 + (np.arange(n) // 128) % 5)).astype(np.float32)
+    elif case == "signed":
+        pm[::7, 3] *= -1
+    return pm
+
+
+@pytest.mark.parametrize("case", ["equal", "equal but one", "zeros", "equal in sets", "signed"])
+def test_mass_forms(cuda, case):
+    n = 6500
+    pm = _mass_case(case, n)
+    out = _run(nb.force_newton3, pm, 1e-4)
+    assert nb.last_status() == 0
+    f = O.ieee().forces_f64(pm, float(np.float32(1e-4)))
+    scale = np.linalg.norm(O.ieee().forces_f64(np.abs(pm), float(np.float32(1e-4))), axis=1)
+    # signed masses cancel: errors relative to the unsigned system's forces
+    ref = np.maximum(np.linalg.norm(f, axis=1), scale if case == "signed" else 0)
+    assert (np.linalg.norm(out[:, :3] - f, axis=1) / ref).max() <= TOL_VS_FP64
+
+
+@pytest.mark.parametrize("where", ["all", "some", "tiny"])
+def test_far_positions_keep_the_one_sided_range(cuda, where):
+    """Beyond 2^40 from the origin (or eps2 below 2^-80) (|d|^2+eps2)^-3/2
+    alone leaves the binary32 range while m times it does not."""
+    n = 6300
+    pm, _ = nb.ic_uniform_ball(n, 6, 1.0, 0.5, 1.5)
+    pm = pm.copy()
+    k, eps2 = {"all": (43, 1e-4 * 2.0 ** 86), "some": (43, 1e-4), "tiny": (-45, 1e-4 * 2.0 ** -90)}[
+        where]
+    sel = slice(None) if where != "some" else slice(1000, 4000)
+    pm[sel, :3] *= np.float32(2.0 ** k)
+    pm[:, 3] *= np.float32(2.0 ** (60 if k > 0 else -60))
+    out = _run(nb.force, pm, eps2)
+    assert nb.force_kind(n)[0] == "pairs" and nb.last_status() == 0
+    one = _run(nb.force, pm, eps2, config=ONE_SIDED)
+    assert np.all(np.isfinite(out)) and np.any(one != 0)
+    r = np.linalg.norm(one.astype(np.float64), axis=1)
+    d = np.linalg.norm(out.astype(np.float64) - one, axis=1)
+    assert np.all(d <= 2e-5 * r + 2e-5 * np.median(r) * (where == "some"))
+
+
+@pytest.mark.parametrize("what,value", [("x", np.nan), ("x", np.inf), ("x", 1e20), ("m", np.inf)])
+def test_special_values_as_the_one_sided_kernel(cuda, what, value):
+    n = 6200
+    pm, _ = nb.ic_uniform_ball(n, 7, 1.0, 0.5, 1.5)
+    pm = pm.copy()
+    pm[4321, 0 if what == "x" else 3] = value
+    out = _run(nb.force, pm, 1e-4)
+    one = _run(nb.force, pm, 1e-4, config=ONE_SIDED)
+    nb.last_status()
+    assert np.array_equal(np.isnan(out), np.isnan(one))
+    assert np.array_equal(np.isinf(out), np.isinf(one))
+    assert np.array_equal(np.sign(out[np.isinf(out)]), np.sign(one[np.isinf(one)]))
+
+
+def test_negative_masses_stay_refused_by_the_stream_ordered_force(cuda):
+    """As a log-domain plan: NaN forces and the status bit from nb.force; the
+    drop-in evaluates again and takes any sign."""
+    import torch
+    n = 7000
+    pm = _mass_case("signed", n)
+    out = _run(nb.force, pm, 1e-4)
+    assert nb.last_status() == 0x8 and np.all(np.isnan(out[:, :3]))
+    t = torch.from_numpy(pm).cuda()
+    f = torch.zeros_like(t)
+    assert nb.ComputeGravitation_GPU_GB300(f, t, 1e-4, n) > 0.0
+    assert nb.last_status() == 0
+    assert np.array_equal(f.cpu().numpy(), _run(nb.force_newton3, pm, 1e-4))
+
+
+@pytest.mark.parametrize("n", [6144, 9001])
+def test_whole_row_slice_is_the_default_force(cuda, n):
+    pm, _ = nb.ic_uniform_ball(n, 8, 1.0, 0.5, 1.5)
+    assert np.array_equal(_run(nb.force_rows, pm, 1e-4, 0, n), _run(nb.force, pm, 1e-4))
