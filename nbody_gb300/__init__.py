@@ -173,7 +173,12 @@ def force(posMass, softeningSquared: float, out=None, stream=None, workspace: Wo
         out = torch.empty((n, 4), dtype=torch.float32, device=posMass.device)
     if n == 0:
         return out
-    _, _, wsb = force_plan(n, config, nsplit)
+    if config == -1 and nsplit == -1:
+        wsb = load().nbgb_force_workspace_bytes(n)
+        if wsb == 0:
+            raise NbgbError(-1, "nbgb_force_workspace_bytes")
+    else:
+        _, _, wsb = force_plan(n, config, nsplit)
     ws = (workspace or _default_ws).get(wsb)
     check(load().nbgb_force_ex(_dev(out), _dev(posMass), softeningSquared, n, ws.data_ptr(),
                                ws.numel(), config, nsplit, _stream(stream)), "nbgb_force")

@@ -850,21 +850,21 @@ static int plan_force_among(size_t n, const std::vector<int> &cands, int force_n
         [](const ForcePlan &) { return true; }, d);
 }
 
-// Evaluate pairs once (force_pair.cu) from kMinPairForce bodies on: 14-16
-// FP32 operations for two interactions against 23.  Microseconds a call,
-// pairs against the one-sided plan (back to back in a graph, GB300, uniform
-// ball): N = 4,096 16 / 15, 6,000 24 / 23, 8,192 31 / 37, 10,007 40 / 53,
-// 16,384 85 / 110, 131,072 4,415 / 5,820; equal masses (Plummer) 100,003
-// 2,390 / 3,480, 131,072 4,065 / 5,820, 2^20 253,200 / 369,100.  Below the line the one-sided kernel's finer split wins; above
-// kMaxPairForce a phase's pieces (12 N bytes a row) take too much workspace.
+// Evaluate pairs once (force_pair.cu) up to kMaxPairForce bodies: 14-16 FP32
+// operations for two interactions against 23.  Microseconds a call, pairs
+// against the one-sided plan and its pack launch (back to back in a graph,
+// GB300, uniform ball): N = 300 5.3 / 8.8, 1,000 5.9 / 10.1, 2,048 7.0 / 12,
+// 4,096 11 / 15, 8,192 27 / 37, 10,007 37 / 53, 16,384 85 / 110, 131,072
+// 4,415 / 5,820; equal masses (Plummer) 100,003 2,390 / 3,480, 131,072 4,065
+// / 5,820, 2^20 253,200 / 369,100.  Above the line a phase's pieces (12 N
+// bytes a row) take too much workspace.
 // Results of pair plans are closer to 64 bits at every size (3.7e-8 against
 // 8.5e-8 at 100,003).  A plan that would take log-domain pairs refuses
 // negative masses as that plan does.
 static void use_pair_plan(ForcePlan &pl, const DeviceInfo *d, size_t max_bytes = 0) {
     if (!d)
         d = device_info();
-    if (!d || pl.n < kMinPairForce || pl.n > kMaxPairForce ||
-        !plan_pair(pl.n, d->sms, max_bytes, pl.pair))
+    if (!d || pl.n > kMaxPairForce || !plan_pair(pl.n, d->sms, max_bytes, pl.pair))
         return;
     pl.use_pair = 1;
     pl.pair.status = pl.js_log ? d->status : nullptr;
@@ -893,11 +893,31 @@ int plan_force(size_t n, int force_config, int force_nsplit, ForcePlan &pl) {
     return plan_force_on(n, force_config, force_nsplit, pl, nullptr);
 }
 
+// The default force: as plan_force(n, -1, -1) without costing the one-sided
+// plans (3-200 us of host time) where pairs are evaluated once.
+int plan_force_default(size_t n, ForcePlan &pl) {
+    if (n == 0 || n > kMaxBodies)
+        return NBGB_ERR_INVALID_ARGUMENT;
+    const DeviceInfo *d = device_info();
+    if (!d)
+        return NBGB_ERR_CUDA;
+    pl = ForcePlan{};
+    pl.n = n;
+    pl.js_log = 1;  // the default one-sided plans are log-domain ones
+    use_pair_plan(pl, d);
+    return pl.use_pair ? NBGB_OK : plan_force(n, -1, -1, pl);
+}
+
+int pair_device_sms() {
+    const DeviceInfo *d = device_info();
+    return d ? d->sms : 0;
+}
+
 int plan_force_rows(size_t n, size_t rows, ForcePlan &pl) {
     if (n == 0 || n > kMaxBodies || rows == 0 || rows > n)
         return NBGB_ERR_INVALID_ARGUMENT;
     if (rows == n)  // the whole force
-        return plan_force(n, -1, -1, pl);
+        return plan_force_default(n, pl);
     return plan_force_among(n,
                             std::vector<int>(std::begin(kDefaultCandidates),
                                              std::end(kDefaultCandidates)),
@@ -921,11 +941,15 @@ int plan_force_rsqrt(size_t n, ForcePlan &pl) {
 int plan_force_within(size_t n, size_t max_bytes, ForcePlan &pl) {
     if (n == 0 || n > kMaxBodies)
         return NBGB_ERR_INVALID_ARGUMENT;
+    pl = ForcePlan{};
+    pl.n = n;
+    pl.js_log = 1;  // as plan_force_default
+    use_pair_plan(pl, nullptr, max_bytes);
+    if (pl.use_pair)
+        return NBGB_OK;
     const int rc = plan_enumerate(
         n, 0, kDefaultCandidates, (int)(sizeof(kDefaultCandidates) / sizeof(int)), -1, pl,
         [max_bytes](const ForcePlan &c) { return c.workspace_bytes <= max_bytes; });
-    if (rc == NBGB_OK)
-        use_pair_plan(pl, nullptr, max_bytes);
     return rc == NBGB_ERR_UNSUPPORTED ? NBGB_ERR_TOO_LARGE : rc;
 }
 
@@ -1080,7 +1104,7 @@ extern "C" {
 
 NBGB_API size_t nbgb_force_workspace_bytes(size_t N) {
     ForcePlan pl;
-    if (plan_force(N, -1, -1, pl) != NBGB_OK)
+    if (plan_force_default(N, pl) != NBGB_OK)
         return 0;
     return pl.workspace_bytes;
 }
@@ -1149,7 +1173,7 @@ NBGB_API int nbgb_force_plan(size_t N, int config, int nsplit, int *out_config, 
 // evaluates each pair once, *launches the kernels of one call.
 NBGB_API int nbgb_force_kind(size_t N, int *pairs, int *launches) {
     ForcePlan pl;
-    int rc = plan_force(N, -1, -1, pl);
+    int rc = plan_force_default(N, pl);
     if (rc != NBGB_OK)
         return rc;
     if (pairs)
@@ -1183,7 +1207,8 @@ NBGB_API int nbgb_force_ex(float *force, const float *posMass, float softeningSq
     if (((uintptr_t)force | (uintptr_t)posMass) & 15u)
         return NBGB_ERR_INVALID_ARGUMENT;
     ForcePlan pl;
-    int rc = plan_force(N, config, nsplit, pl);
+    int rc = config < 0 && nsplit == -1 ? plan_force_default(N, pl)
+                                        : plan_force(N, config, nsplit, pl);
     if (rc != NBGB_OK)
         return rc;
     if (!workspace || workspace_bytes < pl.workspace_bytes || ((uintptr_t)workspace & 255u))
@@ -1244,7 +1269,7 @@ NBGB_API float ComputeGravitation_GPU_GB300(float *force, float *posMass, float 
     void *ws = nullptr;
     if (N == 0 || !force || !posMass)
         return 0.0f;
-    if (plan_force(N, -1, -1, pl) != NBGB_OK)
+    if (plan_force_default(N, pl) != NBGB_OK)
         return 0.0f;
     ws = cached_workspace(pl.workspace_bytes);
     if (!ws)
@@ -1268,8 +1293,8 @@ NBGB_API float ComputeGravitation_GPU_GB300(float *force, float *posMass, float 
             goto done;
         if (bits == 0)
             break;
-        // Negative masses met a log-domain plan: evaluate again with rsqrt
-        // only (the reference's arithmetic accepts any sign).
+        // Negative masses met a plan that refuses them: evaluate again with
+        // one that does not (the reference's arithmetic accepts any sign).
         if (bits != NBGB_STATUS_NEGATIVE_MASS || attempt > 0 ||
             plan_force_rsqrt(N, pl) != NBGB_OK || !(ws = cached_workspace(pl.workspace_bytes)) ||
             cudaEventRecord(ev0, nullptr) != cudaSuccess)

@@ -28,6 +28,10 @@
 // a scheduler with 8 targets were 2 % slower than 2 with 12).  The next set
 // comes by cp.async, which holds no registers.
 //
+// Narrow rows (512 bodies, 4 targets a lane) serve n below kNarrowBelow, where
+// rows of 1,408 are too few pieces of work: 14,000 bodies take 64.7 us narrow
+// and 65.4 us wide, 4,096 11.0 and 15.0, 16,384 87.0 and 83.8.
+//
 // Split.  The steps of all (row, set) meetings form one line, and the host
 // cuts it into equal stretches of cost, one per resident CTA: one wave without
 // a tail at every N.  A stretch may begin and end inside a set or a row.
@@ -83,7 +87,8 @@ struct Geo {
     static constexpr int kRaw = kSet * 4;                     // floats
     static constexpr size_t kSmem = (size_t)(kHl + kRed + kSrc + kRaw) * 4;
 };
-typedef Geo<4, 11, 2, 2> G;
+typedef Geo<4, 11, 2, 2> Wide;
+typedef Geo<4, 4, 2, 2> Narrow;
 
 constexpr float kRange = 1.0995116e12f;  // 2^40
 
@@ -97,11 +102,12 @@ struct Params {
     float eps2;
     int short_ok;               // eps2 in the short forms' range
     unsigned *__restrict__ status;  // not null: refuse masses < 0
-    int ncta;
+    int ncta, parts;                // parts > 0: stretches are parts of meetings
     unsigned step[kMaxPairCtas + 1];  // first step of each CTA's stretch
 };
 
 // (row, set) meetings of the rows before b, counted from row 0.
+template <class G>
 __host__ __device__ inline long long meetings_before(int b, int nsets) {
     return (long long)b * nsets - (long long)G::kRowSets * b * (b - 1) / 2;
 }
@@ -112,7 +118,7 @@ enum : int { kEqual = 0, kShort = 1, kWide = 2, kOneSided = 3 };
 // the warp's reaction sums [3][kSet] (overwritten), times rs.  The travelling
 // reactions are added to them every kHop steps: chains of kHop KI terms
 // instead of 32 KI, so that they are no longer than the targets' chains.
-template <int MODE>
+template <class G, int MODE>
 __device__ __forceinline__ void
 meet(const ulonglong2 *src, int t0, int t1, const f2 (&nx)[G::KI], const f2 (&ny)[G::KI],
      const f2 (&nz)[G::KI], const f2 (&nm)[G::KI], f2 (&ax)[G::KI], f2 (&ay)[G::KI],
@@ -209,6 +215,7 @@ meet(const ulonglong2 *src, int t0, int t1, const f2 (&nx)[G::KI], const f2 (&ny
     }
 }
 
+template <class G>
 __global__ void __launch_bounds__(G::kThreads, G::kCtas)
     pair_kernel(const __grid_constant__ Params P) {
     constexpr int KI = G::KI, NC = G::NC, NT = G::kThreads, kSet = G::kSet;
@@ -223,14 +230,14 @@ __global__ void __launch_bounds__(G::kThreads, G::kCtas)
     const int cta = blockIdx.x;
     unsigned s = P.step[cta];
     const unsigned s_end = P.step[cta + 1];
-    const long long g0 = meetings_before(P.row0, P.nsets);
+    const long long g0 = meetings_before<G>(P.row0, P.nsets);
     int b;
     {  // the row that holds meeting s / 32
         const long long g = g0 + (s >> 5);
         int lo = P.row0, hi = P.row1 - 1;
         while (lo < hi) {
             const int mid = (lo + hi + 1) >> 1;
-            if (meetings_before(mid, P.nsets) <= g)
+            if (meetings_before<G>(mid, P.nsets) <= g)
                 lo = mid;
             else
                 hi = mid - 1;
@@ -242,10 +249,11 @@ __global__ void __launch_bounds__(G::kThreads, G::kCtas)
     grid_dependents_launch();
     grid_dependency_wait();
 
-    // a plan that refuses negative masses turns them into NaN, which every
-    // body's sum then meets
-    auto checked = [&](float4 v) {
-        if (P.status && !(v.w >= 0.f)) {
+    // A plan that refuses negative masses refuses them where a log-domain
+    // j-stream would hold log2 m (jstream_log_slot): it turns them into NaN,
+    // which every body's sum then meets.
+    auto checked = [&](float4 v, int i) {
+        if (P.status && jstream_log_slot(i >> 1) && !(v.w >= 0.f)) {
             atomicOr(P.status, NBGB_STATUS_NEGATIVE_MASS);
             v.w = __int_as_float(0x7fc00000);
         }
@@ -264,7 +272,7 @@ __global__ void __launch_bounds__(G::kThreads, G::kCtas)
         async_wait_all();
         if (tid >= kSet)
             return;
-        const float4 v = checked(raw[tid]);
+        const float4 v = checked(raw[tid], tid);  // sets are whole groups of pairs
         const float m0 = __shfl_sync(0xffffffffu, v.w, 0);
         const bool far = !(fabsf(v.x) < kRange && fabsf(v.y) < kRange && fabsf(v.z) < kRange);
         const bool mixed = !(v.w == m0 && fabsf(m0) < 1e30f);
@@ -286,7 +294,7 @@ __global__ void __launch_bounds__(G::kThreads, G::kCtas)
 
     int buf = 0;
     while (s < s_end) {
-        const long long gb = meetings_before(b, P.nsets) - g0;  // row b's first meeting
+        const long long gb = meetings_before<G>(b, P.nsets) - g0;  // row b's first meeting
         const int row_set = b * G::kRowSets;
         const unsigned seg_end =
             min(s_end, (unsigned)((gb + (P.nsets - row_set)) << 5));
@@ -297,7 +305,7 @@ __global__ void __launch_bounds__(G::kThreads, G::kCtas)
         for (int k = 0; k < KI; k++) {
             const int i = b * G::kRow + warp * 32 * KI + lane + 32 * k;
             const float4 v =
-                i < P.n ? checked(P.pm[i]) : make_float4(0.f, 0.f, 0.f, 0.f);
+                i < P.n ? checked(P.pm[i], i) : make_float4(0.f, 0.f, 0.f, 0.f);
             if (k == 0)
                 tm0 = __shfl_sync(0xffffffffu, v.w, 0);
             tfar |= !(fabsf(v.x) < kRange && fabsf(v.y) < kRange && fabsf(v.z) < kRange);
@@ -365,13 +373,13 @@ __global__ void __launch_bounds__(G::kThreads, G::kCtas)
             float *rw = rb + (size_t)warp * 3 * kSet;
             const float rs = equal ? -tm0 : 1.f;
             if (equal)
-                meet<kEqual>(src, t0, t1, nx, ny, nz, nm, ax, ay, az, eps2p, lane, rw, rs);
+                meet<G, kEqual>(src, t0, t1, nx, ny, nz, nm, ax, ay, az, eps2p, lane, rw, rs);
             else if (one_sided)
-                meet<kOneSided>(src, t0, t1, nx, ny, nz, nm, ax, ay, az, eps2p, lane, rw, rs);
+                meet<G, kOneSided>(src, t0, t1, nx, ny, nz, nm, ax, ay, az, eps2p, lane, rw, rs);
             else if (in_range)
-                meet<kShort>(src, t0, t1, nx, ny, nz, nm, ax, ay, az, eps2p, lane, rw, rs);
+                meet<G, kShort>(src, t0, t1, nx, ny, nz, nm, ax, ay, az, eps2p, lane, rw, rs);
             else
-                meet<kWide>(src, t0, t1, nx, ny, nz, nm, ax, ay, az, eps2p, lane, rw, rs);
+                meet<G, kWide>(src, t0, t1, nx, ny, nz, nm, ax, ay, az, eps2p, lane, rw, rs);
             folded_steps += t1 - t0;
             if (folded_steps + 32 > G::kFoldSteps)
                 fold();
@@ -416,62 +424,64 @@ struct ReduceParams {
     FusedIntegrate fi;  // fi.vel == nullptr: forces only
 };
 
-// kReduceBodies bodies a block, kReduceGroups x 3 (components) threads a body:
-// the body's reaction pieces (one list for the block, from the phase's earlier
+// kReduceBodies bodies a block, kGroups x 3 (components) threads a body: the
+// body's reaction pieces (one list for the block, from the phase's earlier
 // rows in row order) and then its row's target pieces form one sequence; each
 // group adds a contiguous part of it, eight loads in flight, and the parts
-// are added in order.  A latency problem, not a bandwidth one: at N = 16,384
-// there are about 35 pieces a body and 49,152 sums.
-constexpr int kReduceBodies = 32, kReduceGroups = 4;
-constexpr int kReduceThreads = 3 * kReduceBodies * kReduceGroups;
+// are added in order.  A latency problem, not a bandwidth one: at N = 3,000
+// about 50 pieces a body and 9,000 sums, where four groups took 4 us more
+// than with few pieces.
+constexpr int kReduceBodies = 32;
 
-__global__ void __launch_bounds__(kReduceThreads)
+template <class G, int kGroups>
+__global__ void __launch_bounds__(3 * kReduceBodies * kGroups)
     pair_reduce_kernel(const __grid_constant__ ReduceParams R) {
     constexpr int kSet = G::kSet, kB = kReduceBodies, kPart = kSet / kB;
     static_assert(kSet % kB == 0, "blocks are parts of a set");
-    __shared__ unsigned short first[kMaxPairRows], count[kMaxPairRows];
     __shared__ int list[kMaxPairRows + kMaxPairCtas];
-    __shared__ int n_list;
-    __shared__ float part[kReduceGroups - 1][2][3][kB], out[3][kB];
+    __shared__ int n_list, t_first, t_count;
+    __shared__ float part[kGroups - 1][2][3][kB], out[3][kB];
     const Params &P = R.p;
     const int tid = threadIdx.x, group = tid / (3 * kB), comp = (tid / kB) % 3, j = tid % kB;
     const int set = P.row0 * G::kRowSets + blockIdx.x / kPart;
     const int sub = blockIdx.x % kPart;  // part of the set
     const int b = set / G::kRowSets;
-    const long long g0 = meetings_before(P.row0, P.nsets);
-    // CTAs f..l (inclusive) whose stretches touch steps [a, e); no stretch is
-    // empty
-    auto ctas = [&](unsigned a, unsigned e, int &f, int &l) {
-        int lo = 0, hi = P.ncta - 1;  // last c with step[c] <= a
-        while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (P.step[mid] <= a)
-                lo = mid;
-            else
-                hi = mid - 1;
-        }
-        f = lo;
-        while (lo + 1 < P.ncta && P.step[lo + 1] < e)
-            lo++;
-        l = lo;
-    };
-    const int nrow = min(b, P.row1) - P.row0;  // earlier rows of this phase
-    auto meeting = [&](int r) {  // of row row0 + r with the set, in the phase
-        const int row = P.row0 + r;
-        return (int)(meetings_before(row, P.nsets) - g0) + (set - row * G::kRowSets);
-    };
-    for (int r = tid; r < nrow; r += kReduceThreads) {
-        const unsigned g = (unsigned)meeting(r);
-        int f, l;
-        ctas(g << 5, (g << 5) + 32, f, l);
-        first[r] = (unsigned short)f;
-        count[r] = (unsigned short)(l - f + 1);
-    }
-    __syncthreads();
-    if (tid < 32) {  // list of slots, in row order
+    if (tid < 32) {  // one warp finds the pieces
+        const long long g0 = meetings_before<G>(P.row0, P.nsets);
+        // CTAs f..l (inclusive) whose stretches touch steps [a, e); no stretch
+        // is empty
+        auto ctas = [&](unsigned a, unsigned e, int &f, int &l) {
+            if (P.parts) {
+                f = (int)(a >> 5) * P.parts;
+                l = (int)(e >> 5) * P.parts - 1;
+                return;
+            }
+            int lo = 0, hi = P.ncta - 1;  // last c with step[c] <= a
+            while (lo < hi) {
+                const int mid = (lo + hi + 1) >> 1;
+                if (P.step[mid] <= a)
+                    lo = mid;
+                else
+                    hi = mid - 1;
+            }
+            f = lo;
+            while (lo + 1 < P.ncta && P.step[lo + 1] < e)
+                lo++;
+            l = lo;
+        };
+        const int nrow = min(b, P.row1) - P.row0;  // earlier rows of this phase
         int base = 0;
-        for (int r0 = 0; r0 < nrow; r0 += 32) {
-            const int r = r0 + tid, c = r < nrow ? count[r] : 0;
+        for (int r0 = 0; r0 < nrow; r0 += 32) {  // list of slots, in row order
+            const int row = P.row0 + r0 + tid;
+            int slot = 0, c = 0;
+            if (r0 + tid < nrow) {
+                const int g = (int)(meetings_before<G>(row, P.nsets) - g0) +
+                              (set - row * G::kRowSets);
+                int f, l;
+                ctas((unsigned)g << 5, ((unsigned)g << 5) + 32, f, l);
+                slot = g + f;
+                c = l - f + 1;
+            }
             int incl = c;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
@@ -479,25 +489,24 @@ __global__ void __launch_bounds__(kReduceThreads)
                 if (tid >= o)
                     incl += v;
             }
-            if (c) {
-                const int slot = meeting(r) + first[r];
-                for (int q = 0; q < c; q++)
-                    list[base + incl - c + q] = slot + q;
-            }
+            for (int q = 0; q < c; q++)
+                list[base + incl - c + q] = slot + q;
             base += __shfl_sync(0xffffffffu, incl, 31);
         }
-        if (tid == 0)
+        if (tid == 0) {
+            int tf = 0, tl = -1;
+            if (b < P.row1)
+                ctas((unsigned)((meetings_before<G>(b, P.nsets) - g0) << 5),
+                     (unsigned)((meetings_before<G>(b + 1, P.nsets) - g0) << 5), tf, tl);
             n_list = base;
+            t_first = tf;
+            t_count = tl - tf + 1;
+        }
     }
     __syncthreads();
     const bool final = b < P.row1;  // else rows to come add to these bodies
-    const int nr = n_list;
-    int tf = 0, tl = -1;
-    if (final)
-        ctas((unsigned)((meetings_before(b, P.nsets) - g0) << 5),
-             (unsigned)((meetings_before(b + 1, P.nsets) - g0) << 5), tf, tl);
-    const int total = nr + (tl - tf + 1);
-    const int q0 = total * group / kReduceGroups, q1 = total * (group + 1) / kReduceGroups;
+    const int nr = n_list, tf = t_first, total = nr + t_count;
+    const int q0 = total * group / kGroups, q1 = total * (group + 1) / kGroups;
     const float *react = P.react + (size_t)comp * kSet + sub * kB + j;
     const int i = set * kSet + sub * kB + j;
     const float *tsum = P.tsum + (size_t)comp * G::kRow + (i - b * G::kRow) +
@@ -539,7 +548,7 @@ __global__ void __launch_bounds__(kReduceThreads)
     __syncthreads();
     if (group == 0) {
 #pragma unroll
-        for (int q = 0; q < kReduceGroups - 1; q++) {
+        for (int q = 0; q < kGroups - 1; q++) {
             comp_add(hi, lo, part[q][0][comp][j]);
             lo += part[q][1][comp][j];
         }
@@ -564,74 +573,116 @@ __global__ void __launch_bounds__(kReduceThreads)
 }
 
 // Cost of a step: both ways against one-sided (measured 4 : 3); a stretch has
-// at least kMinCost (no stretch is empty, and few pieces at small N).
-constexpr int kCostBoth = 4, kCostOne = 3, kMinCost = 32;
+// at least kMinCost (no stretch is empty, and few pieces at small N), a part
+// of a meeting at least kMinPartSteps steps.
+constexpr int kCostBoth = 4, kCostOne = 3, kMinCost = 32, kMinPartSteps = 4;
+constexpr size_t kLoneSmem = 120 * 1024;  // one CTA an SM
 
+template <class G>
 static int sets_of(size_t n) { return (int)((n + G::kSet - 1) / G::kSet); }
+template <class G>
 static int rows_of(size_t n) { return (int)((n + G::kRow - 1) / G::kRow); }
 
 // Cost of the rows before b, from row 0 (meetings x 32 steps).
+template <class G>
 static long long cost_before(int b, int nsets) {
-    return 32 * (kCostBoth * meetings_before(b, nsets) -
+    return 32 * (kCostBoth * meetings_before<G>(b, nsets) -
                  (long long)(kCostBoth - kCostOne) * std::min((long long)G::kRowSets * b,
                                                               (long long)nsets));
 }
 
-// The step at cost offset `at` from row0 (rows row0..row1-1), rounded up to
-// a whole step.
-static unsigned step_at(long long at, int row0, int row1, int nsets) {
-    const long long c0 = cost_before(row0, nsets), g0 = meetings_before(row0, nsets);
-    int lo = row0, hi = row1 - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (cost_before(mid, nsets) - c0 <= at)
-            lo = mid;
-        else
-            hi = mid - 1;
+// First steps of ncta stretches over rows row0..row1-1, and the end.  parts >
+// 0: every meeting is cut into that many stretches of its own.
+template <class G>
+static void cut_steps(int row0, int row1, int nsets, int ncta, int parts, unsigned *step) {
+    const unsigned end = (unsigned)((meetings_before<G>(row1, nsets) -
+                                     meetings_before<G>(row0, nsets))
+                                    << 5);
+    if (parts > 0) {
+        for (int c = 0; c <= ncta; c++)
+            step[c] = (unsigned)(c / parts * 32 + c % parts * 32 / parts);
+        return;
     }
-    long long off = at - (cost_before(lo, nsets) - c0);
-    const long long own = 32LL * kCostOne * std::min(G::kRowSets, nsets - lo * G::kRowSets);
-    long long steps = 32 * (meetings_before(lo, nsets) - g0);
-    if (off <= own)
-        steps += (off + kCostOne - 1) / kCostOne;
-    else
-        steps += own / kCostOne + (off - own + kCostBoth - 1) / kCostBoth;
-    return (unsigned)steps;
+    const long long c0 = cost_before<G>(row0, nsets), total = cost_before<G>(row1, nsets) - c0;
+    int row = row0;
+    long long steps = 0;                          // before the row
+    long long begin = 0;                          // the row's first cost
+    long long next = cost_before<G>(row + 1, nsets) - c0;
+    for (int c = 0; c < ncta; c++) {
+        const long long at = total * c / ncta;
+        while (at >= next && row + 1 < row1) {
+            steps += 32LL * (nsets - row * G::kRowSets);
+            row++;
+            begin = next;
+            next = cost_before<G>(row + 1, nsets) - c0;
+        }
+        const long long off = at - begin;
+        const long long own = 32LL * kCostOne * std::min(G::kRowSets, nsets - row * G::kRowSets);
+        step[c] = (unsigned)(steps + (off <= own ? (off + kCostOne - 1) / kCostOne
+                                                 : own / kCostOne +
+                                                       (off - own + kCostBoth - 1) / kCostBoth));
+    }
+    step[ncta] = end;
 }
 
 }  // namespace pair
 
-using pair::G;
-
 static size_t align256(size_t x) { return (x + 255) / 256 * 256; }
 
 // Reaction pieces of one phase of rows [row0, row1).
+template <class G>
 static size_t react_bytes(int row0, int row1, int nsets, int ncta) {
-    const long long g = pair::meetings_before(row1, nsets) - pair::meetings_before(row0, nsets);
+    const long long g = pair::meetings_before<G>(row1, nsets) - pair::meetings_before<G>(row0, nsets);
     return (size_t)(g + ncta) * 3 * G::kSet * 4;
 }
 
 // Rows of the phase that starts at `row`: as many as fit (0: not even one).
+template <class G>
 static int phase_end(int row, int rows, int nsets, int ncta, size_t room) {
     int end = row;
     while (end < rows && end - row < kMaxPairRows &&
-           react_bytes(row, end + 1, nsets, ncta) <= room)
+           react_bytes<G>(row, end + 1, nsets, ncta) <= room)
         end++;
     return end;
 }
 
-bool plan_pair(size_t n, int sms, size_t max_bytes, PairPlan &pl) {
-    if (n == 0 || n > kMaxBodies || sms <= 0)
-        return false;
-    pl = PairPlan{};
-    pl.n = n;
-    const int nsets = pair::sets_of(n), rows = pair::rows_of(n);
-    pl.ncta = (int)std::min<long long>(std::min(sms * G::kCtas, kMaxPairCtas),
-                                       pair::cost_before(rows, nsets) / pair::kMinCost);
+template <class G>
+static bool plan_geometry(size_t n, int sms, size_t max_bytes, PairPlan &pl) {
+    const int nsets = pair::sets_of<G>(n), rows = pair::rows_of<G>(n);
+    // Stretches of equal cost, or, for small n, every meeting in `parts` equal
+    // parts of its own, so that no stretch has two pieces.  Estimated in
+    // microseconds (narrow rows): a step takes 0.21 where a CTA has its SM to
+    // itself and 0.34 for two, a body's target piece 0.05 of the reduction, a
+    // second piece of a stretch 1.2.
+    const int slots = std::min(sms * G::kCtas, kMaxPairCtas);
+    const long long cost = pair::cost_before<G>(rows, nsets);
+    const long long meetings = pair::meetings_before<G>(rows, nsets);
+    auto estimate = [&](double steps, long long ncta) {
+        return steps * (ncta <= sms ? 0.21 : 0.34) + 0.05 * (double)ncta / rows;
+    };
+    pl.ncta = (int)std::min<long long>(slots, cost / pair::kMinCost);
+    double best = estimate((double)cost / pl.ncta / pair::kCostBoth, pl.ncta) + 1.2;
+    for (int parts = 1; parts <= 32 / pair::kMinPartSteps && meetings * parts <= slots; parts++) {
+        const double t = estimate((32 + parts - 1) / parts, meetings * parts);
+        if (rows <= kMaxPairRows && t < best) {
+            best = t;
+            pl.parts = parts;
+        }
+    }
+    if (pl.parts)
+        pl.ncta = (int)meetings * pl.parts;
+    // CTAs of this kernel start while the previous one still holds some SMs;
+    // more shared memory than two can have keeps them from sharing an SM when
+    // there is one for each
+    pl.lone = pl.ncta <= sms;
+    // eight reduction threads a body where it has many pieces (N = 6,000, 31:
+    // 16.5 us against 17.5 with four), four where their smaller blocks fit
+    // beside the pair kernel's CTAs and start early (8,192, 27: 26.6 / 27.5)
+    pl.groups8 = pl.ncta / rows + rows / 2 >= 28 && rows <= 16;
     const size_t tsum =
         align256((size_t)(std::min(rows, kMaxPairRows) + pl.ncta) * 3 * G::kRow * 4);
     const size_t carry = align256((size_t)nsets * G::kSet * 6 * 4);
-    const size_t all = align256(react_bytes(0, rows, nsets, pl.ncta));
+    const size_t all = align256(react_bytes<G>(0, rows, nsets, pl.ncta));
     // a phase of 256 MiB of pieces is about 16 ms of work; always at least
     // four rows
     size_t room = std::max((size_t)256 << 20, (size_t)4 * (nsets + pl.ncta) * 3 * G::kSet * 4);
@@ -644,7 +695,9 @@ bool plan_pair(size_t n, int sms, size_t max_bytes, PairPlan &pl) {
             return false;
     }
     const bool one = rows <= kMaxPairRows && all <= room;
-    if (!one && phase_end(0, rows, nsets, pl.ncta, room) == 0)
+    if (!one)
+        pl.parts = 0;
+    if (!one && phase_end<G>(0, rows, nsets, pl.ncta, room) == 0)
         return false;
     pl.react_bytes = one ? all : room;
     pl.off_react = 0;
@@ -654,10 +707,11 @@ bool plan_pair(size_t n, int sms, size_t max_bytes, PairPlan &pl) {
     return !max_bytes || pl.workspace_bytes <= max_bytes;
 }
 
-int launch_pair(const PairPlan &pl, float4 *force, const float4 *posMass, float eps2,
-                void *workspace, cudaStream_t st, const FusedIntegrate *fi) {
+template <class G>
+static int launch_geometry(const PairPlan &pl, float4 *force, const float4 *posMass, float eps2,
+                           void *workspace, cudaStream_t st, const FusedIntegrate *fi) {
     static_assert(sizeof(pair::ReduceParams) <= 4096, "kernel parameters");
-    const int nsets = pair::sets_of(pl.n), rows = pair::rows_of(pl.n);
+    const int nsets = pair::sets_of<G>(pl.n), rows = pair::rows_of<G>(pl.n);
     char *ws = (char *)workspace;
     pair::ReduceParams R;
     pair::Params &P = R.p;
@@ -675,32 +729,37 @@ int launch_pair(const PairPlan &pl, float4 *force, const float4 *posMass, float 
     R.fi = fi ? *fi : FusedIntegrate{};
     R.fi.js = nullptr;
     for (P.row0 = 0; P.row0 < rows; P.row0 = P.row1) {
-        P.row1 = phase_end(P.row0, rows, nsets, pl.ncta, pl.react_bytes);
+        P.row1 = phase_end<G>(P.row0, rows, nsets, pl.ncta, pl.react_bytes);
         if (P.row1 == P.row0)
             return NBGB_ERR_WORKSPACE;
         const long long total =
-            pair::cost_before(P.row1, nsets) - pair::cost_before(P.row0, nsets);
+            pair::cost_before<G>(P.row1, nsets) - pair::cost_before<G>(P.row0, nsets);
         P.ncta = (int)std::min<long long>(pl.ncta, total / pair::kMinCost);
-        for (int c = 0; c < P.ncta; c++)
-            P.step[c] = pair::step_at(total * c / P.ncta, P.row0, P.row1, nsets);
-        P.step[P.ncta] = (unsigned)((pair::meetings_before(P.row1, nsets) -
-                                     pair::meetings_before(P.row0, nsets))
-                                    << 5);
-        if (launch_dependent(pair::pair_kernel, P.ncta, G::kThreads, G::kSmem, st, P) !=
+        P.parts = pl.parts;
+        if (pl.parts)
+            P.ncta = pl.ncta;
+        pair::cut_steps<G>(P.row0, P.row1, nsets, P.ncta, pl.parts, P.step);
+        const size_t smem = pl.lone ? pair::kLoneSmem : G::kSmem;
+        const unsigned blocks =
+            (nsets - P.row0 * G::kRowSets) * (G::kSet / pair::kReduceBodies);
+        if (launch_dependent(pair::pair_kernel<G>, P.ncta, G::kThreads, smem, st, P) !=
                 cudaSuccess ||
-            launch_dependent(pair::pair_reduce_kernel,
-                             (nsets - P.row0 * G::kRowSets) * (G::kSet / pair::kReduceBodies),
-                             pair::kReduceThreads, 0, st, R) != cudaSuccess)
+            (pl.groups8 ? launch_dependent(pair::pair_reduce_kernel<G, 8>, blocks,
+                                           3 * pair::kReduceBodies * 8, 0, st, R)
+                        : launch_dependent(pair::pair_reduce_kernel<G, 4>, blocks,
+                                           3 * pair::kReduceBodies * 4, 0, st, R)) !=
+                cudaSuccess)
             return NBGB_ERR_CUDA;
     }
     return NBGB_OK;
 }
 
-int pair_launches(const PairPlan &pl) {
-    const int nsets = pair::sets_of(pl.n), rows = pair::rows_of(pl.n);
+template <class G>
+static int launches_geometry(const PairPlan &pl) {
+    const int nsets = pair::sets_of<G>(pl.n), rows = pair::rows_of<G>(pl.n);
     int k = 0;
     for (int row = 0; row < rows; k++) {
-        const int end = phase_end(row, rows, nsets, pl.ncta, pl.react_bytes);
+        const int end = phase_end<G>(row, rows, nsets, pl.ncta, pl.react_bytes);
         if (end == row)
             break;
         row = end;
@@ -708,9 +767,36 @@ int pair_launches(const PairPlan &pl) {
     return 2 * k;
 }
 
+template <class G>
+static cudaError_t prepare_geometry() {
+    return cudaFuncSetAttribute(pair::pair_kernel<G>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)std::max(G::kSmem, pair::kLoneSmem));
+}
+
+bool plan_pair(size_t n, int sms, size_t max_bytes, PairPlan &pl) {
+    if (n == 0 || n > kMaxBodies || sms <= 0)
+        return false;
+    pl = PairPlan{};
+    pl.n = n;
+    pl.narrow = n < kNarrowBelow;
+    return pl.narrow ? plan_geometry<pair::Narrow>(n, sms, max_bytes, pl)
+                     : plan_geometry<pair::Wide>(n, sms, max_bytes, pl);
+}
+
+int launch_pair(const PairPlan &pl, float4 *force, const float4 *posMass, float eps2,
+                void *workspace, cudaStream_t st, const FusedIntegrate *fi) {
+    return pl.narrow
+               ? launch_geometry<pair::Narrow>(pl, force, posMass, eps2, workspace, st, fi)
+               : launch_geometry<pair::Wide>(pl, force, posMass, eps2, workspace, st, fi);
+}
+
+int pair_launches(const PairPlan &pl) {
+    return pl.narrow ? launches_geometry<pair::Narrow>(pl) : launches_geometry<pair::Wide>(pl);
+}
+
 int pair_prepare() {
-    return cudaFuncSetAttribute(pair::pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)G::kSmem) == cudaSuccess
+    return prepare_geometry<pair::Narrow>() == cudaSuccess &&
+                   prepare_geometry<pair::Wide>() == cudaSuccess
                ? NBGB_OK
                : NBGB_ERR_CUDA;
 }

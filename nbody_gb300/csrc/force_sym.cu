@@ -317,14 +317,8 @@ int sym_block_bodies() { return sym::Geo<sym::kWideKI>::kBlock; }
 namespace {
 
 int device_sms() {
-    int dev = 0, sms = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-        sms <= 0) {
-        cudaGetLastError();  // no device: plan for a 152-SM GB300
-        sms = 152;
-    }
-    return sms;
+    const int sms = nbgb::pair_device_sms();
+    return sms > 0 ? sms : 152;  // no device: plan for a GB300
 }
 
 }  // namespace
@@ -347,7 +341,7 @@ NBGB_API int nbgb_force_newton3(float *force, const float *posMass, float soften
     if (((uintptr_t)force | (uintptr_t)posMass) & 15u)
         return NBGB_ERR_INVALID_ARGUMENT;
     nbgb::PairPlan pl;
-    if (!nbgb::plan_pair(N, device_sms(), 0, pl) || nbgb::pair_prepare() != NBGB_OK)
+    if (!nbgb::plan_pair(N, device_sms(), 0, pl))
         return NBGB_ERR_CUDA;
     if (!workspace || workspace_bytes < pl.workspace_bytes || ((uintptr_t)workspace & 255u))
         return NBGB_ERR_WORKSPACE;

@@ -20,7 +20,11 @@ int current_context(int *device, unsigned long long *ctx_id);
 // The pair kernel's decomposition and workspace layout (force_pair.cu).
 struct PairPlan {
     size_t n = 0;
+    int narrow = 0;           // geometry: narrow rows for small n
     int ncta = 0;             // stretches (resident CTAs)
+    int parts = 0;            // > 0: each meeting is so many stretches of its own
+    int lone = 0;             // one CTA an SM
+    int groups8 = 0;          // eight reduction threads a body (else four)
     size_t react_bytes = 0;   // reaction pieces of one phase, at most
     size_t off_react = 0, off_tsum = 0, off_carry = 0;
     size_t workspace_bytes = 0;
@@ -72,6 +76,9 @@ struct ForcePlan {
 };
 
 int plan_force(size_t n, int force_config, int force_nsplit, ForcePlan &pl);
+// The plan of nbgb_force: plan_force(n, -1, -1), but without a one-sided plan
+// when it evaluates pairs once.
+int plan_force_default(size_t n, ForcePlan &pl);
 // As plan_force(n, -1, -1), among configurations without log-domain pairs
 // (for masses < 0, which have no logarithm).
 int plan_force_rsqrt(size_t n, ForcePlan &pl);
@@ -112,13 +119,14 @@ int launch_force(const ForcePlan &pl, float4 *force, const float4 *posMass, cons
 // and the launches (no j-stream; fi as for launch_force, fi->js ignored).
 constexpr int kMaxPairCtas = 512;          // step table in the kernel parameters
 constexpr int kMaxPairRows = 1024;         // rows of a phase
-constexpr size_t kMinPairForce = 6144;     // force(): sizes that take the pair kernel
-constexpr size_t kMaxPairForce = (size_t)1 << 23;
+constexpr size_t kNarrowBelow = 14336;     // sizes that take the narrow rows
+constexpr size_t kMaxPairForce = (size_t)1 << 23;  // force(): larger sizes stay one-sided
 bool plan_pair(size_t n, int sms, size_t max_bytes, PairPlan &pl);
 int launch_pair(const PairPlan &pl, float4 *force, const float4 *posMass, float eps2,
                 void *workspace, cudaStream_t st, const FusedIntegrate *fi = nullptr);
 int pair_launches(const PairPlan &pl);
 int pair_prepare();  // kernel attributes of the current context
+int pair_device_sms();  // SMs of the current device, attributes set (0: no device)
 int read_and_clear_status(unsigned *bits);
 int read_status_ensemble(unsigned *bits);
 int read_status_integrate(unsigned *bits);

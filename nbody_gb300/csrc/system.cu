@@ -408,8 +408,8 @@ NBGB_API nbgb_system *nbgb_system_create(size_t N, int integrator, float softeni
     ok = ok && cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking) == cudaSuccess;
     ok = ok && cudaMalloc(&s->pm, N * 16) == cudaSuccess;
     ok = ok && cudaMalloc(&s->force, N * 16) == cudaSuccess;
-    ok = ok && cudaMalloc(&s->ws, s->plan.workspace_bytes) == cudaSuccess;
-    s->ws_bytes = s->plan.workspace_bytes;
+    s->ws_bytes = s->plan.use_pair ? s->plan.pair.workspace_bytes : s->plan.workspace_bytes;
+    ok = ok && cudaMalloc(&s->ws, s->ws_bytes) == cudaSuccess;
     if (reference_integrator(integrator)) {
         ok = ok && cudaMalloc(&s->vel, N * 16) == cudaSuccess;
         ok = ok && alloc_js2(s) == NBGB_OK;
@@ -422,7 +422,8 @@ NBGB_API nbgb_system *nbgb_system_create(size_t N, int integrator, float softeni
     }
     ok = ok && cudaMemsetAsync(s->force, 0, N * 16, s->stream) == cudaSuccess;
     // counters start at zero; every force launch leaves them at zero
-    ok = ok && cudaMemsetAsync(s->ws, 0, s->plan.workspace_bytes, s->stream) == cudaSuccess;
+    ok = ok && (s->plan.use_pair ||
+                cudaMemsetAsync(s->ws, 0, s->ws_bytes, s->stream) == cudaSuccess);
     ok = ok && cudaStreamSynchronize(s->stream) == cudaSuccess;
     if (!ok) {
         free_all(s);

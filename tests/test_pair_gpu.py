@@ -1,7 +1,7 @@
 """Forces with each pair evaluated once (nbgb_force_newton3 at every N, the
 default force at larger N) at the edges of its tiles, against FP64 and the
-one-sided kernel: sets of 128 sources, rows of 1,408 targets, the sizes where
-the default force changes kernels, phases, and the forms for equal masses and
+one-sided kernel: sets of 128 sources, rows of 512 targets (1,408
+from N = 14,336 on), phases, and the forms for equal masses and
 for positions far from the origin."""
 import numpy as np
 import pytest
@@ -31,21 +31,20 @@ def _err(out, pm, eps2, idx=None):
     return (np.linalg.norm(o[:, :3] - f, axis=1) / np.linalg.norm(f, axis=1)).max()
 
 
-@pytest.mark.parametrize("n", [2, 63, 64, 65, 127, 128, 129, 1407, 1408, 1409, 1535, 1537, 2817,
-                               6143, 6144, 6145, 7681])
+@pytest.mark.parametrize("n", [2, 63, 64, 65, 127, 128, 129, 511, 512, 513, 641, 1025, 4097, 14335,
+                               14336, 14463, 14465, 15489])
 def test_edges_of_sets_and_rows(cuda, n):
     pm, _ = nb.ic_uniform_ball(n, 40 + n, 1.0, 0.5, 1.5)
     out = _run(nb.force_newton3, pm, 1e-4)
     assert nb.last_status() == 0
     assert _err(out, pm, 1e-4) <= TOL_VS_FP64
     assert np.array_equal(out, _run(nb.force_newton3, pm, 1e-4))  # deterministic
-    if nb.force_kind(n)[0] == "pairs":
-        assert np.array_equal(_run(nb.force, pm, 1e-4), out)
+    assert np.array_equal(_run(nb.force, pm, 1e-4), out)
 
 
 def test_kinds_and_launches(cuda):
-    assert nb.force_kind(1000) == ("onesided", 2)
-    assert nb.force_kind(16384) == ("pairs", 2)
+    for n in (1, 1000, 16384):
+        assert nb.force_kind(n) == ("pairs", 2)
     kind, launches = nb.force_kind(400000)  # several phases
     assert kind == "pairs" and launches > 2 and launches % 2 == 0
 
