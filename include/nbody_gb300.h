@@ -298,7 +298,9 @@ NBGB_API void nbgb_ensemble_destroy(nbgb_ensemble *ens);
 NBGB_API size_t nbgb_ensemble_device_bytes(nbgb_ensemble *ens);
 /* Plan for N in [2^bucket, 2^(bucket+1)): variant 0..3 = (targets per
    thread, unroll) (1,8) (2,4) (1,4) (2,8); tile a power of two in 16..1024
-   bodies; j-split 1..4; variant -1 = the default rule. */
+   bodies; j-split 1..4; variant -1 = the default rule: each pair of bodies
+   evaluated once (nbgb_ensemble_slot_info then reports variant -1, tile 0),
+   for systems of up to about 290,000 bodies. */
 NBGB_API int nbgb_ensemble_set_bucket_plan(nbgb_ensemble *ens, int bucket, int variant, int jt,
                                            int nsplit);
 /* Admit a system (HOST double[n][3] x, v; float m[n]); NBGB_ERR_NO_MEMORY if
@@ -328,11 +330,13 @@ NBGB_API int nbgb_ensemble_set_substeps(nbgb_ensemble *ens, int slot, int sub);
    together fit the resident slots run side by side on their own streams. */
 NBGB_API int nbgb_ensemble_set_grid(nbgb_ensemble *ens, int ctas);
 NBGB_API int nbgb_ensemble_max_grid(nbgb_ensemble *ens);
-/* Systems admitted afterwards with N >= nmin are evaluated with the
-   Newton's-third-law kernel (as nbgb_force_newton3: each pair once, FP64
-   block-pair sums) instead of the work queue; 0 = none (the default).  Their
-   results repeat to FP64 rounding order rather than bit for bit.  The first
-   nonzero call allocates an FP64 sums arena (24 B per body of capacity). */
+/* Systems admitted afterwards with N >= nmin are evaluated with each pair
+   once, as by the default plan, whatever their bucket's plan; they move one
+   step per tick.  0 = none (the default).  The first nonzero call grows the
+   scratch arena (to 1 GiB at most).  Systems too large for it (above about
+   410,000 bodies) take block pairs with FP64 sums instead, whose results repeat
+   to FP64 rounding order rather than bit for bit (arena of 24 B per body of
+   capacity, allocated when such a system could be admitted). */
 NBGB_API int nbgb_ensemble_set_newton3_min(nbgb_ensemble *ens, size_t nmin);
 /* high != 0: the ensemble's stream gets the device's greatest priority, so
    its CTAs are dispatched ahead of other streams' pending ones (an ensemble

@@ -4,8 +4,29 @@
 // posMass array, src/nbody.h:68); running thousands of small systems that way
 // costs a launch (and a host round trip) per system per step and leaves most
 // of the GPU idle.  Here every active system's state is resident in one arena
-// and a tick advances all of them by one FP64 kick-drift-kick step with three
-// launches:
+// and a tick advances all of them by one FP64 kick-drift-kick step.
+//
+// Pair systems (the default plan): every pair of bodies evaluated once, in
+// three launches chained by programmatic dependence:
+//
+//   ens_drift      v += a dt/2; x += v dt (FP64) for moving systems, FP32
+//                  posMass of every active system; one body per thread, 32
+//                  bodies of one system per warp
+//   ens_pair       persistent CTAs take (system, row, chunk of source sets)
+//                  items from a device queue, largest first, and evaluate
+//                  them as force_pair.cu does; every partial sum has a place
+//                  of its own in the scratch arena.  Small systems are tasks
+//                  of single warps instead, four to an item: 128 targets
+//                  against all sources, one-sided, with the closing kick
+//   ens_reduce     adds each body's partial sums in a fixed order, writes the
+//                  FP32 acceleration and applies the closing v += a dt/2
+//
+// The items and the places of a system's sums depend only on its N.  Systems
+// whose scratch together exceeds the arena are evaluated in groups, one
+// ens_pair and ens_reduce each.
+//
+// Systems with an explicit bucket plan, and those too large for the arena, use
+// the one-sided work queue with three launches of its own:
 //
 //   ens_kick_drift   v += a dt/2; x += v dt (FP64) for moving systems, and
 //                    rewrite every active system's FP32 posMass and j-stream
@@ -21,10 +42,10 @@
 //   ens_kick         v += a dt/2 for moving systems
 //
 // Newton-3 systems (opt-in, nbgb_ensemble_set_newton3_min): systems of at
-// least that many bodies skip the work queue; pass 0 of each tick evaluates
-// them with the Newton's-third-law kernel (block pairs, FP64 sums; one launch
-// for all of them) and rounds their sums to FP32 accelerations.  Their
-// results repeat to FP64 rounding order (not bit for bit).
+// least that many bodies are pair systems whatever their bucket's plan, and
+// move in pass 0 of each tick only.  Those too large for the scratch arena are
+// evaluated with block pairs and FP64 sums (force_sym.cu), whose results
+// repeat to FP64 rounding order (not bit for bit).
 //
 // Sub-cycling: a system may take up to kMaxSub steps per tick (its `sub`).
 // A tick then runs passes p = 0 .. max sub - 1, each the three launches above
@@ -51,6 +72,7 @@
 
 #include "nbgb_device.cuh"
 #include "nbgb_internal.h"
+#include "nbgb_pair.cuh"
 #include "nbody_gb300.h"
 
 namespace nbgb {
@@ -84,6 +106,11 @@ struct Desc {
     int sub;             // passes of this tick the system moves in (1..kMaxSub)
     float eps2;
     double dt;
+    // pair systems
+    int pair;            // 0 no, 1 narrow rows, 2 wide rows, 3 warp tasks
+    int nsets;           // source sets
+    int ch;              // sets per item
+    long long react_off, tsum_off;  // into the scratch arena (floats)
 };
 
 struct Params {
@@ -409,6 +436,303 @@ __global__ void ens_kdk_kernel(const Desc *__restrict__ desc, const int *__restr
     }
 }
 
+// ---------------------------------------------------------------------------
+// Pair systems
+// ---------------------------------------------------------------------------
+typedef pair::Narrow Narrow;
+typedef pair::Wide Wide;
+constexpr int kPairCtaThreads = Narrow::kThreads;
+static_assert(Wide::kThreads == Narrow::kThreads && Wide::kSet == Narrow::kSet,
+              "one persistent kernel for both geometries");
+constexpr size_t kPairSmem = Wide::kSmem > Narrow::kSmem ? Wide::kSmem : Narrow::kSmem;
+constexpr int kBodyBlock = 32;  // bodies of one entry of the block map
+
+struct PairParams {
+    const Desc *__restrict__ desc;
+    const int4 *__restrict__ items;  // {system, row, chunk, 0} or {-1, first task, 0, 0}
+    const int2 *__restrict__ tasks;  // {system, tile}, four to an item ({-1, 0}: none)
+    int n_items, pass;
+    unsigned *head;                  // zeroed by ens_drift
+    const float4 *pm;
+    float *scratch;
+    float4 *acc;
+    double *x64;
+    size_t stride;
+};
+
+// Entry e of the block map: bodies 32 blk .. 32 blk + 31 of one pair system.
+__device__ __forceinline__ bool takes_part(const Desc &d, int pass) {
+    return (d.flags & kInForce) && (pass == 0 || ((d.flags & kMove) && d.sub > pass));
+}
+
+// Bodies 128 tile .. 128 tile + 127 of a small system by one warp: forces from
+// all its sources, acceleration and closing half kick.  buf: the warp's part
+// of the CTA's shared memory.  A system of up to kTaskBelow - 1 bodies is too
+// small for rows: most of a row's targets would be padding and its items
+// short (1,024 systems a tick, GB300, against rows and the one-sided queue:
+// see kTaskBelow).
+constexpr int kTaskBodies = 32 * Narrow::KI;
+
+__device__ __forceinline__ void warp_task(const PairParams &P, const Desc &d, int tile,
+                                          float *buf) {
+    constexpr int KI = Narrow::KI, kSet = Narrow::kSet;
+    static_assert(kSet == kTaskBodies, "a lane stages as many sources as it has targets");
+    const int lane = threadIdx.x & 31;
+    const float4 *pm = P.pm + d.body_off;
+    const f2 eps2p = f2_pack(d.eps2, d.eps2), zero2 = f2_pack(0.f, 0.f);
+    f2 nx[KI], ny[KI], nz[KI], nm[KI], ax[KI], ay[KI], az[KI];
+    float hi[3][KI], lo[3][KI];
+    float4 next[KI];
+#pragma unroll
+    for (int k = 0; k < KI; k++) {
+        const int i = tile * kTaskBodies + lane + 32 * k, j = lane + 32 * k;
+        const float4 v = i < d.n ? pm[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+        next[k] = j < d.n ? pm[j] : make_float4(0.f, 0.f, 0.f, 0.f);
+        nx[k] = f2_pack(-v.x, -v.x);
+        ny[k] = f2_pack(-v.y, -v.y);
+        nz[k] = f2_pack(-v.z, -v.z);
+        nm[k] = zero2;
+        ax[k] = ay[k] = az[k] = zero2;
+#pragma unroll
+        for (int c = 0; c < 3; c++)
+            hi[c][k] = lo[c][k] = 0.f;
+    }
+    for (int set = 0; set < d.nsets; set++) {
+        __syncwarp();
+#pragma unroll
+        for (int k = 0; k < KI; k++) {
+            pair::store_source<Narrow>(buf, lane + 32 * k, next[k]);
+            const int j = (set + 1) * kSet + lane + 32 * k;
+            next[k] = j < d.n ? pm[j] : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        __syncwarp();
+        pair::meet<Narrow, pair::kOneSided>(reinterpret_cast<const ulonglong2 *>(buf) + lane, 0,
+                                            32, nx, ny, nz, nm, ax, ay, az, eps2p, lane, nullptr,
+                                            1.f);
+#pragma unroll
+        for (int k = 0; k < KI; k++) {
+            float l, h;
+            f2_unpack(ax[k], l, h);
+            comp_add(hi[0][k], lo[0][k], l + h);
+            f2_unpack(ay[k], l, h);
+            comp_add(hi[1][k], lo[1][k], l + h);
+            f2_unpack(az[k], l, h);
+            comp_add(hi[2][k], lo[2][k], l + h);
+            ax[k] = ay[k] = az[k] = zero2;
+        }
+    }
+    const double kdt = 0.5 * d.dt;
+#pragma unroll
+    for (int k = 0; k < KI; k++) {
+        const int b = tile * kTaskBodies + lane + 32 * k;
+        if (b >= d.n)
+            continue;
+        const size_t i = (size_t)d.body_off + b;
+        const float a[3] = {hi[0][k] + lo[0][k], hi[1][k] + lo[1][k], hi[2][k] + lo[2][k]};
+        P.acc[i] = make_float4(a[0], a[1], a[2], 0.f);
+        if (d.flags & kMove)
+#pragma unroll
+            for (int c = 0; c < 3; c++) {
+                double *v = P.x64 + (3 + c) * P.stride + i;
+                *v = fma(widen_f32(a[c]), kdt, *v);
+            }
+    }
+}
+
+// Target piece of a row's first item: every row has at most one item more than
+// its meetings / ch, so the places of two rows never overlap.
+template <class G>
+__device__ __forceinline__ long long row_piece(int row, int nsets, int ch) {
+    return pair::meetings_before<G>(row, nsets) / ch + row;
+}
+
+// One item, in shared memory (row_stretch asks for its parts).
+struct Item {
+    const float4 *pm_;
+    float *react_, *tsum_;
+    int n_, row, set, nset, kind;    // kind: the system's Desc::pair, or 3: tasks from `row` on
+    float eps2_;
+    __device__ __forceinline__ const float4 *pm() const { return pm_; }
+    __device__ __forceinline__ int n() const { return n_; }
+    __device__ __forceinline__ float eps2() const { return eps2_; }
+    __device__ __forceinline__ int short_ok() const { return pair::eps2_short_ok(eps2_); }
+    __device__ __forceinline__ unsigned *status() const { return nullptr; }
+    __device__ __forceinline__ float *react(unsigned s) const {
+        return react_ + (size_t)(s >> 5) * (3 * Narrow::kSet);
+    }
+    __device__ __forceinline__ float *tsum() const { return tsum_; }
+};
+
+template <class G>
+__device__ __forceinline__ void set_item(Item &t, const PairParams &P, const Desc &d, int row,
+                                         int chunk) {
+    const int set = row * G::kRowSets + chunk * d.ch;
+    const long long g = pair::meetings_before<G>(row, d.nsets) + chunk * d.ch;
+    t.pm_ = P.pm + d.body_off;
+    t.react_ = P.scratch + d.react_off + g * (3 * G::kSet);
+    t.tsum_ = P.scratch + d.tsum_off +
+              (row_piece<G>(row, d.nsets, d.ch) + chunk) * (3 * G::kRow);
+    t.n_ = d.n;
+    t.row = row;
+    t.set = set;
+    t.nset = min(d.ch, d.nsets - set);
+    t.kind = d.pair;
+    t.eps2_ = d.eps2;
+}
+
+__global__ void __launch_bounds__(kPairCtaThreads, 2) ens_pair_kernel(PairParams P) {
+    extern __shared__ __align__(128) float smem_f[];
+    __shared__ Item item;
+    __shared__ int s_next[2];
+    grid_dependents_launch();
+    grid_dependency_wait();
+    for (int it = blockIdx.x, k = 0; it < P.n_items; it = s_next[k], k ^= 1) {
+        if (threadIdx.x == 0) {
+            const int next = (int)(atomicAdd(P.head, 1u) + gridDim.x);
+            const int4 v = P.items[it];
+            if (v.x < 0) {
+                item.kind = 3;
+                item.row = v.y;
+            } else if (P.desc[v.x].pair == 1) {
+                set_item<Narrow>(item, P, P.desc[v.x], v.y, v.z);
+            } else {
+                set_item<Wide>(item, P, P.desc[v.x], v.y, v.z);
+            }
+            s_next[k] = next;
+        }
+        __syncthreads();
+        if (item.kind == 3) {
+            const int warp = threadIdx.x >> 5;
+            const int2 t = P.tasks[item.row + warp];
+            if (t.x >= 0 && takes_part(P.desc[t.x], P.pass))
+                warp_task(P, P.desc[t.x], t.y, smem_f + warp * Narrow::kSource);
+            __syncthreads();
+        } else if (item.kind == 1) {
+            pair::row_stretch<Narrow, true>(item, smem_f, item.row, item.set, 0u,
+                                            32u * (unsigned)item.nset);
+        } else {
+            pair::row_stretch<Wide, false>(item, smem_f, item.row, item.set, 0u,
+                                           32u * (unsigned)item.nset);
+        }
+    }
+}
+
+// Opening half kick and drift of moving systems, FP32 positions of all;
+// zeroes the item queues.
+__global__ void __launch_bounds__(256)
+    ens_drift_kernel(const Desc *__restrict__ desc, const int2 *__restrict__ blocks, int n_blocks,
+                     double *__restrict__ x64, size_t stride, const float *__restrict__ mass,
+                     const float4 *__restrict__ acc, float4 *__restrict__ pm,
+                     unsigned *__restrict__ heads, int n_heads, int pass) {
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    grid_dependents_launch();
+    grid_dependency_wait();
+    if (q < n_heads)
+        heads[q] = 0u;
+    const int e = q / kBodyBlock;
+    if (e >= n_blocks)
+        return;
+    const int2 blk = blocks[e];
+    const Desc &d = desc[blk.x];
+    const int b = blk.y * kBodyBlock + q % kBodyBlock;
+    if (!takes_part(d, pass) || b >= d.n)
+        return;
+    const size_t i = (size_t)d.body_off + b;
+    double x = x64[i], y = x64[stride + i], z = x64[2 * stride + i];
+    const float m = mass[i];
+    if (d.flags & kMove) {
+        double u = x64[3 * stride + i], v = x64[4 * stride + i], w = x64[5 * stride + i];
+        const float4 a = acc[i];
+        const double dt = d.dt, kdt = 0.5 * dt;
+        u = fma(widen_f32(a.x), kdt, u);
+        v = fma(widen_f32(a.y), kdt, v);
+        w = fma(widen_f32(a.z), kdt, w);
+        x = fma(u, dt, x);
+        y = fma(v, dt, y);
+        z = fma(w, dt, z);
+        x64[i] = x;
+        x64[stride + i] = y;
+        x64[2 * stride + i] = z;
+        x64[3 * stride + i] = u;
+        x64[4 * stride + i] = v;
+        x64[5 * stride + i] = w;
+    }
+    pm[i] = make_float4(narrow_f64(x), narrow_f64(y), narrow_f64(z), m);
+}
+
+// One block per entry: kReduceGroups x 3 (components) threads a body add its
+// reaction pieces (rows before its own, in row order) and its row's target
+// pieces, eight loads in flight; then the acceleration and the closing half
+// kick.
+constexpr int kReduceGroups = 4;
+constexpr int kReduceThreads = 3 * kBodyBlock * kReduceGroups;
+
+template <class G>
+__device__ __forceinline__ void reduce_entry(const Desc &d, int blk, const float *scratch,
+                                             double *x64, size_t stride, float4 *acc) {
+    constexpr int kB = kBodyBlock, kSet = G::kSet;
+    __shared__ float part[kReduceGroups - 1][2][3][kB], out[3][kB];
+    const int tid = threadIdx.x, group = tid / (3 * kB), comp = (tid / kB) % 3, j = tid % kB;
+    const int i = blk * kB + j, set = blk * kB / kSet, b = set / G::kRowSets;
+    const int nt = (d.nsets - b * G::kRowSets + d.ch - 1) / d.ch, total = b + nt;
+    const int q0 = total * group / kReduceGroups, q1 = total * (group + 1) / kReduceGroups;
+    const float *react = scratch + d.react_off + (size_t)comp * kSet + (i - set * kSet);
+    const float *tsum = scratch + d.tsum_off + (size_t)comp * G::kRow + (i - b * G::kRow) +
+                        row_piece<G>(b, d.nsets, d.ch) * (3 * G::kRow);
+    auto piece = [&](int q) {
+        return q < b ? react + (pair::meetings_before<G>(q, d.nsets) + set - q * G::kRowSets) *
+                                   (3 * kSet)
+                     : tsum + (long long)(q - b) * (3 * G::kRow);
+    };
+    float hi = 0.f, lo = 0.f;
+    for (int q = q0; q < q1; q += 8) {
+        float v[8];
+#pragma unroll
+        for (int u = 0; u < 8; u++)
+            v[u] = q + u < q1 ? __ldcs(piece(q + u)) : 0.f;
+#pragma unroll
+        for (int u = 0; u < 8; u++)
+            comp_add(hi, lo, v[u]);
+    }
+    if (group) {
+        part[group - 1][0][comp][j] = hi;
+        part[group - 1][1][comp][j] = lo;
+    }
+    __syncthreads();
+    if (group == 0) {
+#pragma unroll
+        for (int q = 0; q < kReduceGroups - 1; q++) {
+            comp_add(hi, lo, part[q][0][comp][j]);
+            lo += part[q][1][comp][j];
+        }
+        const float a = hi + lo;
+        out[comp][j] = a;
+        if (i < d.n && (d.flags & kMove)) {
+            double *v = x64 + (3 + comp) * stride + d.body_off + i;
+            *v = fma(widen_f32(a), 0.5 * d.dt, *v);
+        }
+    }
+    __syncthreads();
+    if (tid < kB && i < d.n)
+        acc[(size_t)d.body_off + i] = make_float4(out[0][j], out[1][j], out[2][j], 0.f);
+}
+
+__global__ void __launch_bounds__(kReduceThreads)
+    ens_reduce_kernel(const Desc *__restrict__ desc, const int2 *__restrict__ blocks,
+                      const float *__restrict__ scratch, double *__restrict__ x64, size_t stride,
+                      float4 *__restrict__ acc, int pass) {
+    grid_dependents_launch();
+    grid_dependency_wait();
+    const int2 blk = blocks[blockIdx.x];
+    const Desc &d = desc[blk.x];
+    if (!takes_part(d, pass))
+        return;
+    if (d.pair == 1)
+        reduce_entry<Narrow>(d, blk.y, scratch, x64, stride, acc);
+    else
+        reduce_entry<Wide>(d, blk.y, scratch, x64, stride, acc);
+}
+
 static NBGB_STATUS_READER(read_status_ens)
 
 }  // namespace ens
@@ -494,7 +818,12 @@ struct HostSys {
     long long steps_done = 0;
     bool log_mass = false;  // every mass >= 0: log-domain pairs (kLogMass)
     int sub = 1;            // steps per tick (1..kMaxSub)
-    bool n3 = false;        // Newton-3 system (no work items)
+    bool n3 = false;        // Newton-3 system
+    bool sym = false;       // Newton-3 system too large for pair items
+    int pair = 0;           // pair system: 1 narrow rows, 2 wide rows, 3 warp tasks
+    int nsets = 0, ch = 0, rows = 0;
+    size_t react_len = 0, scratch_len = 0;  // floats
+    size_t scratch_off = 0;                 // within its group's scratch
     size_t acc_off = 0, acc_len = 0;  // its FP64 sums ([3][npad] doubles)
 };
 
@@ -504,6 +833,85 @@ inline int sub_eff(const HostSys &h) {
         return 1;  // the initial-force pass; Newton-3 systems run in pass 0 only
     return (int)std::min<long long>(h.sub, h.steps_left);
 }
+
+// Items of a pair system are whole source sets of one row: few enough that an
+// item's start-up (2-3 us) is small beside its steps (11 us a set with narrow
+// rows, 30 us with wide ones), many enough that one system alone fills the
+// GPU.  Depends on n only, as does the geometry: rows of 512 targets below
+// 8,192 bodies (more, smaller items, less padding), 1,408 above.
+int sets_per_item(size_t n) {
+    if (n < 8192)
+        return n < 2048 ? 4 : 2;
+    int ch = 1;
+    for (size_t m = 16384; m <= n && ch < 32; m *= 2)
+        ch *= 2;
+    return ch;
+}
+
+template <class G>
+void pair_shape(size_t n, HostSys &h) {
+    h.nsets = (int)((n + G::kSet - 1) / G::kSet);
+    h.rows = (int)((n + G::kRow - 1) / G::kRow);
+    h.ch = sets_per_item(n);
+    const size_t meetings = (size_t)nbgb::pair::meetings_before<G>(h.rows, h.nsets);
+    h.react_len = meetings * 3 * G::kSet;
+    h.scratch_len = h.react_len + (meetings / h.ch + h.rows) * 3 * G::kRow;  // row_piece
+}
+
+// Sizes evaluated by warp tasks.  Microseconds a tick of 1,024 systems (one
+// system), tasks / rows / the one-sided queue's tuned plan: N = 91 29 / 52 /
+// 46 (17 / 19 / 21), 362 104 / 166 / 124 (26 / 19 / 32), 724 304 / 403 / 309
+// (38 / 20 / 43), 1,280 728 / 809 / 1,011 (57 / 39 / 102): above the line rows
+// are little slower for many systems and much faster for few.
+constexpr size_t kTaskBelow = 1024;
+
+// The pair plan of n bodies if its scratch is at most max_floats.
+bool pair_plan(size_t n, size_t max_floats, HostSys &h) {
+    HostSys t;
+    if (n < kTaskBelow) {
+        h.pair = 3;
+        h.nsets = (int)((n + nbgb::ens::Narrow::kSet - 1) / nbgb::ens::Narrow::kSet);
+        return true;
+    }
+    if (n < 8192)
+        pair_shape<nbgb::ens::Narrow>(n, t);
+    else
+        pair_shape<nbgb::ens::Wide>(n, t);
+    if (t.scratch_len > max_floats)
+        return false;
+    h.pair = n < 8192 ? 1 : 2;
+    h.nsets = t.nsets;
+    h.rows = t.rows;
+    h.ch = t.ch;
+    h.react_len = t.react_len;
+    h.scratch_len = t.scratch_len;
+    return true;
+}
+
+// Scratch arena (floats): what the largest pair system of max_bodies needs,
+// at most `limit`.  Systems that need more than the limit are not pair
+// systems: a rule on n alone.
+constexpr size_t kPairScratch = ((size_t)512 << 20) / 4;     // to about 290,000 bodies
+constexpr size_t kPairScratchN3 = ((size_t)1 << 30) / 4;     // Newton-3: to about 410,000
+size_t scratch_for(size_t max_bodies, size_t limit) {
+    size_t most = 0;
+    for (size_t n : {(size_t)8191, (size_t)16383, (size_t)32767, (size_t)65535,
+                     (size_t)131071, (size_t)262143, max_bodies}) {
+        HostSys h;
+        n = std::min(n, max_bodies);
+        if (pair_plan(n, ~(size_t)0, h))
+            most = std::max(most, h.scratch_len);
+    }
+    return std::min(most, limit);
+}
+
+// Pair systems evaluated together: their items and body blocks, and the
+// first item of each pass (items sorted by sub).
+struct PairGroup {
+    int first = 0, n = 0;
+    int block0 = 0, nblocks = 0;
+    int pass_first[nbgb::ens::kMaxSub];
+};
 
 // Per-N-bucket plan: bucket b covers N in [2^b, 2^(b+1)).
 struct BucketPlan {
@@ -544,6 +952,19 @@ struct nbgb_ensemble {
     RangeAlloc a_acc;
     nbgb::SymSystem *d_sym = nullptr, *h_sym = nullptr;
     int n_sym = 0;
+    // pair systems
+    float *scratch = nullptr;             // partial sums of one group
+    size_t scratch_cap = 0, scratch_limit = kPairScratch;  // floats
+    char *d_lists = nullptr, *h_lists = nullptr;  // items, tasks, blocks
+    int4 *d_pitems = nullptr, *h_pitems = nullptr;
+    size_t pitems_cap = 0;
+    int2 *d_blocks = nullptr, *h_blocks = nullptr;
+    size_t blocks_cap = 0;
+    unsigned *heads = nullptr;            // one queue per group
+    int2 *d_tasks = nullptr, *h_tasks = nullptr;
+    size_t tasks_cap = 0;
+    int n_blocks = 0, n_tasks = 0;
+    std::vector<PairGroup> groups;
     int pass_first[nbgb::ens::kMaxSub];   // first item of pass p (items sorted by sub)
     bool dirty = true;
     cudaGraphExec_t graph = nullptr;
@@ -564,15 +985,14 @@ int bucket_of(int n) {
     return b;
 }
 
-// Default per-bucket rule (used until an autotuner sets bucket plans): small
-// systems 1 target per thread and 128-body tiles, larger ones 2 per thread
-// with tiles up to 512 bodies; no j-split below 16 i-blocks.
+// Default per-bucket rule: pair systems (pair_plan); the ones too large for
+// its scratch 2 targets per thread and 512-body tiles.
 void choose_plan(nbgb_ensemble *e, int n, HostSys &h) {
     const BucketPlan &bp = e->bucket[bucket_of(n)];
     int variant = bp.variant, jt = bp.jt, nsplit = bp.nsplit;
     if (variant < 0) {
-        variant = n <= 1024 ? 0 : 1;
-        jt = n <= 512 ? 128 : (n <= 4096 ? 256 : 512);
+        variant = 1;
+        jt = 512;
         nsplit = 1;
     }
     const int bi = nbgb::ens::kThreads * ((variant == 0 || variant == 2) ? 1 : 2);
@@ -603,6 +1023,114 @@ void fill_desc(nbgb_ensemble *e, int slot, Desc &d) {
     d.sub = h.used ? sub_eff(h) : 1;
     d.eps2 = e->eps2;
     d.dt = h.dt;
+    d.pair = h.pair;
+    d.nsets = h.nsets;
+    d.ch = h.ch;
+    d.react_off = (long long)h.scratch_off;
+    d.tsum_off = (long long)(h.scratch_off + h.react_len);
+}
+
+// Groups, items and body blocks of this tick's pair systems (before the
+// descriptors are filled: scratch places are set here).
+int rebuild_pairs(nbgb_ensemble *e) {
+    struct It {
+        int4 v;
+        int cost, sub;
+    };
+    std::vector<It> items;
+    size_t used = 0, n_items = 0;
+    e->n_blocks = 0;
+    e->groups.clear();
+    auto close_group = [&]() -> int {
+        PairGroup &g = e->groups.back();
+        std::stable_sort(items.begin(), items.end(), [](const It &a, const It &b) {
+            return a.sub != b.sub ? a.sub < b.sub : a.cost > b.cost;
+        });
+        if (n_items + items.size() > e->pitems_cap)
+            return NBGB_ERR_NO_MEMORY;
+        g.first = (int)n_items;
+        g.n = (int)items.size();
+        g.nblocks = e->n_blocks - g.block0;
+        for (const It &it : items)
+            e->h_pitems[n_items++] = it.v;
+        int k = 0;
+        for (int p = 0; p < nbgb::ens::kMaxSub; p++) {
+            while (p > 0 && k < g.n && items[k].sub <= p)
+                k++;
+            g.pass_first[p] = k;
+        }
+        for (const It &it : items)
+            e->n_pass = std::max(e->n_pass, it.sub);
+        items.clear();
+        used = 0;
+        return NBGB_OK;
+    };
+    auto add_blocks = [&](int s) {
+        const int nblk = (e->sys[s].n + nbgb::ens::kBodyBlock - 1) / nbgb::ens::kBodyBlock;
+        if ((size_t)(e->n_blocks + nblk) > e->blocks_cap)
+            return false;
+        for (int k = 0; k < nblk; k++)
+            e->h_blocks[e->n_blocks++] = make_int2(s, k);
+        return true;
+    };
+    // warp tasks, four of one sub and like length to an item, in the first
+    // group; their bodies need no reduction
+    std::vector<It> tasks;
+    for (int s = 0; s < e->max_systems; s++) {
+        const HostSys &h = e->sys[s];
+        if (!h.used || h.pair != 3 || !(h.steps_left > 0 || !h.started))
+            continue;
+        for (int t = 0; t < h.nsets; t++)  // as many tiles as sets
+            tasks.push_back(It{make_int4(s, t, 0, 0), h.nsets, sub_eff(h)});
+        if (!add_blocks(s))
+            return NBGB_ERR_NO_MEMORY;
+    }
+    std::stable_sort(tasks.begin(), tasks.end(), [](const It &a, const It &b) {
+        return a.sub != b.sub ? a.sub < b.sub : a.cost > b.cost;
+    });
+    e->n_tasks = 0;
+    if (!tasks.empty()) {
+        e->groups.emplace_back();
+        e->groups.back().block0 = e->n_blocks;
+    }
+    for (size_t k = 0; k < tasks.size();) {
+        if ((size_t)e->n_tasks + 4 > e->tasks_cap)
+            return NBGB_ERR_NO_MEMORY;
+        const int sub = tasks[k].sub;
+        // a one-sided step of four warps costs three quarters of one of a row
+        items.push_back(It{make_int4(-1, e->n_tasks, 0, 0),
+                           (tasks[k].cost * nbgb::ens::Narrow::KI * 3 + 3) / 4, sub});
+        for (int q = 0; q < 4; q++, e->n_tasks++) {
+            const bool have = k < tasks.size() && tasks[k].sub == sub;
+            e->h_tasks[e->n_tasks] =
+                have ? make_int2(tasks[k].v.x, tasks[k].v.y) : make_int2(-1, 0);
+            k += have;
+        }
+    }
+    for (int s = 0; s < e->max_systems; s++) {
+        HostSys &h = e->sys[s];
+        if (!h.used || !h.pair || h.pair == 3 || !(h.steps_left > 0 || !h.started))
+            continue;
+        if (e->groups.empty() || used + h.scratch_len > e->scratch_cap) {
+            if (!e->groups.empty() && close_group() != NBGB_OK)
+                return NBGB_ERR_NO_MEMORY;
+            e->groups.emplace_back();
+            e->groups.back().block0 = e->n_blocks;
+        }
+        h.scratch_off = used;
+        used += (h.scratch_len + 63) / 64 * 64;
+        const int row_sets = h.pair == 1 ? nbgb::ens::Narrow::kRowSets : nbgb::ens::Wide::kRowSets;
+        const int ki = h.pair == 1 ? nbgb::ens::Narrow::KI : nbgb::ens::Wide::KI;
+        for (int row = 0; row < h.rows; row++)
+            for (int set = row * row_sets, c = 0; set < h.nsets; set += h.ch, c++)
+                items.push_back(It{make_int4(s, row, c, 0),
+                                   std::min(h.ch, h.nsets - set) * ki, sub_eff(h)});
+        if (!add_blocks(s))
+            return NBGB_ERR_NO_MEMORY;
+    }
+    if (!e->groups.empty() && close_group() != NBGB_OK)
+        return NBGB_ERR_NO_MEMORY;
+    return NBGB_OK;
 }
 
 // Rebuild descriptors, the j-stream slot map and the largest-first item list.
@@ -617,6 +1145,10 @@ int rebuild(nbgb_ensemble *e) {
         int sub;
     };
     std::vector<It> items;
+    e->n_pass = 1;
+    const int prc = rebuild_pairs(e);
+    if (prc != NBGB_OK)
+        return prc;
     for (int s = 0; s < e->max_systems; s++) {
         fill_desc(e, s, e->h_desc[s]);
         const HostSys &h = e->sys[s];
@@ -627,8 +1159,8 @@ int rebuild(nbgb_ensemble *e) {
             e->h_desc[s].flags = 0;
             continue;
         }
-        if (h.n3)
-            continue;  // evaluated by the Newton-3 launch
+        if (h.sym || h.pair)
+            continue;  // evaluated by launches of their own
         const int bi = nbgb::ens::kThreads * ((h.variant == 0 || h.variant == 2) ? 1 : 2);
         for (int b = 0; b < h.nblocks; b++)
             for (int r = 0; r < h.nsplit; r++) {
@@ -648,7 +1180,6 @@ int rebuild(nbgb_ensemble *e) {
     for (size_t k = 0; k < items.size(); k++)
         e->h_items[k] = items[k].v;
     e->n_items = (int)items.size();
-    e->n_pass = 1;
     for (const It &it : items)
         e->n_pass = std::max(e->n_pass, it.sub);
     for (int p = 0; p < nbgb::ens::kMaxSub; p++) {
@@ -678,7 +1209,7 @@ int rebuild(nbgb_ensemble *e) {
     const int sb = nbgb::sym_block_bodies();
     for (int s = 0; s < e->max_systems; s++) {
         const HostSys &h = e->sys[s];
-        if (!h.used || !h.n3 || !(h.steps_left > 0 || !h.started))
+        if (!h.used || !h.sym || !(h.steps_left > 0 || !h.started))
             continue;
         nbgb::SymSystem &t = e->h_sym[e->n_sym++];
         t.pm = e->pm + h.body_off;
@@ -693,6 +1224,15 @@ int rebuild(nbgb_ensemble *e) {
         pairs += (long long)t.nblocks * (t.nblocks + 1) / 2;
     }
     cudaStream_t st = e->stream;
+    if (!e->groups.empty() &&
+        (cudaMemcpyAsync(e->d_pitems, e->h_pitems,
+                         sizeof(int4) * (e->groups.back().first + e->groups.back().n),
+                         cudaMemcpyHostToDevice, st) != cudaSuccess ||
+         (e->n_tasks && cudaMemcpyAsync(e->d_tasks, e->h_tasks, sizeof(int2) * e->n_tasks,
+                                        cudaMemcpyHostToDevice, st) != cudaSuccess) ||
+         cudaMemcpyAsync(e->d_blocks, e->h_blocks, sizeof(int2) * e->n_blocks,
+                         cudaMemcpyHostToDevice, st) != cudaSuccess))
+        return NBGB_ERR_CUDA;
     if (e->n_sym && cudaMemcpyAsync(e->d_sym, e->h_sym, sizeof(nbgb::SymSystem) * e->n_sym,
                                     cudaMemcpyHostToDevice, st) != cudaSuccess)
         return NBGB_ERR_CUDA;
@@ -712,15 +1252,58 @@ int rebuild(nbgb_ensemble *e) {
     return NBGB_OK;
 }
 
+// The pair systems that move in this pass (all of them in pass 0).
+int launch_pair_pass(nbgb_ensemble *e, int pass) {
+    cudaStream_t st = e->stream;
+    const int n_groups = (int)e->groups.size();
+    const int work = std::max(e->n_blocks * nbgb::ens::kBodyBlock, n_groups);
+    bool ok = nbgb::launch_dependent_n(nbgb::ens::ens_drift_kernel, (work + 255) / 256, 256, 0, st,
+                                       e->d_desc, e->d_blocks, e->n_blocks, e->x64, e->max_bodies,
+                                       e->mass, e->acc, e->pm, e->heads, n_groups,
+                                       pass) == cudaSuccess;
+    for (int k = 0; k < n_groups && ok; k++) {
+        const PairGroup &g = e->groups[k];
+        const int first = g.pass_first[pass], n = g.n - first;
+        if (n <= 0)
+            continue;
+        nbgb::ens::PairParams P;
+        P.desc = e->d_desc;
+        P.items = e->d_pitems + g.first + first;
+        P.tasks = e->d_tasks;
+        P.n_items = n;
+        P.pass = pass;
+        P.head = e->heads + k;
+        P.pm = e->pm;
+        P.scratch = e->scratch;
+        P.acc = e->acc;
+        P.x64 = e->x64;
+        P.stride = e->max_bodies;
+        ok = nbgb::launch_dependent_n(nbgb::ens::ens_pair_kernel, std::min(e->grid, n),
+                                      nbgb::ens::kPairCtaThreads, nbgb::ens::kPairSmem, st,
+                                      P) == cudaSuccess &&
+             (g.nblocks == 0 ||
+              nbgb::launch_dependent_n(nbgb::ens::ens_reduce_kernel, g.nblocks,
+                                       nbgb::ens::kReduceThreads, 0, st, e->d_desc,
+                                       e->d_blocks + g.block0, e->scratch, e->x64, e->max_bodies,
+                                       e->acc, pass) == cudaSuccess);
+    }
+    return ok ? NBGB_OK : NBGB_ERR_CUDA;
+}
+
 int launch_tick(nbgb_ensemble *e) {
     cudaStream_t st = e->stream;
     const int tb = 256;
     const int nb = std::max(1, (e->n_slots + tb - 1) / tb);
     for (int pass = 0; pass < e->n_pass; pass++) {
+        if (!e->groups.empty()) {
+            const int rc = launch_pair_pass(e, pass);
+            if (rc != NBGB_OK)
+                return rc;
+        }
         const int first = e->pass_first[pass];
         const int n_items = e->n_items - first;
-        if (pass > 0 && n_items <= 0)
-            break;
+        if (n_items <= 0 && (pass > 0 || e->n_sym == 0))
+            continue;
         nbgb::ens::ens_kdk_kernel<<<nb, tb, 0, st>>>(e->d_desc, e->d_slot_sys, e->n_slots,
                                                      e->x64, e->max_bodies, e->mass, e->acc,
                                                      e->pm, e->js, 0, pass);
@@ -766,6 +1349,10 @@ void free_ens(nbgb_ensemble *e) {
     cudaFree(e->d_items);
     cudaFree(e->d_slot_sys);
     cudaFree(e->acc64);
+    cudaFree(e->scratch);
+    cudaFree(e->d_lists);
+    cudaFree(e->heads);
+    cudaFreeHost(e->h_lists);
     cudaFree(e->d_sym);
     cudaFreeHost(e->h_sym);
     cudaFreeHost(e->h_desc);
@@ -780,7 +1367,8 @@ void free_ens(nbgb_ensemble *e) {
 extern "C" {
 
 // Capacity: max_bodies bodies in total, max_systems concurrent systems.  The
-// device arena is allocated once here (about 250 B per body of capacity,
+// device arena is allocated once here (about 250 B per body of capacity plus
+// the pair systems' scratch, up to 512 MiB,
 // including partials for j-splits of up to 4); admission never allocates.
 NBGB_API nbgb_ensemble *nbgb_ensemble_create(size_t max_bodies, int max_systems,
                                              float softeningSquared) {
@@ -802,6 +1390,13 @@ NBGB_API nbgb_ensemble *nbgb_ensemble_create(size_t max_bodies, int max_systems,
     e->part_cap = 8 * (max_bodies + (size_t)max_systems * 512);
     e->cnt_cap = max_bodies / 256 + (size_t)max_systems + 1;
     e->items_cap = 4 * (max_bodies / 256 + (size_t)max_systems) + 64;
+    // pair items (at most 0.05 a body, where sets_per_item is about to grow,
+    // and four for the smallest systems) and 32-body blocks
+    e->scratch_cap = scratch_for(max_bodies, kPairScratch);
+    e->pitems_cap = max_bodies / 12 + 4 * (size_t)max_systems + 64;
+    e->tasks_cap = max_bodies / nbgb::ens::kTaskBodies + (size_t)max_systems +
+                   4 * (size_t)nbgb::ens::kMaxSub;
+    e->blocks_cap = max_bodies / nbgb::ens::kBodyBlock + (size_t)max_systems + 1;
     e->sys.assign(max_systems, HostSys());
     e->a_body.init(max_bodies);
     e->a_js.init(e->js_cap);
@@ -820,6 +1415,22 @@ NBGB_API nbgb_ensemble *nbgb_ensemble_create(size_t max_bodies, int max_systems,
     ok = ok && cudaMalloc(&e->d_desc, sizeof(Desc) * max_systems) == cudaSuccess;
     ok = ok && cudaMalloc(&e->d_items, sizeof(int4) * e->items_cap) == cudaSuccess;
     ok = ok && cudaMalloc(&e->d_slot_sys, sizeof(int) * (e->js_cap / 2)) == cudaSuccess;
+    ok = ok && cudaMalloc(&e->scratch, e->scratch_cap * 4) == cudaSuccess;
+    const size_t off_tasks = sizeof(int4) * e->pitems_cap;
+    const size_t off_blocks = off_tasks + sizeof(int2) * e->tasks_cap;
+    const size_t list_bytes = off_blocks + sizeof(int2) * e->blocks_cap;
+    ok = ok && cudaMalloc(&e->d_lists, list_bytes) == cudaSuccess;
+    ok = ok && cudaMallocHost(&e->h_lists, list_bytes) == cudaSuccess;
+    e->d_pitems = (int4 *)e->d_lists;
+    e->h_pitems = (int4 *)e->h_lists;
+    e->d_tasks = (int2 *)(e->d_lists + off_tasks);
+    e->h_tasks = (int2 *)(e->h_lists + off_tasks);
+    e->d_blocks = (int2 *)(e->d_lists + off_blocks);
+    e->h_blocks = (int2 *)(e->h_lists + off_blocks);
+    ok = ok && cudaMalloc(&e->heads, 4 * ((size_t)max_systems + 1)) == cudaSuccess;
+    ok = ok && cudaFuncSetAttribute(nbgb::ens::ens_pair_kernel,
+                                    cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)nbgb::ens::kPairSmem) == cudaSuccess;
     ok = ok && cudaMallocHost(&e->h_desc, sizeof(Desc) * max_systems) == cudaSuccess;
     ok = ok && cudaMallocHost(&e->h_items, sizeof(int4) * e->items_cap) == cudaSuccess;
     ok = ok && cudaMallocHost(&e->h_slot_sys, sizeof(int) * (e->js_cap / 2)) == cudaSuccess;
@@ -845,7 +1456,7 @@ NBGB_API nbgb_ensemble *nbgb_ensemble_create(size_t max_bodies, int max_systems,
     e->grid = sms * occ;
     e->grid_max = e->grid;
     e->bytes_total = max_bodies * (6 * 8 + 4 + 16 + 16) + e->js_cap * 16 + e->part_cap * 16 +
-                     e->cnt_cap * 4;
+                     e->cnt_cap * 4 + e->scratch_cap * 4;
     return e;
 }
 
@@ -897,7 +1508,12 @@ NBGB_API int nbgb_ensemble_add(nbgb_ensemble *e, const double *pos3, const doubl
     choose_plan(e, (int)n, h);
     h.body_len = n;
     h.n3 = e->n3_min > 0 && n >= e->n3_min;
-    if (h.n3) {  // j-stream padded to whole Newton-3 blocks, FP64 sums
+    if (h.n3 || e->bucket[bucket_of((int)n)].variant < 0)
+        pair_plan(n, h.n3 ? kPairScratchN3 : kPairScratch, h);
+    h.sym = h.n3 && !h.pair;
+    if (h.pair) {  // scratch is placed tick by tick
+        h.js_len = h.part_len = h.cnt_len = 0;
+    } else if (h.sym) {  // j-stream padded to whole Newton-3 blocks, FP64 sums
         const size_t sb = (size_t)nbgb::sym_block_bodies();
         h.js_len = (n + sb - 1) / sb * sb;
         h.acc_len = 3 * h.js_len;
@@ -942,7 +1558,7 @@ NBGB_API int nbgb_ensemble_add(nbgb_ensemble *e, const double *pos3, const doubl
     h.dt = dt;
     h.steps_left = steps;
     h.used = true;
-    h.log_mass = !h.n3;  // the Newton-3 kernel reads plain masses
+    h.log_mass = !h.sym && !h.pair;  // the other kernels read plain masses
     for (size_t i = 0; i < n && h.log_mass; i++)
         h.log_mass = mass[i] >= 0.f;
     // upload state (SoA FP64, masses), zero the j-stream range
@@ -959,7 +1575,8 @@ NBGB_API int nbgb_ensemble_add(nbgb_ensemble *e, const double *pos3, const doubl
     }
     if (cudaMemcpyAsync(e->mass + ob, mass, n * sizeof(float), cudaMemcpyHostToDevice, st) !=
             cudaSuccess ||
-        cudaMemsetAsync(e->js + oj, 0, h.js_len * 16, st) != cudaSuccess ||
+        (h.js_len &&
+         cudaMemsetAsync(e->js + oj, 0, h.js_len * 16, st) != cudaSuccess) ||
         (h.acc_len &&
          cudaMemsetAsync(e->acc64 + oa, 0, h.acc_len * sizeof(double), st) != cudaSuccess) ||
         cudaStreamSynchronize(st) != cudaSuccess)
@@ -1115,9 +1732,9 @@ NBGB_API int nbgb_ensemble_slot_info(nbgb_ensemble *e, int slot, long long *info
     info6[0] = h.used ? h.n : 0;
     info6[1] = h.steps_done;
     info6[2] = h.steps_left;
-    info6[3] = h.variant;
-    info6[4] = h.jt;
-    info6[5] = h.nsplit;
+    info6[3] = h.pair ? -1 : h.variant;  // pair systems: variant -1, no tile
+    info6[4] = h.pair ? 0 : h.jt;
+    info6[5] = h.pair ? 1 : h.nsplit;
     return NBGB_OK;
 }
 
@@ -1156,13 +1773,28 @@ NBGB_API int nbgb_ensemble_set_priority(nbgb_ensemble *e, int high) {
     return NBGB_OK;
 }
 
-// Systems admitted from now on with at least nmin bodies use the Newton-3
-// kernel (0: none).  The first nonzero call allocates the FP64 sums arena
-// (24 B per body of capacity).
+// Systems admitted from now on with at least nmin bodies are pair systems
+// whatever their bucket's plan (0: none).  The first nonzero call grows the
+// scratch arena, and where a system could still exceed it allocates the FP64
+// sums arena of the block-pair kernel (24 B per body of capacity).
 NBGB_API int nbgb_ensemble_set_newton3_min(nbgb_ensemble *e, size_t nmin) {
     if (!e)
         return NBGB_ERR_INVALID_ARGUMENT;
-    if (nmin > 0 && !e->acc64) {
+    const size_t need = scratch_for(e->max_bodies, kPairScratchN3);
+    if (nmin > 0 && need > e->scratch_cap) {  // larger pair systems
+        float *p = nullptr;
+        if (cudaStreamSynchronize(e->stream) != cudaSuccess)
+            return NBGB_ERR_CUDA;
+        if (cudaMalloc(&p, need * 4) != cudaSuccess)
+            return NBGB_ERR_NO_MEMORY;
+        cudaFree(e->scratch);
+        e->bytes_total += (need - e->scratch_cap) * 4;
+        e->scratch = p;
+        e->scratch_cap = need;
+        e->dirty = true;  // the captured tick holds the old arena
+    }
+    HostSys largest;
+    if (nmin > 0 && !e->acc64 && !pair_plan(e->max_bodies, kPairScratchN3, largest)) {
         const size_t cap = 3 * (e->max_bodies + (size_t)e->max_systems *
                                                     (size_t)nbgb::sym_block_bodies());
         if (cudaMalloc(&e->acc64, cap * sizeof(double)) != cudaSuccess) {

@@ -36,9 +36,9 @@ struct PairPlan {
 // Launches a kernel with programmatic dependence on the stream's previous
 // kernel: its CTAs may start early, so the kernel must call
 // grid_dependency_wait() before it touches global memory.
-template <typename Args>
-cudaError_t launch_dependent(void (*kernel)(Args), unsigned grid, unsigned block, size_t smem,
-                             cudaStream_t st, const Args &args) {
+template <typename... Args, typename... Vals>
+cudaError_t launch_dependent_n(void (*kernel)(Args...), unsigned grid, unsigned block, size_t smem,
+                               cudaStream_t st, const Vals &...vals) {
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
@@ -49,7 +49,12 @@ cudaError_t launch_dependent(void (*kernel)(Args), unsigned grid, unsigned block
     cfg.stream = st;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, args);
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<Args>(vals)...);
+}
+template <typename Args>
+cudaError_t launch_dependent(void (*kernel)(Args), unsigned grid, unsigned block, size_t smem,
+                             cudaStream_t st, const Args &args) {
+    return launch_dependent_n(kernel, grid, block, smem, st, args);
 }
 
 // One force evaluation's decomposition and workspace layout.
