@@ -132,6 +132,13 @@ int launch_pair(const PairPlan &pl, float4 *force, const float4 *posMass, float 
 int pair_launches(const PairPlan &pl);
 int pair_prepare();  // kernel attributes of the current context
 int pair_device_sms();  // SMs of the current device, attributes set (0: no device)
+// Potential sums with each pair evaluated once (pair_potential.cu): phi[i].w
+// such that sum_i m_i phi_i / 2 is the potential energy (not body i's own
+// potential).  Up to kMaxPotentialPairs bodies (32-bit steps).
+constexpr size_t kMaxPotentialPairs = (size_t)1 << 22;
+size_t potential_workspace_bytes(size_t n, int sms);
+int launch_potential(size_t n, int sms, const float4 *posMass, float eps2, void *workspace,
+                     float4 *phi, cudaStream_t st);
 int read_and_clear_status(unsigned *bits);
 int read_status_ensemble(unsigned *bits);
 int read_status_integrate(unsigned *bits);

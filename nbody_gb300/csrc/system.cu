@@ -747,20 +747,37 @@ NBGB_API int nbgb_system_diagnostics(nbgb_system *s, double *out) {
     int sync_rc = sync_velocities(s);  // kinetic energy and momenta need v(t)
     if (sync_rc != NBGB_OK)
         return sync_rc;
+    // each pair once, or, for more bodies than its step counters hold, the
+    // one-sided force kernel's potential configuration
+    const bool pairs = n <= nbgb::kMaxPotentialPairs;
+    const int sms = nbgb::pair_device_sms();
     if (!s->diag_ws) {
-        int rc = nbgb::plan_force(n, nbgb::kPotentialConfig, -1, s->diag_plan);
-        if (rc != NBGB_OK)
-            return rc;
-        if (cudaMalloc(&s->diag_ws, s->diag_plan.workspace_bytes) != cudaSuccess ||
+        size_t bytes = 0;
+        if (sms <= 0)
+            return NBGB_ERR_CUDA;
+        if (pairs) {
+            bytes = nbgb::potential_workspace_bytes(n, sms);
+        } else {
+            int rc = nbgb::plan_force(n, nbgb::kPotentialConfig, -1, s->diag_plan);
+            if (rc != NBGB_OK)
+                return rc;
+            bytes = s->diag_plan.workspace_bytes;
+        }
+        if (cudaMalloc(&s->diag_ws, bytes) != cudaSuccess ||
             cudaMalloc(&s->phi, n * 16) != cudaSuccess ||
             cudaMalloc(&s->diag_scratch, nbgb::diag_scratch_bytes()) != cudaSuccess ||
             cudaMalloc(&s->diag_out, 8 * sizeof(double)) != cudaSuccess)
             return NBGB_ERR_NO_MEMORY;
     }
-    int rc = nbgb::launch_pack(s->diag_plan, s->pm, s->diag_ws, s->stream);
-    if (rc == NBGB_OK)
-        rc = nbgb::launch_force(s->diag_plan, s->phi, s->pm, nullptr, s->eps2, s->diag_ws,
-                                s->stream);
+    int rc = NBGB_OK;
+    if (pairs) {
+        rc = nbgb::launch_potential(n, sms, s->pm, s->eps2, s->diag_ws, s->phi, s->stream);
+    } else {
+        rc = nbgb::launch_pack(s->diag_plan, s->pm, s->diag_ws, s->stream);
+        if (rc == NBGB_OK)
+            rc = nbgb::launch_force(s->diag_plan, s->phi, s->pm, nullptr, s->eps2, s->diag_ws,
+                                    s->stream);
+    }
     if (rc == NBGB_OK)
         rc = nbgb::launch_diagnostics((int)n, s->x64, s->ld, s->mass, s->pm, s->vel, s->phi,
                                       s->diag_scratch, s->diag_out, s->stream);
