@@ -346,19 +346,19 @@ class System:
         return a.value, b.value
 
     def get_state(self):
-        pm = np.zeros((self.n, 4), np.float32)
-        vm = np.zeros((self.n, 4), np.float32)
+        pm = np.empty((self.n, 4), np.float32)
+        vm = np.empty((self.n, 4), np.float32)
         check(self.lib.nbgb_system_get_state(self.h, _f32p(pm), _f32p(vm)), "get_state")
         return pm, vm
 
     def get_state64(self):
-        p = np.zeros((self.n, 3), np.float64)
-        v = np.zeros((self.n, 3), np.float64)
+        p = np.empty((self.n, 3), np.float64)
+        v = np.empty((self.n, 3), np.float64)
         check(self.lib.nbgb_system_get_state64(self.h, _f64p(p), _f64p(v)), "get_state64")
         return p, v
 
     def get_force(self) -> np.ndarray:
-        f = np.zeros((self.n, 4), np.float32)
+        f = np.empty((self.n, 4), np.float32)
         check(self.lib.nbgb_system_get_force(self.h, _f32p(f)), "get_force")
         return f
 
@@ -453,9 +453,9 @@ class Ensemble:
 
     def get_state(self, slot: int):
         n = self._n[slot]
-        p = np.zeros((n, 3), np.float64)
-        v = np.zeros((n, 3), np.float64)
-        a = np.zeros((n, 4), np.float32)
+        p = np.empty((n, 3), np.float64)
+        v = np.empty((n, 3), np.float64)
+        a = np.empty((n, 4), np.float32)
         check(self.lib.nbgb_ensemble_get_state(self.h, slot, _f64p(p), _f64p(v), _f32p(a)),
               "ensemble_get_state")
         return p, v, a

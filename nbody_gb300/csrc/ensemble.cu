@@ -72,6 +72,7 @@
 
 #include "nbgb_device.cuh"
 #include "nbgb_internal.h"
+#include "nbgb_snapshot.h"
 #include "nbgb_pair.cuh"
 #include "nbody_gb300.h"
 
@@ -738,6 +739,7 @@ static NBGB_STATUS_READER(read_status_ens)
 }  // namespace ens
 
 int read_status_ensemble(unsigned *bits) { return ens::read_status_ens(bits); }
+const unsigned *status_address_ensemble() { return status_address(); }
 
 }  // namespace nbgb
 
@@ -974,6 +976,7 @@ struct nbgb_ensemble {
     int grid_max = 0;  // SMs x resident CTAs per SM
     size_t bytes_total = 0;
     long long ticks = 0;
+    nbgb::Snapshot snap;
 };
 
 namespace {
@@ -1358,6 +1361,7 @@ void free_ens(nbgb_ensemble *e) {
     cudaFreeHost(e->h_desc);
     cudaFreeHost(e->h_items);
     cudaFreeHost(e->h_slot_sys);
+    e->snap.destroy();
     if (e->stream)
         cudaStreamDestroy(e->stream);
 }
@@ -1441,6 +1445,8 @@ NBGB_API nbgb_ensemble *nbgb_ensemble_create(size_t max_bodies, int max_systems,
     ok = ok && cudaFuncSetAttribute(nbgb::ens::ens_force_kernel,
                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     nbgb::ens::kStages * nbgb::ens::kStageBytes) == cudaSuccess;
+    const unsigned *status = nbgb::status_address_ensemble();
+    ok = ok && status && e->snap.create(max_bodies, &status, 1) == NBGB_OK;
     int occ = 0, sms = 0;
     ok = ok && cudaOccupancyMaxActiveBlocksPerMultiprocessor(
                    &occ, nbgb::ens::ens_force_kernel, nbgb::ens::kThreads,
@@ -1562,24 +1568,19 @@ NBGB_API int nbgb_ensemble_add(nbgb_ensemble *e, const double *pos3, const doubl
     for (size_t i = 0; i < n && h.log_mass; i++)
         h.log_mass = mass[i] >= 0.f;
     // upload state (SoA FP64, masses), zero the j-stream range
-    std::vector<double> tmp(n);
     cudaStream_t st = e->stream;
-    for (int c = 0; c < 6; c++) {
-        const double *src = c < 3 ? pos3 : vel3;
-        for (size_t i = 0; i < n; i++)
-            tmp[i] = src[3 * i + (c % 3)];
-        if (cudaMemcpyAsync(e->x64 + (size_t)c * e->max_bodies + ob, tmp.data(),
-                            n * sizeof(double), cudaMemcpyHostToDevice, st) != cudaSuccess ||
-            cudaStreamSynchronize(st) != cudaSuccess)
-            return NBGB_ERR_CUDA;
-    }
-    if (cudaMemcpyAsync(e->mass + ob, mass, n * sizeof(float), cudaMemcpyHostToDevice, st) !=
-            cudaSuccess ||
-        (h.js_len &&
-         cudaMemsetAsync(e->js + oj, 0, h.js_len * 16, st) != cudaSuccess) ||
+    nbgb::UploadJob job;
+    job.n = n;
+    job.pos3 = pos3;
+    job.vel3 = vel3;
+    job.mass = mass;
+    job.x64 = e->x64 + ob;
+    job.ld = e->max_bodies;
+    job.mass_out = e->mass + ob;
+    if ((h.js_len && cudaMemsetAsync(e->js + oj, 0, h.js_len * 16, st) != cudaSuccess) ||
         (h.acc_len &&
          cudaMemsetAsync(e->acc64 + oa, 0, h.acc_len * sizeof(double), st) != cudaSuccess) ||
-        cudaStreamSynchronize(st) != cudaSuccess)
+        e->snap.upload(job, st) != NBGB_OK)
         return NBGB_ERR_CUDA;
     e->sys[s] = h;
     e->dirty = true;
@@ -1677,10 +1678,9 @@ NBGB_API int nbgb_ensemble_set_graph(nbgb_ensemble *e, int enable) {
 NBGB_API int nbgb_ensemble_synchronize(nbgb_ensemble *e) {
     if (!e)
         return NBGB_ERR_INVALID_ARGUMENT;
-    if (cudaStreamSynchronize(e->stream) != cudaSuccess)
-        return NBGB_ERR_CUDA;
     unsigned bits = 0;
-    if (nbgb::read_status_ensemble(&bits) != NBGB_OK)
+    if (e->snap.run(nbgb::SnapshotJob(), e->stream, &bits) != NBGB_OK ||
+        (bits && nbgb::read_status_ensemble(&bits) != NBGB_OK))
         return NBGB_ERR_CUDA;
     return bits ? NBGB_ERR_DEVICE : NBGB_OK;
 }
@@ -1702,26 +1702,16 @@ NBGB_API int nbgb_ensemble_get_state(nbgb_ensemble *e, int slot, double *pos3, d
     if (!e || slot < 0 || slot >= e->max_systems || !e->sys[slot].used)
         return NBGB_ERR_INVALID_ARGUMENT;
     const HostSys &h = e->sys[slot];
-    const size_t n = h.n;
-    std::vector<double> tmp(6 * n);
-    cudaStream_t st = e->stream;
-    for (int c = 0; c < 6; c++)
-        if (cudaMemcpyAsync(tmp.data() + c * n, e->x64 + (size_t)c * e->max_bodies + h.body_off,
-                            n * sizeof(double), cudaMemcpyDeviceToHost, st) != cudaSuccess)
-            return NBGB_ERR_CUDA;
-    if (acc4 && cudaMemcpyAsync(acc4, e->acc + h.body_off, n * 16, cudaMemcpyDeviceToHost, st) !=
-                    cudaSuccess)
-        return NBGB_ERR_CUDA;
-    if (cudaStreamSynchronize(st) != cudaSuccess)
-        return NBGB_ERR_CUDA;
-    for (size_t i = 0; i < n; i++)
-        for (int c = 0; c < 3; c++) {
-            if (pos3)
-                pos3[3 * i + c] = tmp[c * n + i];
-            if (vel3)
-                vel3[3 * i + c] = tmp[(3 + c) * n + i];
-        }
-    return NBGB_OK;
+    nbgb::SnapshotJob job;
+    job.n = (size_t)h.n;
+    job.vec[0] = e->acc + h.body_off;
+    job.out[0] = acc4;
+    job.x64 = e->x64 + h.body_off;
+    job.ld = e->max_bodies;
+    job.pos3 = pos3;
+    job.vel3 = vel3;
+    unsigned bits = 0;
+    return e->snap.run(job, e->stream, &bits);  // (synchronize() reports the status)
 }
 
 // Slot info: bodies, steps done, steps left, plan (variant, tile, split).

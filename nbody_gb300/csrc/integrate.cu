@@ -220,6 +220,7 @@ __global__ void conversion_selftest_kernel(unsigned long long seed, long long n,
 static NBGB_STATUS_READER(read_status_integrate_tu)
 
 int read_status_integrate(unsigned *bits) { return read_status_integrate_tu(bits); }
+const unsigned *status_address_integrate() { return status_address(); }
 
 }  // namespace nbgb
 

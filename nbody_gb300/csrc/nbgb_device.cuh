@@ -33,6 +33,12 @@ static __device__ unsigned int g_status = 0;
         return NBGB_OK;                                                            \
     }
 
+// Its device address in the current context (null: none)
+static inline const unsigned *status_address() {
+    void *p = nullptr;
+    return cudaGetSymbolAddress(&p, g_status) == cudaSuccess ? (const unsigned *)p : nullptr;
+}
+
 // ---------------------------------------------------------------------------
 // Packed FP32 pairs.  A u64 holds (lo, hi) = two binary32 values in adjacent
 // registers; add/fma/mul.f32x2 run both halves in one instruction.

@@ -140,6 +140,10 @@ size_t potential_workspace_bytes(size_t n, int sms);
 int launch_potential(size_t n, int sms, const float4 *posMass, float eps2, void *workspace,
                      float4 *phi, cudaStream_t st);
 int read_and_clear_status(unsigned *bits);
+// the three status words' addresses in the current context
+int status_addresses(const unsigned **out3);
+const unsigned *status_address_ensemble();
+const unsigned *status_address_integrate();
 int read_status_ensemble(unsigned *bits);
 int read_status_integrate(unsigned *bits);
 // js_vpb, js_log: j-stream layout of the plan the j-stream is written for.

@@ -28,6 +28,7 @@
 #include <vector>
 
 #include "nbgb_internal.h"
+#include "nbgb_snapshot.h"
 #include "nbody_gb300.h"
 
 using nbgb::ForcePlan;
@@ -80,6 +81,7 @@ struct nbgb_system {
     double *diag_scratch = nullptr;
     double *diag_out = nullptr;
     int status = NBGB_OK;
+    nbgb::Snapshot snap;
 };
 
 namespace {
@@ -297,9 +299,24 @@ int fit_plan_to_masses(nbgb_system *s, const float *m, size_t stride) {
     return NBGB_OK;
 }
 
-int check_device_status() {
+// An upload into the FP64 components (the host arrays are the caller's to fill in).
+nbgb::UploadJob upload_job(nbgb_system *s) {
+    nbgb::UploadJob job;
+    job.n = s->n;
+    job.x64 = s->x64;
+    job.ld = s->ld;
+    job.pad = s->ld - s->n;
+    job.mass_out = s->mass;
+    job.pm = s->pm;
+    return job;
+}
+
+// The job after everything on the stream; reports and clears the device
+// status.
+int download(nbgb_system *s, const nbgb::SnapshotJob &job) {
     unsigned bits = 0;
-    if (nbgb::read_and_clear_status(&bits) != NBGB_OK)
+    if (s->snap.run(job, s->stream, &bits) != NBGB_OK ||
+        (bits && nbgb::read_and_clear_status(&bits) != NBGB_OK))
         return NBGB_ERR_CUDA;
     return bits ? NBGB_ERR_DEVICE : NBGB_OK;
 }
@@ -325,6 +342,7 @@ void free_all(nbgb_system *s) {
     cudaFree(s->phi);
     cudaFree(s->diag_scratch);
     cudaFree(s->diag_out);
+    s->snap.destroy();
     if (s->stream)
         cudaStreamDestroy(s->stream);
 }
@@ -424,6 +442,9 @@ NBGB_API nbgb_system *nbgb_system_create(size_t N, int integrator, float softeni
     // counters start at zero; every force launch leaves them at zero
     ok = ok && (s->plan.use_pair ||
                 cudaMemsetAsync(s->ws, 0, s->ws_bytes, s->stream) == cudaSuccess);
+    const unsigned *status[3];
+    ok = ok && nbgb::status_addresses(status) == NBGB_OK &&
+         s->snap.create(N, status, 3) == NBGB_OK;
     ok = ok && cudaStreamSynchronize(s->stream) == cudaSuccess;
     if (!ok) {
         free_all(s);
@@ -458,29 +479,18 @@ NBGB_API int nbgb_system_set_state(nbgb_system *s, const float *posMass, const f
     int rc = fit_plan_to_masses(s, posMass + 3, 4);
     if (rc != NBGB_OK)
         return rc;
-    if (cudaMemcpyAsync(s->pm, posMass, n * 16, cudaMemcpyHostToDevice, s->stream) != cudaSuccess)
-        return NBGB_ERR_CUDA;
     if (reference_integrator(s->integrator)) {
-        if (cudaMemcpyAsync(s->vel, velInvMass, n * 16, cudaMemcpyHostToDevice, s->stream) !=
-            cudaSuccess)
+        if (cudaMemcpyAsync(s->pm, posMass, n * 16, cudaMemcpyHostToDevice, s->stream) !=
+                cudaSuccess ||
+            cudaMemcpyAsync(s->vel, velInvMass, n * 16, cudaMemcpyHostToDevice, s->stream) !=
+                cudaSuccess)
             return NBGB_ERR_CUDA;
     } else {
-        const size_t ld = s->ld;
-        std::vector<double> h(ld * 6, 0.0);
-        std::vector<float> m(n);
-        for (size_t i = 0; i < n; i++) {
-            for (int c = 0; c < 3; c++) {
-                h[c * ld + i] = posMass[4 * i + c];
-                h[(3 + c) * ld + i] = velInvMass[4 * i + c];
-            }
-            m[i] = posMass[4 * i + 3];
-        }
-        if (cudaMemcpyAsync(s->x64, h.data(), ld * 6 * sizeof(double), cudaMemcpyHostToDevice,
-                            s->stream) != cudaSuccess ||
-            cudaMemcpyAsync(s->mass, m.data(), n * sizeof(float), cudaMemcpyHostToDevice,
-                            s->stream) != cudaSuccess ||
-            cudaStreamSynchronize(s->stream) != cudaSuccess)
-            return NBGB_ERR_CUDA;
+        nbgb::UploadJob job = upload_job(s);
+        job.posMass = posMass;
+        job.velInvMass = velInvMass;
+        if ((rc = s->snap.upload(job, s->stream)) != NBGB_OK)
+            return rc;
     }
     s->js_valid = false;
     s->accel_valid = false;
@@ -497,25 +507,12 @@ NBGB_API int nbgb_system_set_state64(nbgb_system *s, const double *pos3, const d
     int rc = fit_plan_to_masses(s, mass, 1);
     if (rc != NBGB_OK)
         return rc;
-    const size_t ld = s->ld;
-    std::vector<double> h(ld * 6, 0.0);
-    std::vector<float> pm(n * 4);
-    for (size_t i = 0; i < n; i++) {
-        for (int c = 0; c < 3; c++) {
-            h[c * ld + i] = pos3[3 * i + c];
-            h[(3 + c) * ld + i] = vel3[3 * i + c];
-            pm[4 * i + c] = (float)pos3[3 * i + c];
-        }
-        pm[4 * i + 3] = mass[i];
-    }
-    if (cudaMemcpyAsync(s->x64, h.data(), ld * 6 * sizeof(double), cudaMemcpyHostToDevice,
-                        s->stream) != cudaSuccess ||
-        cudaMemcpyAsync(s->mass, mass, n * sizeof(float), cudaMemcpyHostToDevice, s->stream) !=
-            cudaSuccess ||
-        cudaMemcpyAsync(s->pm, pm.data(), n * 16, cudaMemcpyHostToDevice, s->stream) !=
-            cudaSuccess ||
-        cudaStreamSynchronize(s->stream) != cudaSuccess)
-        return NBGB_ERR_CUDA;
+    nbgb::UploadJob job = upload_job(s);
+    job.pos3 = pos3;
+    job.vel3 = vel3;
+    job.mass = mass;
+    if ((rc = s->snap.upload(job, s->stream)) != NBGB_OK)
+        return rc;
     s->js_valid = false;
     s->accel_valid = false;
     s->v_lag = false;
@@ -656,9 +653,7 @@ NBGB_API int nbgb_system_last_force_ms(nbgb_system *s, float *ms) {
 NBGB_API int nbgb_system_synchronize(nbgb_system *s) {
     if (!s)
         return NBGB_ERR_INVALID_ARGUMENT;
-    if (cudaStreamSynchronize(s->stream) != cudaSuccess)
-        return NBGB_ERR_CUDA;
-    return check_device_status();
+    return download(s, nbgb::SnapshotJob());
 }
 
 NBGB_API int nbgb_system_get_state(nbgb_system *s, float *posMass, float *velInvMass) {
@@ -670,58 +665,38 @@ NBGB_API int nbgb_system_get_state(nbgb_system *s, float *posMass, float *velInv
         if (rc != NBGB_OK)
             return rc;
     }
-    if (posMass &&
-        cudaMemcpyAsync(posMass, s->pm, n * 16, cudaMemcpyDeviceToHost, s->stream) != cudaSuccess)
-        return NBGB_ERR_CUDA;
-    if (velInvMass) {
-        if (reference_integrator(s->integrator)) {
-            if (cudaMemcpyAsync(velInvMass, s->vel, n * 16, cudaMemcpyDeviceToHost, s->stream) !=
-                cudaSuccess)
-                return NBGB_ERR_CUDA;
-        } else {
-            const size_t ld = s->ld;
-            std::vector<double> h(ld * 3);
-            std::vector<float> m(n);
-            if (cudaMemcpyAsync(h.data(), comp(s, 3), ld * 3 * sizeof(double),
-                                cudaMemcpyDeviceToHost, s->stream) != cudaSuccess ||
-                cudaMemcpyAsync(m.data(), s->mass, n * sizeof(float), cudaMemcpyDeviceToHost,
-                                s->stream) != cudaSuccess ||
-                cudaStreamSynchronize(s->stream) != cudaSuccess)
-                return NBGB_ERR_CUDA;
-            for (size_t i = 0; i < n; i++) {
-                for (int c = 0; c < 3; c++)
-                    velInvMass[4 * i + c] = (float)h[c * ld + i];
-                velInvMass[4 * i + 3] = 1.0f / m[i];
-            }
-        }
+    nbgb::SnapshotJob job;
+    job.n = n;
+    job.vec[0] = s->pm;
+    job.out[0] = posMass;
+    if (reference_integrator(s->integrator)) {
+        job.vec[1] = s->vel;
+        job.out[1] = velInvMass;
+    } else {
+        job.x64 = s->x64;
+        job.ld = s->ld;
+        job.mass = s->mass;
+        job.velinv = velInvMass;
     }
-    if (cudaStreamSynchronize(s->stream) != cudaSuccess)
-        return NBGB_ERR_CUDA;
-    return check_device_status();
+    return download(s, job);
 }
 
+// FP64 state out (KDK only): x, v as double[N][3] (AOS).
 NBGB_API int nbgb_system_get_state64(nbgb_system *s, double *pos3, double *vel3) {
     if (!s || s->integrator != NBGB_INTEGRATOR_KDK64)
         return NBGB_ERR_INVALID_ARGUMENT;
-    const size_t n = s->n, ld = s->ld;
     if (vel3) {
         int rc = sync_velocities(s);
         if (rc != NBGB_OK)
             return rc;
     }
-    std::vector<double> h(ld * 6);
-    if (cudaMemcpyAsync(h.data(), s->x64, ld * 6 * sizeof(double), cudaMemcpyDeviceToHost,
-                        s->stream) != cudaSuccess ||
-        cudaStreamSynchronize(s->stream) != cudaSuccess)
-        return NBGB_ERR_CUDA;
-    for (size_t i = 0; i < n; i++)
-        for (int c = 0; c < 3; c++) {
-            if (pos3)
-                pos3[3 * i + c] = h[c * ld + i];
-            if (vel3)
-                vel3[3 * i + c] = h[(3 + c) * ld + i];
-        }
-    return check_device_status();
+    nbgb::SnapshotJob job;
+    job.n = s->n;
+    job.x64 = s->x64;
+    job.ld = s->ld;
+    job.pos3 = pos3;
+    job.vel3 = vel3;
+    return download(s, job);
 }
 
 // Forces of the last force pass (reference: F(x) before the integrate; KDK:
@@ -729,11 +704,11 @@ NBGB_API int nbgb_system_get_state64(nbgb_system *s, double *pos3, double *vel3)
 NBGB_API int nbgb_system_get_force(nbgb_system *s, float *force) {
     if (!s || !force)
         return NBGB_ERR_INVALID_ARGUMENT;
-    if (cudaMemcpyAsync(force, s->force, s->n * 16, cudaMemcpyDeviceToHost, s->stream) !=
-            cudaSuccess ||
-        cudaStreamSynchronize(s->stream) != cudaSuccess)
-        return NBGB_ERR_CUDA;
-    return check_device_status();
+    nbgb::SnapshotJob job;
+    job.n = s->n;
+    job.vec[0] = s->force;
+    job.out[0] = force;
+    return download(s, job);
 }
 
 // Conserved quantities at the current state, FP64: out[0] kinetic energy,
@@ -783,11 +758,11 @@ NBGB_API int nbgb_system_diagnostics(nbgb_system *s, double *out) {
                                       s->diag_scratch, s->diag_out, s->stream);
     if (rc != NBGB_OK)
         return rc;
-    if (cudaMemcpyAsync(out, s->diag_out, 8 * sizeof(double), cudaMemcpyDeviceToHost,
-                        s->stream) != cudaSuccess ||
-        cudaStreamSynchronize(s->stream) != cudaSuccess)
-        return NBGB_ERR_CUDA;
-    return check_device_status();
+    nbgb::SnapshotJob job;
+    job.n = 4;  // 8 doubles
+    job.vec[0] = (const float4 *)s->diag_out;
+    job.out[0] = (float *)out;
+    return download(s, job);
 }
 
 // Device pointers for callers that manage copies themselves.
