@@ -446,7 +446,7 @@ constexpr int kPairCtaThreads = Narrow::kThreads;
 static_assert(Wide::kThreads == Narrow::kThreads && Wide::kSet == Narrow::kSet,
               "one persistent kernel for both geometries");
 constexpr size_t kPairSmem = Wide::kSmem > Narrow::kSmem ? Wide::kSmem : Narrow::kSmem;
-constexpr int kBodyBlock = 32;  // bodies of one entry of the block map
+constexpr int kBodyBlock = 64;  // bodies of one entry of the block map, two a reduction thread
 
 struct PairParams {
     const Desc *__restrict__ desc;
@@ -461,7 +461,7 @@ struct PairParams {
     size_t stride;
 };
 
-// Entry e of the block map: bodies 32 blk .. 32 blk + 31 of one pair system.
+// Entry e of the block map: bodies kBodyBlock blk and on of one pair system.
 __device__ __forceinline__ bool takes_part(const Desc &d, int pass) {
     return (d.flags & kInForce) && (pass == 0 || ((d.flags & kMove) && d.sub > pass));
 }
@@ -661,19 +661,25 @@ __global__ void __launch_bounds__(256)
     pm[i] = make_float4(narrow_f64(x), narrow_f64(y), narrow_f64(z), m);
 }
 
-// One block per entry: kReduceGroups x 3 (components) threads a body add its
-// reaction pieces (rows before its own, in row order) and its row's target
-// pieces, eight loads in flight; then the acceleration and the closing half
-// kick.
-constexpr int kReduceGroups = 4;
-constexpr int kReduceThreads = 3 * kBodyBlock * kReduceGroups;
+// One block per entry: kReduceGroups x 3 (components) threads for two bodies
+// add their reaction pieces (rows before their own, in row order) and their
+// row's target pieces, eight loads in flight; then the acceleration and the
+// closing half kick, whose velocities are loaded beside the pieces.  Bound by
+// the latency of one block (the entry, its system, the pieces), times the
+// blocks that follow one another on an SM: with one body and four groups a
+// thread, 3.9 thousand blocks for 64 systems of 64 to 7,205 bodies and 172 us
+// a tick; with two bodies 169, and two groups 165; 8 systems of 8,701 to
+// 58,144: 3,089 -> 3,051 us.
+constexpr int kReduceGroups = 2;
+constexpr int kReduceThreads = 3 * 32 * kReduceGroups;
 
 template <class G>
 __device__ __forceinline__ void reduce_entry(const Desc &d, int blk, const float *scratch,
                                              double *x64, size_t stride, float4 *acc) {
     constexpr int kB = kBodyBlock, kSet = G::kSet;
-    __shared__ float part[kReduceGroups - 1][2][3][kB], out[3][kB];
-    const int tid = threadIdx.x, group = tid / (3 * kB), comp = (tid / kB) % 3, j = tid % kB;
+    __shared__ __align__(8) float part[kReduceGroups - 1][2][3][kB], out[3][kB];
+    static_assert(kB == 64, "two bodies a lane");
+    const int tid = threadIdx.x, group = tid / (3 * 32), comp = (tid / 32) % 3, j = 2 * (tid & 31);
     const int i = blk * kB + j, set = blk * kB / kSet, b = set / G::kRowSets;
     const int nt = (d.nsets - b * G::kRowSets + d.ch - 1) / d.ch, total = b + nt;
     const int q0 = total * group / kReduceGroups, q1 = total * (group + 1) / kReduceGroups;
@@ -685,37 +691,48 @@ __device__ __forceinline__ void reduce_entry(const Desc &d, int blk, const float
                                    (3 * kSet)
                      : tsum + (long long)(q - b) * (3 * G::kRow);
     };
-    float hi = 0.f, lo = 0.f;
+    // the group that kicks has its velocities in flight beside the pieces
+    const bool kick = group == 0 && (d.flags & kMove);
+    double *vel = x64 + (3 + comp) * stride + d.body_off + i;
+    const double v0 = kick && i < d.n ? vel[0] : 0.0, v1 = kick && i + 1 < d.n ? vel[1] : 0.0;
+    float2 hi = make_float2(0.f, 0.f), lo = hi;
     for (int q = q0; q < q1; q += 8) {
-        float v[8];
+        float2 v[8];
 #pragma unroll
         for (int u = 0; u < 8; u++)
-            v[u] = q + u < q1 ? __ldcs(piece(q + u)) : 0.f;
+            v[u] = q + u < q1 ? __ldcs((const float2 *)piece(q + u)) : make_float2(0.f, 0.f);
 #pragma unroll
-        for (int u = 0; u < 8; u++)
-            comp_add(hi, lo, v[u]);
+        for (int u = 0; u < 8; u++) {
+            comp_add(hi.x, lo.x, v[u].x);
+            comp_add(hi.y, lo.y, v[u].y);
+        }
     }
     if (group) {
-        part[group - 1][0][comp][j] = hi;
-        part[group - 1][1][comp][j] = lo;
+        *(float2 *)&part[group - 1][0][comp][j] = hi;
+        *(float2 *)&part[group - 1][1][comp][j] = lo;
     }
     __syncthreads();
     if (group == 0) {
 #pragma unroll
         for (int q = 0; q < kReduceGroups - 1; q++) {
-            comp_add(hi, lo, part[q][0][comp][j]);
-            lo += part[q][1][comp][j];
+            const float2 h = *(const float2 *)&part[q][0][comp][j];
+            const float2 l = *(const float2 *)&part[q][1][comp][j];
+            comp_add(hi.x, lo.x, h.x);
+            lo.x += l.x;
+            comp_add(hi.y, lo.y, h.y);
+            lo.y += l.y;
         }
-        const float a = hi + lo;
-        out[comp][j] = a;
-        if (i < d.n && (d.flags & kMove)) {
-            double *v = x64 + (3 + comp) * stride + d.body_off + i;
-            *v = fma(widen_f32(a), 0.5 * d.dt, *v);
-        }
+        const float2 a = make_float2(hi.x + lo.x, hi.y + lo.y);
+        *(float2 *)&out[comp][j] = a;
+        if (kick && i < d.n)
+            vel[0] = fma(widen_f32(a.x), 0.5 * d.dt, v0);
+        if (kick && i + 1 < d.n)
+            vel[1] = fma(widen_f32(a.y), 0.5 * d.dt, v1);
     }
     __syncthreads();
-    if (tid < kB && i < d.n)
-        acc[(size_t)d.body_off + i] = make_float4(out[0][j], out[1][j], out[2][j], 0.f);
+    const int ib = blk * kB + tid;
+    if (tid < kB && ib < d.n)
+        acc[(size_t)d.body_off + ib] = make_float4(out[0][tid], out[1][tid], out[2][tid], 0.f);
 }
 
 __global__ void __launch_bounds__(kReduceThreads)

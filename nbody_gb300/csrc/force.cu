@@ -450,7 +450,7 @@ __global__ void __launch_bounds__(W * 32, MINB) force_kernel(ForceParams p) {
                 const float fx = hx[k] + lx[k], fy = hy[k] + ly[k], fz = hz[k] + lz[k];
                 p.force[i] = make_float4(fx, fy, fz, POT ? -((hp[k] - self[k]) + lp[k]) : 0.f);
                 if (!POT && p.fi.vel)
-                    fused_integrate(p.fi, i, px[k], py[k], pz[k], pm_self[k], fx, fy, fz);
+                    fused_integrate(p.fi, i, p.fi.vel[i], px[k], py[k], pz[k], pm_self[k], fx, fy, fz);
             }
         }
         return;
@@ -506,7 +506,7 @@ __global__ void __launch_bounds__(W * 32, MINB) force_kernel(ForceParams p) {
         const float fx = Hx + Lx, fy = Hy + Ly, fz = Hz + Lz;
         p.force[i] = make_float4(fx, fy, fz, POT ? -((Hp - self[k]) + Lp) : 0.f);
         if (!POT && p.fi.vel)
-            fused_integrate(p.fi, i, px[k], py[k], pz[k], pm_self[k], fx, fy, fz);
+            fused_integrate(p.fi, i, p.fi.vel[i], px[k], py[k], pz[k], pm_self[k], fx, fy, fz);
     }
 }
 

@@ -145,25 +145,37 @@ struct ReduceParams {
     FusedIntegrate fi;  // fi.vel == nullptr: forces only
 };
 
-// kReduceBodies bodies a block, kGroups x 3 (components) threads a body: the
-// body's reaction pieces (one list for the block, from the phase's earlier
-// rows in row order) and then its row's target pieces form one sequence; each
-// group adds a contiguous part of it, eight loads in flight, and the parts
-// are added in order.  A latency problem, not a bandwidth one: at N = 3,000
-// about 50 pieces a body and 9,000 sums, where four groups took 4 us more
-// than with few pieces.
-constexpr int kReduceBodies = 32;
+// 32 kEach bodies a block, kGroups x 3 (components) threads for kEach bodies:
+// the block's reaction pieces (one list, from the phase's earlier rows in row
+// order) and then its row's target pieces form one sequence; each group adds
+// a contiguous part of it, eight loads in flight, and the parts are added in
+// order.  A latency problem, not a bandwidth one: at N = 3,000 about 50 pieces
+// a body and 9,000 sums, where four groups took 4 us more than with few
+// pieces.
+template <int kEach>
+struct alignas(4 * kEach) Bodies {  // one component of a thread's bodies
+    float v[kEach];
+};
+__device__ __forceinline__ Bodies<1> load_once(const Bodies<1> *p) {
+    return {{__ldcs(&p->v[0])}};
+}
+__device__ __forceinline__ Bodies<2> load_once(const Bodies<2> *p) {
+    const float2 a = __ldcs(reinterpret_cast<const float2 *>(p));
+    return {{a.x, a.y}};
+}
 
-template <class G, int kGroups>
-__global__ void __launch_bounds__(3 * kReduceBodies * kGroups)
+template <class G, int kGroups, int kEach>
+__global__ void __launch_bounds__(3 * 32 * kGroups)
     pair_reduce_kernel(const __grid_constant__ ReduceParams R) {
-    constexpr int kSet = G::kSet, kB = kReduceBodies, kPart = kSet / kB;
+    typedef Bodies<kEach> V;
+    constexpr int kSet = G::kSet, kB = 32 * kEach, kPart = kSet / kB;
     static_assert(kSet % kB == 0, "blocks are parts of a set");
     __shared__ int list[kMaxPairRows + kMaxPairCtas];
     __shared__ int n_list, t_first, t_count;
-    __shared__ float part[kGroups - 1][2][3][kB], out[3][kB];
+    __shared__ V part[kGroups - 1][2][3][32], out[3][32];
     const Params &P = R.p;
-    const int tid = threadIdx.x, group = tid / (3 * kB), comp = (tid / kB) % 3, j = tid % kB;
+    const int tid = threadIdx.x, group = tid / (3 * 32), comp = (tid / 32) % 3;
+    const int lane = tid & 31, j = kEach * lane;
     const int set = P.row0 * G::kRowSets + blockIdx.x / kPart;
     const int sub = blockIdx.x % kPart;  // part of the set
     const int b = set / G::kRowSets;
@@ -238,57 +250,71 @@ __global__ void __launch_bounds__(3 * kReduceBodies * kGroups)
     };
     grid_dependents_launch();
     grid_dependency_wait();
-    float hi = 0.f, lo = 0.f;
+    const int ib = set * kSet + sub * kB + tid;
+    const bool writes = final && tid < kB && ib < P.src.n;
+    V hi = {}, lo = {};
+    auto carry = [&](int part) {
+        return reinterpret_cast<V *>(R.carry + (3 * part + comp) * R.npad + i);
+    };
     if (P.row0 > 0 && group == 0) {
-        hi = R.carry[comp * R.npad + i];
-        lo = R.carry[(3 + comp) * R.npad + i];
+        hi = *carry(0);
+        lo = *carry(1);
     }
     int q = q0;
     for (; q + 8 <= q1; q += 8) {
-        float v[8];
+        V v[8];
 #pragma unroll
         for (int u = 0; u < 8; u++)
-            v[u] = __ldcs(piece(q + u));
+            v[u] = load_once(reinterpret_cast<const V *>(piece(q + u)));
 #pragma unroll
         for (int u = 0; u < 8; u++)
-            comp_add(hi, lo, v[u]);
+#pragma unroll
+            for (int k = 0; k < kEach; k++)
+                comp_add(hi.v[k], lo.v[k], v[u].v[k]);
     }
     if (q < q1) {
-        float v[8];
+        V v[8];
 #pragma unroll
         for (int u = 0; u < 8; u++)
-            v[u] = q + u < q1 ? __ldcs(piece(q + u)) : 0.f;
+            v[u] = q + u < q1 ? load_once(reinterpret_cast<const V *>(piece(q + u))) : V{};
 #pragma unroll
         for (int u = 0; u < 8; u++)
-            comp_add(hi, lo, v[u]);
+#pragma unroll
+            for (int k = 0; k < kEach; k++)
+                comp_add(hi.v[k], lo.v[k], v[u].v[k]);
     }
     if (group) {
-        part[group - 1][0][comp][j] = hi;
-        part[group - 1][1][comp][j] = lo;
+        part[group - 1][0][comp][lane] = hi;
+        part[group - 1][1][comp][lane] = lo;
     }
     __syncthreads();
     if (group == 0) {
 #pragma unroll
-        for (int q = 0; q < kGroups - 1; q++) {
-            comp_add(hi, lo, part[q][0][comp][j]);
-            lo += part[q][1][comp][j];
-        }
+        for (int q = 0; q < kGroups - 1; q++)
+#pragma unroll
+            for (int k = 0; k < kEach; k++) {
+                comp_add(hi.v[k], lo.v[k], part[q][0][comp][lane].v[k]);
+                lo.v[k] += part[q][1][comp][lane].v[k];
+            }
         if (!final) {
-            R.carry[comp * R.npad + i] = hi;
-            R.carry[(3 + comp) * R.npad + i] = lo;
+            *carry(0) = hi;
+            *carry(1) = lo;
         }
-        out[comp][j] = hi + lo;
+#pragma unroll
+        for (int k = 0; k < kEach; k++)
+            out[comp][lane].v[k] = hi.v[k] + lo.v[k];
     }
     if (!final)
         return;
     __syncthreads();
-    const int ib = set * kSet + sub * kB + tid;
-    if (tid < kB && ib < P.src.n) {
-        const float fx = out[0][tid], fy = out[1][tid], fz = out[2][tid];
+    if (writes) {
+        const float fx = out[0][tid / kEach].v[tid % kEach];
+        const float fy = out[1][tid / kEach].v[tid % kEach];
+        const float fz = out[2][tid / kEach].v[tid % kEach];
         R.force[ib] = make_float4(fx, fy, fz, 0.f);
         if (R.fi.vel) {
-            const float4 v = P.src.pm[ib];
-            fused_integrate(R.fi, ib, v.x, v.y, v.z, v.w, fx, fy, fz);
+            const float4 pos = P.src.pm[ib], vel = R.fi.vel[ib];
+            fused_integrate(R.fi, ib, vel, pos.x, pos.y, pos.z, pos.w, fx, fy, fz);
         }
     }
 }
@@ -400,6 +426,10 @@ static bool plan_geometry(size_t n, int sms, size_t max_bytes, PairPlan &pl) {
     // 16.5 us against 17.5 with four), four where their smaller blocks fit
     // beside the pair kernel's CTAs and start early (8,192, 27: 26.6 / 27.5)
     pl.groups8 = pl.ncta / rows + rows / 2 >= 28 && rows <= 16;
+    // two bodies a thread where the blocks of one would not be resident
+    // together (16,384 bodies: 86.9 -> 83.0 us, 32,768: 294.7 -> 290.5; with
+    // fewer blocks one is as fast or faster, 1,000: 5.7 / 6.0)
+    pl.each = (long long)nsets * (G::kSet / 32) * (pl.groups8 ? 768 : 384) > sms * 2048LL ? 2 : 1;
     const size_t tsum =
         align256((size_t)(std::min(rows, kMaxPairRows) + pl.ncta) * 3 * G::kRow * 4);
     const size_t carry = align256((size_t)nsets * G::kSet * 6 * 4);
@@ -426,6 +456,17 @@ static bool plan_geometry(size_t n, int sms, size_t max_bytes, PairPlan &pl) {
     pl.off_carry = pl.off_tsum + tsum;
     pl.workspace_bytes = pl.off_carry + (one ? 0 : carry);
     return !max_bytes || pl.workspace_bytes <= max_bytes;
+}
+
+template <class G>
+static cudaError_t launch_reduce(const PairPlan &pl, const pair::ReduceParams &R, int sets,
+                                 cudaStream_t st) {
+    const unsigned blocks = (unsigned)(sets * (G::kSet / 32 / pl.each));
+    if (pl.each == 1)
+        return pl.groups8 ? launch_dependent(pair::pair_reduce_kernel<G, 8, 1>, blocks, 768, 0, st, R)
+                          : launch_dependent(pair::pair_reduce_kernel<G, 4, 1>, blocks, 384, 0, st, R);
+    return pl.groups8 ? launch_dependent(pair::pair_reduce_kernel<G, 8, 2>, blocks, 768, 0, st, R)
+                      : launch_dependent(pair::pair_reduce_kernel<G, 4, 2>, blocks, 384, 0, st, R);
 }
 
 template <class G>
@@ -461,15 +502,9 @@ static int launch_geometry(const PairPlan &pl, float4 *force, const float4 *posM
             P.ncta = pl.ncta;
         pair::cut_steps<G>(P.row0, P.row1, nsets, P.ncta, pl.parts, P.step);
         const size_t smem = pl.lone ? pair::kLoneSmem : G::kSmem;
-        const unsigned blocks =
-            (nsets - P.row0 * G::kRowSets) * (G::kSet / pair::kReduceBodies);
         if (launch_dependent(pair::pair_kernel<G>, P.ncta, G::kThreads, smem, st, P) !=
                 cudaSuccess ||
-            (pl.groups8 ? launch_dependent(pair::pair_reduce_kernel<G, 8>, blocks,
-                                           3 * pair::kReduceBodies * 8, 0, st, R)
-                        : launch_dependent(pair::pair_reduce_kernel<G, 4>, blocks,
-                                           3 * pair::kReduceBodies * 4, 0, st, R)) !=
-                cudaSuccess)
+            launch_reduce<G>(pl, R, nsets - P.row0 * G::kRowSets, st) != cudaSuccess)
             return NBGB_ERR_CUDA;
     }
     return NBGB_OK;

@@ -16,9 +16,10 @@ namespace nbgb {
 // kept, the pair kernel reads posMass).  Only the last unit of an
 // i-block writes its targets, after every unit of that i-block has loaded
 // them, so no unit reads a target this launch has moved.
-__device__ __forceinline__ void fused_integrate(const FusedIntegrate &fi, int i, float x, float y,
-                                                float z, float m, float fx, float fy, float fz) {
-    float4 v = fi.vel[i];
+// v: the body's velInvMass.
+__device__ __forceinline__ void fused_integrate(const FusedIntegrate &fi, int i, float4 v, float x,
+                                                float y, float z, float m, float fx, float fy,
+                                                float fz) {
     const float im = v.w, dt = fi.dt;
     v.x = __fmul_rn(__fadd_rn(v.x, __fmul_rn(__fmul_rn(fx, im), dt)), fi.damping);
     v.y = __fmul_rn(__fadd_rn(v.y, __fmul_rn(__fmul_rn(fy, im), dt)), fi.damping);

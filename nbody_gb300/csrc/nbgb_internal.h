@@ -25,6 +25,7 @@ struct PairPlan {
     int parts = 0;            // > 0: each meeting is so many stretches of its own
     int lone = 0;             // one CTA an SM
     int groups8 = 0;          // eight reduction threads a body (else four)
+    int each = 1;             // bodies of a reduction thread
     size_t react_bytes = 0;   // reaction pieces of one phase, at most
     size_t off_react = 0, off_tsum = 0, off_carry = 0;
     size_t workspace_bytes = 0;
