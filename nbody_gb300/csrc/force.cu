@@ -650,7 +650,7 @@ static const DeviceInfo *device_info() {
         d.occ[c] = occ;
     }
     void *status = nullptr;
-    if (pair_prepare() != NBGB_OK || cudaGetSymbolAddress(&status, g_status) != cudaSuccess)
+    if (pair_prepare() != NBGB_OK || direct_prepare() != NBGB_OK || cudaGetSymbolAddress(&status, g_status) != cudaSuccess)
         return nullptr;
     d.status = (unsigned *)status;
     d.ok = true;
@@ -868,6 +868,7 @@ static void use_pair_plan(ForcePlan &pl, const DeviceInfo *d, size_t max_bytes =
     if (!d || pl.n > kMaxPairForce || !plan_pair(pl.n, d->sms, max_bytes, pl.pair))
         return;
     pl.use_pair = 1;
+    pl.direct = direct_targets(pl.n, d->sms);
     pl.pair.status = pl.js_log ? d->status : nullptr;
     pl.workspace_bytes = std::max(pl.workspace_bytes, pl.pair.workspace_bytes);
 }
@@ -956,6 +957,8 @@ int plan_force_within(size_t n, size_t max_bytes, ForcePlan &pl) {
 
 int launch_force(const ForcePlan &pl, float4 *force, const float4 *posMass, const float4 *jstream,
                  float eps2, void *workspace, cudaStream_t stream, const FusedIntegrate *fi) {
+    if (pl.direct)
+        return launch_direct(pl.n, pl.direct, pl.pair.status, force, posMass, eps2, stream, fi);
     if (pl.use_pair)
         return launch_pair(pl.pair, force, posMass, eps2, workspace, stream, fi);
     const ForceConfig &cf = kConfigs[pl.config];
@@ -1225,9 +1228,9 @@ NBGB_API int nbgb_force_kind(size_t N, int *pairs, int *launches) {
     if (rc != NBGB_OK)
         return rc;
     if (pairs)
-        *pairs = pl.use_pair;
+        *pairs = pl.use_pair && !pl.direct;
     if (launches)
-        *launches = pl.use_pair ? pair_launches(pl.pair) : 2;
+        *launches = pl.direct ? 1 : pl.use_pair ? pair_launches(pl.pair) : 2;
     return NBGB_OK;
 }
 

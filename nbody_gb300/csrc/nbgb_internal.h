@@ -79,6 +79,9 @@ struct ForcePlan {
     // which describes what a forced plan of the same size would run
     int use_pair = 0;
     PairPlan pair;
+    // > 0, with use_pair: the single launch for few bodies instead, with four
+    // times so many targets a CTA (force_direct.cu)
+    int direct = 0;
 };
 
 int plan_force(size_t n, int force_config, int force_nsplit, ForcePlan &pl);
@@ -131,6 +134,15 @@ bool plan_pair(size_t n, int sms, size_t max_bytes, PairPlan &pl);
 int launch_pair(const PairPlan &pl, float4 *force, const float4 *posMass, float eps2,
                 void *workspace, cudaStream_t st, const FusedIntegrate *fi = nullptr);
 int pair_launches(const PairPlan &pl);
+// Few bodies in one launch (force_direct.cu): targets of a CTA / 4, 0: too
+// many bodies (4,864 on 152 SMs, where it takes 11.3 us and pairs 14.2; at
+// 5,472 with 40 targets 15.3, pairs 15.5).  fi: with the reference integrator
+// as a second launch.
+constexpr size_t kMaxDirect = 4864;
+int direct_targets(size_t n, int sms);
+int direct_prepare();
+int launch_direct(size_t n, int targets, unsigned *status, float4 *force, const float4 *posMass,
+                  float eps2, cudaStream_t st, const FusedIntegrate *fi);
 int pair_prepare();  // kernel attributes of the current context
 int pair_device_sms();  // SMs of the current device, attributes set (0: no device)
 // Potential sums with each pair evaluated once (pair_potential.cu): phi[i].w
