@@ -11,10 +11,11 @@
 // the arithmetic outweighs the hand-over.
 //
 // A call in a graph, against the pair and reduction kernels: 64 bodies 4.1 ->
-// 1.6 us, 1,000: 5.7 -> 2.45, 2,048: 7.0 -> 4.0, 3,000: 9.4 -> 6.1, 4,096:
-// 11.0 -> 9.5, 4,864: 14.2 -> 11.3; one launch instead of two from the host:
-// 13.7 -> 9.5 us.  A step of the reference integrator: 1,000 bodies 6.7 ->
-// 3.9 us, 4,096: 12.0 -> 11.3; an FP64 step 8.2 -> 5.4 and 14.2 -> 12.6.
+// 1.6 us, 1,000: 5.7 -> 2.5, 2,048: 7.0 -> 4.1, 3,000: 9.4 -> 6.3, 4,096:
+// 11.0 -> 9.9, 4,864: 14.2 -> 11.4; one launch instead of two from the host:
+// 13.7 -> 8.6 us.  A step of the reference integrator: 1,000 bodies 6.7 ->
+// 3.9 us, 4,096: 12.0 -> 11.2; an FP64 step 8.2 -> 4.1 and 14.2 -> 11.9 (with
+// the integrator's early launch).
 // Errors against 64 bits are the pair kernel's (5.2e-8 to 8.2e-8 rms).
 #include <cuda_runtime.h>
 
@@ -83,7 +84,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     __syncthreads();
     const ulonglong2 *a = reinterpret_cast<const ulonglong2 *>(xy) + warp * kSub + sub;
     const ulonglong2 *b = reinterpret_cast<const ulonglong2 *>(zm) + warp * kSub + sub;
-#pragma unroll 2
+#pragma unroll(KT > 3 ? 1 : 2)
     for (int q = warp * kSub; q < P.np; q += kShares, a += kShares, b += kShares) {
         const ulonglong2 u = *a, v = *b;
 #pragma unroll
@@ -147,19 +148,21 @@ bool prepare_kt() {
 
 }  // namespace
 
-// Targets of a CTA, in fours: as many as give each SM one CTA.  Eight lanes
-// where the number allows it (2,432 bodies 4.5 us; four lanes 4.7), four below
-// 16 (more shares of the sources: 1,000 bodies 2.5 us, 2.9 with eight) and
-// where it is odd.
+// Targets of a CTA, in fours: as many as give each SM one CTA, in eights above
+// 16.  Four lanes below 16 (more shares of the sources: 1,000 bodies 2.5 us,
+// 2.9 with eight), eight from there on (2,432 bodies 4.5 us; four lanes 4.7).
+// 20 and 28 targets on four lanes save 4 and 2 % of a call but take all
+// registers of an SM: the integrator's blocks, which start early, were then
+// all on the two or so SMs without a CTA, and an FP64 step of 3,000 bodies
+// took 11.3 us instead of 8.
 int direct_targets(size_t n, int sms) {
     const size_t fours = (n + (size_t)sms * 4 - 1) / ((size_t)sms * 4);
-    return n <= kMaxDirect && fours <= 8 ? (int)fours : 0;
+    return n <= kMaxDirect && fours <= 8 ? (int)(fours > 4 ? (fours + 1) / 2 * 2 : fours) : 0;
 }
 
 int direct_prepare() {
     return prepare_kt<4, 1>() && prepare_kt<4, 2>() && prepare_kt<4, 3>() && prepare_kt<8, 2>() &&
-                   prepare_kt<4, 5>() && prepare_kt<8, 3>() && prepare_kt<4, 7>() &&
-                   prepare_kt<8, 4>()
+                   prepare_kt<8, 3>() && prepare_kt<8, 4>()
                ? NBGB_OK
                : NBGB_ERR_CUDA;
 }
@@ -179,9 +182,7 @@ int launch_direct(size_t n, int targets, unsigned *status, float4 *force, const 
     case 2: e = launch_kt<4, 2>(P, st); break;
     case 3: e = launch_kt<4, 3>(P, st); break;
     case 4: e = launch_kt<8, 2>(P, st); break;
-    case 5: e = launch_kt<4, 5>(P, st); break;
     case 6: e = launch_kt<8, 3>(P, st); break;
-    case 7: e = launch_kt<4, 7>(P, st); break;
     case 8: e = launch_kt<8, 4>(P, st); break;
     }
     if (e != cudaSuccess)

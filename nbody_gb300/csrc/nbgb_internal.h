@@ -135,7 +135,7 @@ int launch_pair(const PairPlan &pl, float4 *force, const float4 *posMass, float 
                 void *workspace, cudaStream_t st, const FusedIntegrate *fi = nullptr);
 int pair_launches(const PairPlan &pl);
 // Few bodies in one launch (force_direct.cu): targets of a CTA / 4, 0: too
-// many bodies (4,864 on 152 SMs, where it takes 11.3 us and pairs 14.2; at
+// many bodies (4,864 on 152 SMs, where it takes 11.4 us and pairs 14.2; at
 // 5,472 with 40 targets 15.3, pairs 15.5).  fi: with the reference integrator
 // as a second launch.
 constexpr size_t kMaxDirect = 4864;
