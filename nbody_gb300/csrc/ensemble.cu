@@ -857,7 +857,7 @@ inline int sub_eff(const HostSys &h) {
 // item's start-up (2-3 us) is small beside its steps (11 us a set with narrow
 // rows, 30 us with wide ones), many enough that one system alone fills the
 // GPU.  Depends on n only, as does the geometry: rows of 512 targets below
-// 8,192 bodies (more, smaller items, less padding), 1,408 above.
+// 8,192 bodies (more, smaller items, less padding), 1,024 above.
 int sets_per_item(size_t n) {
     if (n < 8192)
         return n < 2048 ? 4 : 2;

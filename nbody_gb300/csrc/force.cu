@@ -854,10 +854,10 @@ static int plan_force_among(size_t n, const std::vector<int> &cands, int force_n
 // Evaluate pairs once (force_pair.cu) up to kMaxPairForce bodies: 14-16 FP32
 // operations for two interactions against 23.  Microseconds a call, pairs
 // against the one-sided plan and its pack launch (back to back in a graph,
-// GB300, uniform ball): N = 300 5.3 / 8.8, 1,000 5.9 / 10.1, 2,048 7.0 / 12,
-// 4,096 11 / 15, 8,192 27 / 37, 10,007 37 / 53, 16,384 85 / 110, 131,072
-// 4,415 / 5,820; equal masses (Plummer) 100,003 2,390 / 3,480, 131,072 4,065
-// / 5,820, 2^20 253,200 / 369,100.  Above the line a phase's pieces (12 N
+// GB300, uniform ball): 5,000 14.8 / 18, 8,192 27 / 37, 10,007 37 / 53, 16,384
+// 81 / 110, 131,072 4,427 / 5,820; equal masses (Plummer) 100,003 2,379 /
+// 3,480, 131,072 4,037 / 5,820, 2^20 254,600 / 369,100.  Few bodies take the
+// single launch of force_direct.cu instead.  Above the line a phase's pieces (12 N
 // bytes a row) take too much workspace.
 // Results of pair plans are closer to 64 bits at every size (3.7e-8 against
 // 8.5e-8 at 100,003).  A plan that would take log-domain pairs refuses

@@ -7,8 +7,8 @@
 // involved are equal), against 11.5-12 for each interaction of the one-sided
 // kernel.  ncu: FMA pipe 82 % busy; the rest are dispatch stalls of
 // three-operand instructions (six of the 16) and the other instructions' issue.
-// GB300, N = 131,072: 4,415 us with mixed masses (3.89e12 interactions/s),
-// 4,065 us with equal ones (4.23e12), against 4,830 us for 8 sources and 8
+// GB300, N = 131,072: 4,427 us with mixed masses (3.88e12 interactions/s),
+// 4,037 us with equal ones (4.26e12), against 4,830 us for 8 sources and 8
 // targets a lane with all source registers shuffled and FP64 atomics, and
 // 5,820 us one-sided.
 //
@@ -22,15 +22,17 @@
 // shuffled but read from shared memory (two 128-bit loads instead of eight
 // shuffles a source pair; each set is stored twice in a row, so lane L + t
 // needs no wrap).  Every instruction beside the FMA-pipe ones costs about as
-// much issue time as one of them, so the tile is as wide in targets as the
-// registers allow (12 targets a lane 4,400 / 4,120 us, 11 4,415 / 4,065, 10
-// 4,515 / 4,040, 8 4,550 / 4,005 at N = 131,072, mixed / equal masses; 3 warps
-// a scheduler with 8 targets were 2 % slower than 2 with 12).  The next set
+// much issue time as one of them, which asks for a tile wide in targets; but
+// the own-row meetings, the pieces and the folds grow with it.  At N = 16,384 /
+// 131,072 / 1,048,576, in us and ms, mixed and equal masses: 11 targets a lane
+// 83.2, 79.7 / 4,415, 4,102 / 280.8, 258.3; 9: 81.7, 77.0 / 4,433, 4,013; 8:
+// 80.8, 77.5 / 4,427, 4,037 / 282.3, 255.0; 7: 81.6, 76.1 / 4,556, 4,147.  The next set
 // comes by cp.async, which holds no registers.
 //
 // Narrow rows (512 bodies, 4 targets a lane) serve n below kNarrowBelow, where
-// rows of 1,408 are too few pieces of work: 14,000 bodies take 64.7 us narrow
-// and 65.4 us wide, 4,096 11.0 and 15.0, 16,384 87.0 and 83.8.
+// rows of 1,024 are too few pieces of work: 12,500 bodies take 52.7 us narrow
+// and 51.2 us wide (equal masses 50.1 and 50.4), 13,000 56.8 and 54.6, 8,192
+// 26.5 and 26.6, 10,007 36.8 and 37.1.
 //
 // Split.  The steps of all (row, set) meetings form one line, and the host
 // cuts it into equal stretches of cost, one per resident CTA: one wave without
@@ -427,9 +429,9 @@ static bool plan_geometry(size_t n, int sms, size_t max_bytes, PairPlan &pl) {
     // beside the pair kernel's CTAs and start early (8,192, 27: 26.6 / 27.5)
     pl.groups8 = pl.ncta / rows + rows / 2 >= 28 && rows <= 16;
     // two bodies a thread where the blocks of one would not be resident
-    // together (16,384 bodies: 86.9 -> 83.0 us, 32,768: 294.7 -> 290.5; with
-    // fewer blocks one is as fast or faster, 1,000: 5.7 / 6.0)
-    pl.each = (long long)nsets * (G::kSet / 32) * (pl.groups8 ? 768 : 384) > sms * 2048LL ? 2 : 1;
+    // together (12,800 bodies: 57.0 -> 53.1 us, 32,768: 294.7 -> 290.5; with
+    // fewer blocks one is as fast or faster: 6,000 16.3 and 16.7)
+    pl.each = (long long)nsets * (G::kSet / 32) > sms * (pl.groups8 ? 2LL : 5LL) ? 2 : 1;
     const size_t tsum =
         align256((size_t)(std::min(rows, kMaxPairRows) + pl.ncta) * 3 * G::kRow * 4);
     const size_t carry = align256((size_t)nsets * G::kSet * 6 * 4);

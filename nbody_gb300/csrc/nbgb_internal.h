@@ -128,7 +128,7 @@ int launch_force(const ForcePlan &pl, float4 *force, const float4 *posMass, cons
 // and the launches (no j-stream; fi as for launch_force, fi->js ignored).
 constexpr int kMaxPairCtas = 512;          // step table in the kernel parameters
 constexpr int kMaxPairRows = 1024;         // rows of a phase
-constexpr size_t kNarrowBelow = 14336;     // sizes that take the narrow rows
+constexpr size_t kNarrowBelow = 12800;     // sizes that take the narrow rows
 constexpr size_t kMaxPairForce = (size_t)1 << 23;  // force(): larger sizes stay one-sided
 bool plan_pair(size_t n, int sms, size_t max_bytes, PairPlan &pl);
 int launch_pair(const PairPlan &pl, float4 *force, const float4 *posMass, float eps2,

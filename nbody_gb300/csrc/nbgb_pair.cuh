@@ -33,7 +33,7 @@ struct Geo {
     static constexpr int kRaw = kSet * 4;                     // floats
     static constexpr size_t kSmem = (size_t)(kHl + kRed + kSrc + kRaw) * 4;
 };
-typedef Geo<4, 11, 2, 2> Wide;
+typedef Geo<4, 8, 2, 2> Wide;
 typedef Geo<4, 4, 2, 2> Narrow;
 
 constexpr float kRange = 1.0995116e12f;  // 2^40

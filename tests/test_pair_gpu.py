@@ -1,7 +1,7 @@
 """Forces with each pair evaluated once (nbgb_force_newton3 at every N, the
 default force at larger N) at the edges of its tiles, against FP64 and the
-one-sided kernel: sets of 128 sources, rows of 512 targets (1,408
-from N = 14,336 on), phases, and the forms for equal masses and
+one-sided kernel: sets of 128 sources, rows of 512 targets (1,024
+from N = 12,800 on), phases, and the forms for equal masses and
 for positions far from the origin."""
 import numpy as np
 import pytest
@@ -32,7 +32,7 @@ def _err(out, pm, eps2, idx=None):
 
 
 @pytest.mark.parametrize("n", [2, 63, 64, 65, 127, 128, 129, 511, 512, 513, 641, 1025, 4097, 14335,
-                               14336, 14463, 14465, 15489])
+                               14336, 14463, 14465, 15489, 12799, 12800, 12801, 13311, 13313])
 def test_edges_of_sets_and_rows(cuda, n):
     pm, _ = nb.ic_uniform_ball(n, 40 + n, 1.0, 0.5, 1.5)
     out = _run(nb.force_newton3, pm, 1e-4)
@@ -60,7 +60,7 @@ def test_phases_against_the_one_sided_kernel(cuda):
     out = _run(nb.force, pm, 1e-4)
     assert nb.last_status() == 0
     idx = np.unique(np.concatenate([np.random.default_rng(2).choice(n, 200, replace=False),
-                                    [0, 1407, 1408, n - 130, n - 1]]))
+                                    [0, 1023, 1024, 1407, 1408, n - 130, n - 1]]))
     assert _err(out, pm, 1e-4, idx) <= TOL_VS_FP64
     one = _run(nb.force, pm, 1e-4, config=ONE_SIDED)
     d = np.linalg.norm(out - one, axis=1) / np.linalg.norm(one, axis=1)
