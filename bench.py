@@ -16,9 +16,12 @@ interaction (src/nbody.cu:1027).
   e2e       the reference-facing drop-in ComputeGravitation_GPU_GB300 with
             HOST buffers: per step pinned H2D of posMass, the call, D2H of the
             forces, all inside a host-clock timed region
-  roofline  the force kernel: 20 N^2 FLOP / its CUDA-event launch time, over
-            the FP32 pipe peak measured by the library's FMA microbenchmark
-            on this GPU (max of scalar and f32x2), plus the MUFU ceiling;
+  roofline  the force launches: the FP32 work they execute / their CUDA-event
+            time, over the FP32 pipe peak measured by the library's FMA
+            microbenchmark on this GPU (max of scalar and f32x2), plus the
+            FMA pipe's issue slots, the MUFU ceiling and, as *_20flop, the
+            reference's 20 N^2 FLOP (more than the peak where each pair is
+            evaluated once);
             `integrate` holds the same for the HBM-bound integrate kernels:
             the FP64 kick+drift and half kick of the resident loop and the
             reference-mode step (algorithmic bytes / CUDA-event time over the
@@ -197,8 +200,8 @@ HBM_FALLBACK_GBS = 6800.0
 
 
 def profiled_traffic(config_name: str, n: int, nsplit: int):
-    """DRAM bytes per force launch measured by ncu for this kernel
-    configuration, N and j-split (nbody_gb300/tuning/force_dram_traffic.json),
+    """DRAM bytes per force evaluation measured by ncu for this kernel
+    configuration ("pairs": all launches of one evaluation), N and j-split (nbody_gb300/tuning/force_dram_traffic.json),
     else None."""
     try:
         table = json.load(open(TRAFFIC_TABLE))
@@ -338,8 +341,21 @@ def run_gb300(args, ws, rank, local):
         sysm.sync_velocities()
         hk_ms.append(sysm.last_integrate_ms()[1])
     cfg, nsplit = sysm.plan()
-    cfg_name = nb.force_config_names()[cfg] if args.force == 'onesided' else 'newton3'
+    kind, force_launches = nb.force_kind(n)
+    cfg_name = "pairs"
+    if args.force == "newton3":
+        kind = "pairs"
+    elif kind == "pairs" or force_launches == 1:
+        cfg_name = kind if kind == "pairs" else "direct"
+    else:
+        cfg_name = nb.force_config_names()[cfg]
+    if cfg_name in ("pairs", "direct"):
+        nsplit = 1
     traffic = profiled_traffic(cfg_name, n, nsplit)
+    # executed per interaction (equal masses): a pair is 14 FMA-pipe operations
+    # and 23 FLOP for two interactions, one-sided 12 operations and 18 FLOP
+    slots, flop = (7.0, 11.5) if kind == "pairs" else (12.0, 18.0)
+    rate = float(n) * float(n) / (kernel_ms * 1e-3)
     sysm.close()
     integrate = integrate_roofline(n, kd_ms, hk_ms,
                                    reference_step_ms(n, dev, torch.cuda.current_stream(), flush))
@@ -378,9 +394,12 @@ def run_gb300(args, ws, rank, local):
                    "nsplit": nsplit,
                    "l2": "flushed between steps (256 MiB read outside the step events)",
                    "parallelism": f"replicas x{ws}"},
-        "roofline": {"bound": "fp32", "achieved": achieved / 1e12, "peak": fp32_peak / 1e12,
-                     "unit": "TFLOP/s", "frac": achieved / fp32_peak, "traffic": traffic,
-                     "traffic_unit": "bytes per launch (ncu dram read+write, "
+        "roofline": {"bound": "fp32", "achieved": flop * rate / 1e12, "peak": fp32_peak / 1e12,
+                     "unit": "TFLOP/s", "frac": flop * rate / fp32_peak,
+                     "fma_pipe_frac": slots * rate / (fp32_peak / 2),
+                     "achieved_20flop": achieved / 1e12, "frac_20flop": achieved / fp32_peak,
+                     "traffic": traffic,
+                     "traffic_unit": "bytes per force evaluation (ncu dram read+write, "
                                      "nbody_gb300/tuning/force_dram_traffic.json)",
                      "algorithmic_bytes": 48 * n,  # read targets + sources, write forces
                      "peak_source": "measured on this GPU by nbgb_measure_peak "
@@ -388,11 +407,12 @@ def run_gb300(args, ws, rank, local):
                                     "TFLOP/s; FMA = 2 FLOP)",
                      "kernel_ms": kernel_ms,
                      "mufu_peak_per_s": mufu,
-                     "mufu_frac": (float(n) * float(n) / (kernel_ms * 1e-3)) / mufu,
+                     "mufu_frac": rate * (0.5 if kind == "pairs" else 1.0) / mufu,
                      "integrate": integrate},
         "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": n * 16,
                 "d2h_bytes_per_step": n * 16},
-        "gpu_launches": 2 * args.steps,  # per step: kick+drift, force
+        # per step: kick+drift and the force's launches
+        "gpu_launches": (1 + force_launches) * args.steps,
         "clocks": clk,
         "wall_s": wall,
     }
@@ -603,9 +623,10 @@ def measure_newton3(args, n, p3, v3, pm_np, dev, ffma, ffma2, fp32_peak, flush):
     return {"value": float(n) * n * args.steps / t / 1e9, "unit": UNIT,
             "ms_per_step": t * 1e3 / args.steps, "force_ms": kms,
             "roofline_20flop_frac": FLOP * float(n) * n / (kms * 1e-3) / fp32_peak,
-            "executed_fp32_frac": 25 * (float(n) * n / 2) / (kms * 1e-3) / fp32_peak,
-            "note": "each pair evaluated once and applied to both bodies (16 FP32 "
-                    "operations = 25 FLOP per pair, FMA = 2, plus one rsqrt); the first "
+            "executed_fp32_frac": 23 * (float(n) * n / 2) / (kms * 1e-3) / fp32_peak,
+            "note": "each pair evaluated once and applied to both bodies (equal masses: 14 "
+                    "FP32 operations = 23 FLOP per pair, FMA = 2, plus one rsqrt); the "
+                    "default force evaluates it the same way; the first "
                     "fraction uses the reference's 20 FLOP per interaction, the second the "
                     "FP32 work actually executed"}
 
