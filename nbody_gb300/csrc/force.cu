@@ -855,8 +855,8 @@ static int plan_force_among(size_t n, const std::vector<int> &cands, int force_n
 // operations for two interactions against 23.  Microseconds a call, pairs
 // against the one-sided plan and its pack launch (back to back in a graph,
 // GB300, uniform ball): 5,000 14.8 / 18, 8,192 27 / 37, 10,007 37 / 53, 16,384
-// 81 / 110, 131,072 4,427 / 5,820; equal masses (Plummer) 100,003 2,379 /
-// 3,480, 131,072 4,037 / 5,820, 2^20 254,600 / 369,100.  Few bodies take the
+// 81 / 110, 131,072 4,256 / 5,820; equal masses (Plummer) 100,003 2,282 /
+// 3,480, 131,072 3,884 / 5,820, 2^20 246,800 / 369,100.  Few bodies take the
 // single launch of force_direct.cu instead.  Above the line a phase's pieces (12 N
 // bytes a row) take too much workspace.
 // Results of pair plans are closer to 64 bits at every size (3.7e-8 against

@@ -7,8 +7,8 @@
 // involved are equal), against 11.5-12 for each interaction of the one-sided
 // kernel.  ncu: FMA pipe 82 % busy; the rest are dispatch stalls of
 // three-operand instructions (six of the 16) and the other instructions' issue.
-// GB300, N = 131,072: 4,427 us with mixed masses (3.88e12 interactions/s),
-// 4,037 us with equal ones (4.26e12), against 4,830 us for 8 sources and 8
+// GB300, N = 131,072: 4,256 us with mixed masses (4.04e12 interactions/s),
+// 3,884 us with equal ones (4.42e12), against 4,830 us for 8 sources and 8
 // targets a lane with all source registers shuffled and FP64 atomics, and
 // 5,820 us one-sided.
 //
@@ -26,7 +26,8 @@
 // the own-row meetings, the pieces and the folds grow with it.  At N = 16,384 /
 // 131,072 / 1,048,576, in us and ms, mixed and equal masses: 11 targets a lane
 // 83.2, 79.7 / 4,415, 4,102 / 280.8, 258.3; 9: 81.7, 77.0 / 4,433, 4,013; 8:
-// 80.8, 77.5 / 4,427, 4,037 / 282.3, 255.0; 7: 81.6, 76.1 / 4,556, 4,147.  The next set
+// 80.8, 77.5 / 4,427, 4,037 / 282.3, 255.0; 7: 81.6, 76.1 / 4,556, 4,147 (all
+// before the late stretches below).  The next set
 // comes by cp.async, which holds no registers.
 //
 // Narrow rows (512 bodies, 4 targets a lane) serve n below kNarrowBelow, where
@@ -35,8 +36,8 @@
 // 26.5 and 26.6, 10,007 36.8 and 37.1.
 //
 // Split.  The steps of all (row, set) meetings form one line, and the host
-// cuts it into equal stretches of cost, one per resident CTA: one wave without
-// a tail at every N.  A stretch may begin and end inside a set or a row.
+// cuts it into equal stretches of cost, one per resident CTA, and, where there
+// is more work, as many short late ones (stretch_cost).  A stretch may begin and end inside a set or a row.
 // Pieces: the reactions of one stretch's part of one (row, set) meeting
 // (kSet x 3 floats, slot = meeting index + CTA index) and the targets' sums
 // of its part of one row (kRow x 3 floats, slot = row + CTA index); both
@@ -340,10 +341,32 @@ static long long cost_before(int b, int nsets) {
                                                               (long long)nsets));
 }
 
+// Late stretches.  Of the CTAs that share an SM one runs ahead of the other
+// (the scheduler's choice; with equal stretches the SMs held 6.2 of 8 warps on
+// average), and the one left runs alone at four fifths of their rate.  So where
+// there is enough work the resident CTAs' stretches are 92 % of it, and as
+// many short ones start as the first of them end.  N = 131,072, mixed and
+// equal masses: all of it at once 4,424 and 4,037 us; 96 % 4,340, 3,920;
+// 94 % 4,297, 3,879; 92 % 4,256, 3,884; 90 % 4,266, 3,893; 88 % 4,275, 4,116;
+// two or three equal stretches a CTA 4,351, 3,973 and 4,329, 3,957; a third
+// wave 4,267, 3,890.  40,000 bodies 429 -> 415 us, 24,576 167.2 -> 165.8, but
+// 20,000 115.7 -> 117.6: the line is at 240 steps a CTA (about 24,000 bodies).
+constexpr int kLateSteps = 240;
+
+// Cost of the first c of ncta stretches, the first `slots` of them resident.
+static long long stretch_cost(long long total, int c, int ncta, int slots) {
+    if (ncta <= slots)
+        return total * c / ncta;
+    const long long early = total * 23 / 25;
+    return c <= slots ? early * c / slots
+                      : early + (total - early) * (c - slots) / (ncta - slots);
+}
+
 // First steps of ncta stretches over rows row0..row1-1, and the end.  parts >
 // 0: every meeting is cut into that many stretches of its own.
 template <class G>
-static void cut_steps(int row0, int row1, int nsets, int ncta, int parts, unsigned *step) {
+static void cut_steps(int row0, int row1, int nsets, int ncta, int slots, int parts,
+                      unsigned *step) {
     const unsigned end = (unsigned)((meetings_before<G>(row1, nsets) -
                                      meetings_before<G>(row0, nsets))
                                     << 5);
@@ -358,7 +381,7 @@ static void cut_steps(int row0, int row1, int nsets, int ncta, int parts, unsign
     long long begin = 0;                          // the row's first cost
     long long next = cost_before<G>(row + 1, nsets) - c0;
     for (int c = 0; c < ncta; c++) {
-        const long long at = total * c / ncta;
+        const long long at = stretch_cost(total, c, ncta, slots);
         while (at >= next && row + 1 < row1) {
             steps += 32LL * (nsets - row * G::kRowSets);
             row++;
@@ -432,6 +455,9 @@ static bool plan_geometry(size_t n, int sms, size_t max_bytes, PairPlan &pl) {
     // together (12,800 bodies: 57.0 -> 53.1 us, 32,768: 294.7 -> 290.5; with
     // fewer blocks one is as fast or faster: 6,000 16.3 and 16.7)
     pl.each = (long long)nsets * (G::kSet / 32) > sms * (pl.groups8 ? 2LL : 5LL) ? 2 : 1;
+    pl.slots = pl.ncta;
+    if (!max_bytes && cost >= (long long)slots * pair::kLateSteps * pair::kCostBoth)
+        pl.ncta = std::min(2 * slots, kMaxPairCtas);
     const size_t tsum =
         align256((size_t)(std::min(rows, kMaxPairRows) + pl.ncta) * 3 * G::kRow * 4);
     const size_t carry = align256((size_t)nsets * G::kSet * 6 * 4);
@@ -498,11 +524,12 @@ static int launch_geometry(const PairPlan &pl, float4 *force, const float4 *posM
             return NBGB_ERR_WORKSPACE;
         const long long total =
             pair::cost_before<G>(P.row1, nsets) - pair::cost_before<G>(P.row0, nsets);
-        P.ncta = (int)std::min<long long>(pl.ncta, total / pair::kMinCost);
+        const bool late = total >= (long long)pl.slots * pair::kLateSteps * pair::kCostBoth;
+        P.ncta = (int)std::min<long long>(late ? pl.ncta : pl.slots, total / pair::kMinCost);
         P.parts = pl.parts;
         if (pl.parts)
             P.ncta = pl.ncta;
-        pair::cut_steps<G>(P.row0, P.row1, nsets, P.ncta, pl.parts, P.step);
+        pair::cut_steps<G>(P.row0, P.row1, nsets, P.ncta, pl.slots, pl.parts, P.step);
         const size_t smem = pl.lone ? pair::kLoneSmem : G::kSmem;
         if (launch_dependent(pair::pair_kernel<G>, P.ncta, G::kThreads, smem, st, P) !=
                 cudaSuccess ||

@@ -21,7 +21,8 @@ int current_context(int *device, unsigned long long *ctx_id);
 struct PairPlan {
     size_t n = 0;
     int narrow = 0;           // geometry: narrow rows for small n
-    int ncta = 0;             // stretches (resident CTAs)
+    int ncta = 0;             // stretches, at most
+    int slots = 0;            // resident CTAs; with more stretches the rest are late ones
     int parts = 0;            // > 0: each meeting is so many stretches of its own
     int lone = 0;             // one CTA an SM
     int groups8 = 0;          // eight reduction threads a body (else four)
@@ -126,7 +127,7 @@ int launch_force(const ForcePlan &pl, float4 *force, const float4 *posMass, cons
 // Pairs evaluated once (force_pair.cu): plan for n bodies on a device with
 // `sms` SMs (max_bytes > 0: within that workspace; false when it cannot),
 // and the launches (no j-stream; fi as for launch_force, fi->js ignored).
-constexpr int kMaxPairCtas = 512;          // step table in the kernel parameters
+constexpr int kMaxPairCtas = 640;          // step table in the kernel parameters
 constexpr int kMaxPairRows = 1024;         // rows of a phase
 constexpr size_t kNarrowBelow = 12800;     // sizes that take the narrow rows
 constexpr size_t kMaxPairForce = (size_t)1 << 23;  // force(): larger sizes stay one-sided

@@ -11,9 +11,9 @@
 // lane) against sets of 128 sources read rotated from shared memory, cut into
 // equal stretches of steps, three resident CTAs per SM, as in force_pair.cu.
 // Diagnostics of 262,144 bodies, with all that is around this kernel: 26.5 ms
-// from the one-sided force-and-potential kernel, 8.4 ms from here (4.1e12
-// pairs/s; the MUFU pipe alone allows 4.7e12); 65,536: 1,780 and 627 us;
-// 20,000: 288 and 154; 8,192: 128 and 117; 4,096: 108 and 106; 1,000: 104 and 97.
+// from the one-sided force-and-potential kernel, 8.0 ms from here (4.3e12
+// pairs/s; the MUFU pipe alone allows 4.7e12); 65,536: 1,780 and 570 us;
+// 20,000: 288 and 119; 8,192: 128 and 117; 4,096: 108 and 106; 1,000: 104 and 97.
 // Against 64 bits both are off by 5.5e-9 of the energy at 262,144 (the MUFU
 // rsqrt's mean error), and where the self pair weighs (eps2 = 0.01, N = 20,000)
 // 2.8e-8 there and 5e-9 here.
@@ -31,24 +31,36 @@ namespace {
 
 typedef pair::Geo<4, 8, 2, 3> PG;
 constexpr int kFoldSets = 2;  // 256 sources between folds
+// From so many steps a CTA on, 12 % of the work is left to late CTAs, which fill
+// the SMs as their first CTAs end (force_pair.cu): 262,144 bodies 8,350 us
+// without, 8,240 with 4 %, 8,120 with 8, 7,990 with 12, 8,020 with 16, 8,045
+// with 20; 65,536: 591 and 570.
+constexpr int kLateSteps = 240;
 constexpr int kMinSteps = 16;  // of a CTA; with 8, 4,096 bodies take longer (more pieces)
 
 struct PotParams {
     const float4 *__restrict__ pm;
     float *__restrict__ tsum;  // [row + CTA][kRow]
-    int n, nsets, rows, ncta;
-    unsigned q, r;  // CTA c takes q steps, one more if c < r
+    int n, nsets, rows, ncta, slots;
+    // The first `slots` CTAs take the first `early` steps, the late ones the
+    // rest: q[] steps each, one more for the first r[] of them
+    unsigned early, q[2], r[2];
     float eps2;
 };
 
 __device__ __forceinline__ unsigned first_step(const PotParams &P, int c) {
-    return (unsigned)c * P.q + min((unsigned)c, P.r);
+    const int w = c > P.slots;
+    const unsigned k = (unsigned)(c - (w ? P.slots : 0));
+    return (w ? P.early : 0u) + k * P.q[w] + min(k, P.r[w]);
 }
 
 // the CTA that takes step s
 __device__ __forceinline__ int holder(const PotParams &P, unsigned s) {
-    const unsigned longer = P.r * (P.q + 1);
-    return (int)(s < longer ? s / (P.q + 1) : P.r + (s - longer) / P.q);
+    const int w = s >= P.early;
+    s -= w ? P.early : 0u;
+    const unsigned longer = P.r[w] * (P.q[w] + 1);
+    return (w ? P.slots : 0) +
+           (int)(s < longer ? s / (P.q[w] + 1) : P.r[w] + (s - longer) / P.q[w]);
 }
 
 __global__ void __launch_bounds__(PG::kThreads, PG::kCtas)
@@ -184,10 +196,19 @@ PotParams params(size_t n, int sms) {
     P.nsets = (int)((n + PG::kSet - 1) / PG::kSet);
     P.rows = (int)((n + PG::kRow - 1) / PG::kRow);
     const long long steps = 32 * pair::meetings_before<PG>(P.rows, P.nsets);
-    P.ncta = (int)std::max<long long>(
+    P.ncta = P.slots = (int)std::max<long long>(
         1, std::min<long long>((long long)sms * PG::kCtas, steps / kMinSteps));
-    P.q = (unsigned)(steps / P.ncta);
-    P.r = (unsigned)(steps % P.ncta);
+    long long part[2] = {steps, 0};
+    if (steps >= (long long)P.slots * kLateSteps) {
+        part[0] = steps * 88 / 100;
+        part[1] = steps - part[0];
+        P.ncta = 2 * P.slots;
+    }
+    P.early = (unsigned)part[0];
+    for (int w = 0; w < 2; w++) {
+        P.q[w] = (unsigned)(part[w] / P.slots);
+        P.r[w] = (unsigned)(part[w] % P.slots);
+    }
     return P;
 }
 

@@ -32,7 +32,7 @@ def _err(out, pm, eps2, idx=None):
 
 
 @pytest.mark.parametrize("n", [2, 63, 64, 65, 127, 128, 129, 511, 512, 513, 641, 1025, 4097, 14335,
-                               14336, 14463, 14465, 15489, 12799, 12800, 12801, 13311, 13313])
+                               14336, 14463, 14465, 15489, 12799, 12800, 12801, 13311, 13313, 23935, 24577])
 def test_edges_of_sets_and_rows(cuda, n):
     pm, _ = nb.ic_uniform_ball(n, 40 + n, 1.0, 0.5, 1.5)
     out = _run(nb.force_newton3, pm, 1e-4)

@@ -1,5 +1,6 @@
 """The diagnostics' potential, each pair evaluated once: at the edges of sets
-(128) and rows (1,024) and with several stretches per row, against FP64 sums."""
+(128) and rows (1,024), with several stretches per row and with late stretches
+(34,011), against FP64 sums."""
 import numpy as np
 import pytest
 
@@ -10,7 +11,7 @@ import nbody_gb300 as nb
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n", [1, 2, 127, 129, 1023, 1024, 1025, 2049, 7000, 20011])
+@pytest.mark.parametrize("n", [1, 2, 127, 129, 1023, 1024, 1025, 2049, 7000, 20011, 34011])
 @pytest.mark.parametrize("equal", [True, False])
 def test_potential_energy(cuda, n, equal):
     rng = np.random.default_rng(n)
