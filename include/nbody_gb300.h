@@ -85,9 +85,9 @@ NBGB_API size_t nbgb_force_workspace_bytes(size_t N);
  * every fourth source pair's m r^-3 as 2^(log2 m - 1.5 log2 r^2), which needs
  * m >= 0.  A negative (or NaN) mass gives NaN forces and sets
  * NBGB_STATUS_NEGATIVE_MASS; for signed masses force an rsqrt-only
- * configuration through nbgb_force_ex.  Larger N (nbgb_force_kind) evaluate
- * each pair once instead, with the same rule for the masses.  Results are
- * deterministic in both forms.
+ * configuration through nbgb_force_ex.  The default force evaluates few bodies
+ * in one launch and more of them pair by pair (nbgb_force_kind), with the
+ * same rule for the masses.  Results are deterministic in every form.
  */
 NBGB_API int nbgb_force(float *force, const float *posMass, float softeningSquared, size_t N,
                         void *workspace, size_t workspace_bytes, void *stream);

@@ -108,7 +108,8 @@ def force_plan(N: int, config: int = -1, nsplit: int = -1):
 
 def force_kind(N: int):
     """("pairs" or "onesided", kernel launches) of force() for N bodies:
-    whether it evaluates each pair once or runs the one-sided plan."""
+    whether it evaluates each pair once, both sides of each in a single launch
+    (1, few bodies) or runs the one-sided plan (2)."""
     p, k = ctypes.c_int(), ctypes.c_int()
     check(load().nbgb_force_kind(N, ctypes.byref(p), ctypes.byref(k)), "nbgb_force_kind")
     return ("pairs" if p.value else "onesided"), k.value
@@ -163,8 +164,8 @@ def force(posMass, softeningSquared: float, out=None, stream=None, workspace: Wo
           config: int = -1, nsplit: int = -1):
     """F_i = sum_j m_j d_ij / (|d_ij|^2 + eps2)^1.5 for a (N,4) float32 CUDA
     tensor {x,y,z,m}; returns (N,4) {fx,fy,fz,0}.  config / nsplit force a
-    one-sided plan (-1, -1: the library's choice, which evaluates each pair
-    once at larger N; -1: the planner's choice; nsplit > 0 splits every i-block's
+    one-sided plan (-1, -1: the library's choice, one launch for few
+    bodies, each pair once for more; -1: the planner's choice; nsplit > 0 splits every i-block's
     sources nsplit ways, nsplit <= -2 only the i-blocks left over after
     whole rounds of CTA slots, -nsplit ways)."""
     torch = _torch()

@@ -6,9 +6,10 @@ For each N (a seeded Plummer sphere) it times the planner's own plan for
 nbgb_force and a grid of forced plans (configuration x slice count: every
 i-block split s ways, and from N = 131,072 also whole i-blocks for the whole
 rounds of CTA slots plus the leftover i-blocks split s ways, nsplit = -s),
-each as a CUDA graph of `calls` back-to-back calls (the pack and force
-kernels, no host work in the timed region), and prints one JSON line per N:
-the planner's plan and time, the fastest three grid plans and the planner's
+each as a CUDA graph of `calls` back-to-back calls (all its kernels,
+no host work in the timed region), and prints one JSON line per N:
+the default force's time (one launch, or pairs, up to 2^23 bodies), the
+one-sided plan of that N, the fastest three grid plans and the planner's
 time over the fastest.  Plans change speed only; results differ at most by
 rounding.
 """
