@@ -880,8 +880,8 @@ void pair_shape(size_t n, HostSys &h) {
 // Sizes evaluated by warp tasks.  Microseconds a tick of 1,024 systems (one
 // system), tasks / rows / the one-sided queue's tuned plan: N = 91 29 / 52 /
 // 46 (17 / 19 / 21), 362 104 / 166 / 124 (26 / 19 / 32), 724 304 / 403 / 309
-// (38 / 20 / 43), 1,280 728 / 809 / 1,011 (57 / 39 / 102): above the line rows
-// are little slower for many systems and much faster for few.
+// (38 / 20 / 43), 1,100 635 / 595 / 1,003 (49 / 39 / 106), 1,280 746 / 694 /
+// 1,010 (53 / 40 / 106), and of 953 systems of 1,448 1,011 / 882 / 925.
 constexpr size_t kTaskBelow = 1024;
 
 // The pair plan of n bodies if its scratch is at most max_floats.
