@@ -957,7 +957,9 @@ int plan_force_within(size_t n, size_t max_bytes, ForcePlan &pl) {
 
 int launch_force(const ForcePlan &pl, float4 *force, const float4 *posMass, const float4 *jstream,
                  float eps2, void *workspace, cudaStream_t stream, const FusedIntegrate *fi) {
-    if (pl.direct)
+    // (force may be posMass itself: the pair kernel has read every body before
+    // a force is written, the CTAs of the direct one have not)
+    if (pl.direct && (force + pl.n <= posMass || posMass + pl.n <= force))
         return launch_direct(pl.n, pl.direct, pl.pair.status, force, posMass, eps2, stream, fi);
     if (pl.use_pair)
         return launch_pair(pl.pair, force, posMass, eps2, workspace, stream, fi);

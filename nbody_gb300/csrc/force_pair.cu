@@ -73,7 +73,7 @@ namespace pair {
 
 // The bodies of the system.
 struct Source {
-    const float4 *__restrict__ pm;
+    const float4 *pm;               // (may be where the forces go)
     int n;
     float eps2;
     int short_ok;                   // eps2 in the short forms' range
@@ -144,7 +144,7 @@ struct ReduceParams {
     Params p;
     float *__restrict__ carry;  // [6][npad]: sums of bodies whose rows come later
     size_t npad;
-    float4 *__restrict__ force;
+    float4 *force;
     FusedIntegrate fi;  // fi.vel == nullptr: forces only
 };
 

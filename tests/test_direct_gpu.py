@@ -78,3 +78,19 @@ def test_special_values(cuda, what, value):
     assert np.array_equal(np.isfinite(out), np.isfinite(one))
     ok = np.isfinite(one)
     assert np.allclose(out[ok], one[ok], rtol=2e-5, atol=2e-6 * np.abs(one[ok]).max())
+
+
+@pytest.mark.parametrize("n", [2, 64, 1000, 2432, 4864, 4865, 20000, 270000])
+def test_in_place(cuda, n):
+    """Forces written over the bodies they are computed from, as the one-sided
+    kernel takes them: every body is read before the first force is written
+    (at 270,000 bodies a phase's bodies before its forces)."""
+    import torch
+    pm, _ = nb.ic_uniform_ball(n, 7 + n, 1.0, 0.5, 1.5)
+    want = nb.force_newton3(torch.from_numpy(pm).cuda(), 1e-4)
+    both = torch.from_numpy(pm).cuda()
+    nb.force(both, 1e-4, out=both)
+    assert torch.equal(both, want)
+    row = torch.from_numpy(pm).cuda()
+    assert nb.ComputeGravitation_GPU_GB300(row, row, 1e-4, n) > 0.0
+    assert torch.equal(row, want)
