@@ -316,6 +316,9 @@ int sym_block_bodies() { return sym::Geo<sym::kWideKI>::kBlock; }
 
 namespace {
 
+// More bodies are refused: 2^31 - 1 pairs of 2,048-body blocks.
+constexpr size_t kMaxNewton3 = (size_t)65535 * 2048;
+
 int device_sms() {
     const int sms = nbgb::pair_device_sms();
     return sms > 0 ? sms : 152;  // no device: plan for a GB300
@@ -345,6 +348,8 @@ NBGB_API int nbgb_force_newton3(float *force, const float *posMass, float soften
         return NBGB_ERR_CUDA;
     if (!workspace || workspace_bytes < pl.workspace_bytes || ((uintptr_t)workspace & 255u))
         return NBGB_ERR_WORKSPACE;
+    if (N > kMaxNewton3)
+        return NBGB_ERR_TOO_LARGE;
     return nbgb::launch_pair(pl, (float4 *)force, (const float4 *)posMass, softeningSquared,
                              workspace, (cudaStream_t)stream);
 }

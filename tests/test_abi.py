@@ -83,3 +83,13 @@ def test_host_error_stats_match_numpy():
     mx, rms = nb.force_error_stats(g["force_aos"], g["force_f64"][:, :3])
     mx2, rms2 = O.per_body_rel_error(g["force_aos"], g["force_f64"])
     assert abs(mx - mx2) <= 1e-12 and abs(rms - rms2) <= 1e-12
+
+
+def test_newton3_refuses_more_bodies_than_it_evaluates():
+    """Refused before anything is launched or read (the addresses are none)."""
+    lib = _lib.load()
+    limit = 65535 * 2048
+    for n in (limit + 1, 1 << 28, 1 << 30):
+        assert lib.nbgb_force_newton3_workspace_bytes(n) > 0
+        assert lib.nbgb_force_newton3(1 << 20, 1 << 20, 1e-4, n, 1 << 20, 1 << 62, None) == -7, n
+        assert lib.nbgb_force_newton3(1 << 20, 1 << 20, 1e-4, n, 1 << 20, 0, None) == -2, n
