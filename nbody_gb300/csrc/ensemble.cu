@@ -449,9 +449,9 @@ constexpr size_t kPairSmem = Wide::kSmem > Narrow::kSmem ? Wide::kSmem : Narrow:
 constexpr int kBodyBlock = 64;  // bodies of one entry of the block map, two a reduction thread
 
 struct PairParams {
-    const Desc *__restrict__ desc;
-    const int4 *__restrict__ items;  // {system, row, chunk, 0} or {-1, first task, 0, 0}
-    const int2 *__restrict__ tasks;  // {system, tile}, four to an item ({-1, 0}: none)
+    const Desc *desc;
+    const int4 *items;  // {system, row, chunk, 0} or {-1, first task, 0, 0}
+    const int2 *tasks;  // {system, tile}, four to an item ({-1, 0}: none)
     int n_items, pass;
     unsigned *head;                  // zeroed by ens_drift
     const float4 *pm;
@@ -621,9 +621,9 @@ __global__ void __launch_bounds__(kPairCtaThreads, 2) ens_pair_kernel(PairParams
 // Opening half kick and drift of moving systems, FP32 positions of all;
 // zeroes the item queues.
 __global__ void __launch_bounds__(256)
-    ens_drift_kernel(const Desc *__restrict__ desc, const int2 *__restrict__ blocks, int n_blocks,
-                     double *__restrict__ x64, size_t stride, const float *__restrict__ mass,
-                     const float4 *__restrict__ acc, float4 *__restrict__ pm,
+    ens_drift_kernel(const Desc *desc, const int2 *blocks, int n_blocks,
+                     double *__restrict__ x64, size_t stride, const float *mass,
+                     const float4 *acc, float4 *__restrict__ pm,
                      unsigned *__restrict__ heads, int n_heads, int pass) {
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     grid_dependents_launch();
@@ -736,8 +736,7 @@ __device__ __forceinline__ void reduce_entry(const Desc &d, int blk, const float
 }
 
 __global__ void __launch_bounds__(kReduceThreads)
-    ens_reduce_kernel(const Desc *__restrict__ desc, const int2 *__restrict__ blocks,
-                      const float *__restrict__ scratch, double *__restrict__ x64, size_t stride,
+    ens_reduce_kernel(const Desc *desc, const int2 *blocks, const float *scratch, double *__restrict__ x64, size_t stride,
                       float4 *__restrict__ acc, int pass) {
     grid_dependents_launch();
     grid_dependency_wait();

@@ -30,7 +30,7 @@ namespace {
 constexpr int kWarps = 16, kThreads = 32 * kWarps;
 
 struct DirectParams {
-    const float4 *__restrict__ pm;
+    const float4 *pm;
     float4 *__restrict__ force;
     unsigned *__restrict__ status;  // not null: refuse masses < 0
     int n, np;  // bodies; pairs of sources, a multiple of every kSub
@@ -124,7 +124,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 // The reference integrator after it (the force kernel's CTAs all read
 // positions to the end of their staging).
 __global__ void __launch_bounds__(128)
-    direct_integrate_kernel(const float4 *__restrict__ force, FusedIntegrate fi, int n) {
+    direct_integrate_kernel(const float4 *force, FusedIntegrate fi, int n) {
     grid_dependents_launch();
     grid_dependency_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;

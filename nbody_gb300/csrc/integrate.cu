@@ -70,7 +70,7 @@ __device__ __forceinline__ float drift(float x, float v, float dt) {
 template <bool FUSED_DRIFT>
 __global__ void __launch_bounds__(kIntegrateThreads)
     integrate_reference_kernel(float4 *__restrict__ pm, float4 *__restrict__ vel,
-                               const float4 *__restrict__ force, float dt, float damping, int n,
+                               const float4 *force, float dt, float damping, int n,
                                float4 *__restrict__ js, int js_vpb, int js_log, int npad,
                                unsigned *__restrict__ counters, int ncounters) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -102,8 +102,8 @@ __global__ void __launch_bounds__(kIntegrateThreads)
 // null) body i's j-stream entry.  x64: six SoA components of leading
 // dimension ld (entries n..ld-1 are padding, never touched).
 __global__ void __launch_bounds__(kIntegrateThreads)
-    kick_drift_kernel(double *__restrict__ x64, size_t ld, const float *__restrict__ mass,
-                      const float4 *__restrict__ accel, double kick_dt, double drift_dt, int n,
+    kick_drift_kernel(double *__restrict__ x64, size_t ld, const float *mass,
+                      const float4 *accel, double kick_dt, double drift_dt, int n,
                       float4 *__restrict__ pm, float4 *__restrict__ js, int js_vpb, int js_log,
                       int npad, unsigned *__restrict__ counters, int ncounters) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -140,7 +140,7 @@ __global__ void __launch_bounds__(kIntegrateThreads)
 
 // FP64 kick of body i (one per thread): v += a * kick_dt.
 __global__ void __launch_bounds__(kIntegrateThreads)
-    half_kick_kernel(double *__restrict__ x64, size_t ld, const float4 *__restrict__ accel,
+    half_kick_kernel(double *__restrict__ x64, size_t ld, const float4 *accel,
                      double kick_dt, int n) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     grid_dependents_launch();

@@ -37,7 +37,11 @@ struct PairPlan {
 
 // Launches a kernel with programmatic dependence on the stream's previous
 // kernel: its CTAs may start early, so the kernel must call
-// grid_dependency_wait() before it touches global memory.
+// grid_dependency_wait() before it touches global memory.  What it reads may
+// be written while it is already running, so none of its pointers to const is
+// __restrict__: the compiler would read through the non-coherent path, which
+// holds for data no one writes during the kernel, and may move such a load
+// ahead of the wait.
 template <typename... Args, typename... Vals>
 cudaError_t launch_dependent_n(void (*kernel)(Args...), unsigned grid, unsigned block, size_t smem,
                                cudaStream_t st, const Vals &...vals) {

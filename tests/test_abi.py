@@ -93,3 +93,32 @@ def test_newton3_refuses_more_bodies_than_it_evaluates():
         assert lib.nbgb_force_newton3_workspace_bytes(n) > 0
         assert lib.nbgb_force_newton3(1 << 20, 1 << 20, 1e-4, n, 1 << 20, 1 << 62, None) == -7, n
         assert lib.nbgb_force_newton3(1 << 20, 1 << 20, 1e-4, n, 1 << 20, 0, None) == -2, n
+
+
+def test_kernels_launched_early_do_not_promise_read_only_data():
+    """A kernel launched with programmatic dependence runs while the kernel
+    before it still writes: no pointer to const among its parameters, or in
+    the structs it takes, may be __restrict__ (loads through one may be
+    non-coherent and may move ahead of the wait)."""
+    src = {os.path.basename(p): re.sub(r"//[^\n]*", "", open(p).read())
+           for p in glob.glob(os.path.join(ROOT, "nbody_gb300", "csrc", "*.cu*"))}
+    everything = "\n".join(src.values())
+    kernels = set()
+    for m in re.finditer(r"launch_dependent(?:_n)?\(([^;]*?)\bst\b", everything):
+        kernels |= set(re.findall(r"\b(\w+_kernel)\b", m.group(1)))
+    assert len(kernels) >= 10, kernels
+    read_only = re.compile(r"const\s+[\w:]+\s*\*\s*__restrict__")
+    structs = set()
+    for k in kernels:
+        m = re.search(r"__global__[^;{]*?\b" + k + r"\s*\(([^{]*?)\)\s*\{", everything)
+        assert m, k
+        assert not read_only.search(m.group(1)), (k, m.group(1))
+        structs |= set(re.findall(r"\b(\w*(?:Params|Integrate))\b", m.group(1)))
+    structs |= {"Source"}  # held by the pair kernels' parameters
+    assert {"Params", "ReduceParams", "DirectParams", "PairParams", "FusedIntegrate"} <= structs
+    for name in structs:
+        for text in src.values():
+            if "launch_dependent" not in text and name != "FusedIntegrate":
+                continue
+            for m in re.finditer(r"struct " + name + r" \{(.*?)\n\};", text, flags=re.S):
+                assert not read_only.search(m.group(1)), (name, m.group(1))
