@@ -111,6 +111,7 @@ struct Desc {
     int pair;            // 0 no, 1 narrow rows, 2 wide rows, 3 warp tasks
     int nsets;           // source sets
     int ch;              // sets per item
+    int target_pieces;   // of an item: its targets' sums, and their remainders
     long long react_off, tsum_off;  // into the scratch arena (floats)
 };
 
@@ -551,7 +552,7 @@ __device__ __forceinline__ long long row_piece(int row, int nsets, int ch) {
 struct Item {
     const float4 *pm_;
     float *react_, *tsum_;
-    int n_, row, set, nset, kind;    // kind: the system's Desc::pair, or 3: tasks from `row` on
+    int n_, row, set, nset, pieces, kind;    // kind: the system's Desc::pair, or 3: tasks from `row` on
     float eps2_;
     __device__ __forceinline__ const float4 *pm() const { return pm_; }
     __device__ __forceinline__ int n() const { return n_; }
@@ -562,6 +563,7 @@ struct Item {
         return react_ + (size_t)(s >> 5) * (3 * Narrow::kSet);
     }
     __device__ __forceinline__ float *tsum() const { return tsum_; }
+    __device__ __forceinline__ bool remainder() const { return pieces > 1; }
 };
 
 template <class G>
@@ -572,7 +574,8 @@ __device__ __forceinline__ void set_item(Item &t, const PairParams &P, const Des
     t.pm_ = P.pm + d.body_off;
     t.react_ = P.scratch + d.react_off + g * (3 * G::kSet);
     t.tsum_ = P.scratch + d.tsum_off +
-              (row_piece<G>(row, d.nsets, d.ch) + chunk) * (3 * G::kRow);
+              (row_piece<G>(row, d.nsets, d.ch) + chunk) * (d.target_pieces * 3 * G::kRow);
+    t.pieces = d.target_pieces;
     t.n_ = d.n;
     t.row = row;
     t.set = set;
@@ -681,11 +684,12 @@ __device__ __forceinline__ void reduce_entry(const Desc &d, int blk, const float
     static_assert(kB == 64, "two bodies a lane");
     const int tid = threadIdx.x, group = tid / (3 * 32), comp = (tid / 32) % 3, j = 2 * (tid & 31);
     const int i = blk * kB + j, set = blk * kB / kSet, b = set / G::kRowSets;
-    const int nt = (d.nsets - b * G::kRowSets + d.ch - 1) / d.ch, total = b + nt;
+    const int nt = (d.nsets - b * G::kRowSets + d.ch - 1) / d.ch * d.target_pieces;
+    const int total = b + nt;
     const int q0 = total * group / kReduceGroups, q1 = total * (group + 1) / kReduceGroups;
     const float *react = scratch + d.react_off + (size_t)comp * kSet + (i - set * kSet);
     const float *tsum = scratch + d.tsum_off + (size_t)comp * G::kRow + (i - b * G::kRow) +
-                        row_piece<G>(b, d.nsets, d.ch) * (3 * G::kRow);
+                        row_piece<G>(b, d.nsets, d.ch) * (d.target_pieces * 3 * G::kRow);
     auto piece = [&](int q) {
         return q < b ? react + (pair::meetings_before<G>(q, d.nsets) + set - q * G::kRowSets) *
                                    (3 * kSet)
@@ -839,7 +843,7 @@ struct HostSys {
     bool n3 = false;        // Newton-3 system
     bool sym = false;       // Newton-3 system too large for pair items
     int pair = 0;           // pair system: 1 narrow rows, 2 wide rows, 3 warp tasks
-    int nsets = 0, ch = 0, rows = 0;
+    int nsets = 0, ch = 0, rows = 0, target_pieces = 1;
     size_t react_len = 0, scratch_len = 0;  // floats
     size_t scratch_off = 0;                 // within its group's scratch
     size_t acc_off = 0, acc_len = 0;  // its FP64 sums ([3][npad] doubles)
@@ -873,7 +877,10 @@ void pair_shape(size_t n, HostSys &h) {
     h.ch = sets_per_item(n);
     const size_t meetings = (size_t)nbgb::pair::meetings_before<G>(h.rows, h.nsets);
     h.react_len = meetings * 3 * G::kSet;
-    h.scratch_len = h.react_len + (meetings / h.ch + h.rows) * 3 * G::kRow;  // row_piece
+    // an item of one set is a single fold, which leaves no remainder
+    h.target_pieces = h.ch > 1 ? 2 : 1;
+    h.scratch_len = h.react_len +
+                    (meetings / h.ch + h.rows) * h.target_pieces * 3 * G::kRow;  // row_piece
 }
 
 // Sizes evaluated by warp tasks.  Microseconds a tick of 1,024 systems (one
@@ -901,6 +908,7 @@ bool pair_plan(size_t n, size_t max_floats, HostSys &h) {
     h.nsets = t.nsets;
     h.rows = t.rows;
     h.ch = t.ch;
+    h.target_pieces = t.target_pieces;
     h.react_len = t.react_len;
     h.scratch_len = t.scratch_len;
     return true;
@@ -1045,6 +1053,7 @@ void fill_desc(nbgb_ensemble *e, int slot, Desc &d) {
     d.pair = h.pair;
     d.nsets = h.nsets;
     d.ch = h.ch;
+    d.target_pieces = h.target_pieces;
     d.react_off = (long long)h.scratch_off;
     d.tsum_off = (long long)(h.scratch_off + h.react_len);
 }

@@ -40,7 +40,8 @@
 // is more work, as many short late ones (stretch_cost).  A stretch may begin and end inside a set or a row.
 // Pieces: the reactions of one stretch's part of one (row, set) meeting
 // (kSet x 3 floats, slot = meeting index + CTA index) and the targets' sums
-// of its part of one row (kRow x 3 floats, slot = row + CTA index); both
+// of its part of one row (kRow x 3 floats and as many for what rounding them
+// leaves out, slot = row + CTA index); both
 // numberings grow strictly along the line, so no two pieces share a slot.
 // The reduce kernel adds each body's pieces in a fixed order with compensated
 // FP32 sums and writes the force (and integrates, when asked).  Both kernels
@@ -83,10 +84,13 @@ struct Source {
 struct Params {
     Source src;
     float *__restrict__ react;  // [slot][3][kSet]
-    float *__restrict__ tsum;   // [slot][3][kRow]
+    float *__restrict__ tsum;   // [slot][3 kPieces][kRow]
     int nsets, row0, row1;      // rows of this phase
     int ncta, parts;                // parts > 0: stretches are parts of meetings
     unsigned step[kMaxPairCtas + 1];  // first step of each CTA's stretch
+    // the targets' sums of a stretch and their remainders; a part of a meeting
+    // is one fold and has none
+    __host__ __device__ int target_pieces() const { return parts ? 1 : 2; }
 };
 
 // Row b's part of this CTA's stretch (row_stretch asks for it).
@@ -103,8 +107,10 @@ struct StretchIo {
         return P.react + ((size_t)(s >> 5) + blockIdx.x) * 3 * G::kSet;
     }
     __device__ __forceinline__ float *tsum() const {
-        return P.tsum + ((size_t)(b - P.row0) + blockIdx.x) * 3 * G::kRow;
+        return P.tsum +
+               ((size_t)(b - P.row0) + blockIdx.x) * P.target_pieces() * 3 * G::kRow;
     }
+    __device__ __forceinline__ bool remainder() const { return P.target_pieces() > 1; }
 };
 
 template <class G>
@@ -236,7 +242,7 @@ __global__ void __launch_bounds__(3 * 32 * kGroups)
                      (unsigned)((meetings_before<G>(b + 1, P.nsets) - g0) << 5), tf, tl);
             n_list = base;
             t_first = tf;
-            t_count = tl - tf + 1;
+            t_count = (tl - tf + 1) * P.target_pieces();
         }
     }
     __syncthreads();
@@ -246,7 +252,7 @@ __global__ void __launch_bounds__(3 * 32 * kGroups)
     const float *react = P.react + (size_t)comp * kSet + sub * kB + j;
     const int i = set * kSet + sub * kB + j;
     const float *tsum = P.tsum + (size_t)comp * G::kRow + (i - b * G::kRow) +
-                        (size_t)(b - P.row0 + tf) * 3 * G::kRow;
+                        (size_t)(b - P.row0 + tf) * P.target_pieces() * 3 * G::kRow;
     auto piece = [&](int q) {
         return q < nr ? react + (size_t)list[q] * 3 * kSet
                       : tsum + (size_t)(q - nr) * 3 * G::kRow;
@@ -410,9 +416,9 @@ static size_t react_bytes(int row0, int row1, int nsets, int ncta) {
 
 // Rows of the phase that starts at `row`: as many as fit (0: not even one).
 template <class G>
-static int phase_end(int row, int rows, int nsets, int ncta, size_t room) {
+static int phase_end(int row, int rows, int nsets, int ncta, int max_rows, size_t room) {
     int end = row;
-    while (end < rows && end - row < kMaxPairRows &&
+    while (end < rows && end - row < max_rows &&
            react_bytes<G>(row, end + 1, nsets, ncta) <= room)
         end++;
     return end;
@@ -458,26 +464,27 @@ static bool plan_geometry(size_t n, int sms, size_t max_bytes, PairPlan &pl) {
     pl.slots = pl.ncta;
     if (!max_bytes && cost >= (long long)slots * pair::kLateSteps * pair::kCostBoth)
         pl.ncta = std::min(2 * slots, kMaxPairCtas);
-    const size_t tsum =
-        align256((size_t)(std::min(rows, kMaxPairRows) + pl.ncta) * 3 * G::kRow * 4);
+    // (a small workspace holds few rows' pieces at a time, which need few
+    // places for the targets' sums)
+    pl.max_rows = max_bytes ? 64 : kMaxPairRows;
+    const size_t tsum = align256((size_t)(std::min(rows, pl.max_rows) + pl.ncta) *
+                                 (pl.parts ? 3 : 6) * G::kRow * 4);
     const size_t carry = align256((size_t)nsets * G::kSet * 6 * 4);
     const size_t all = align256(react_bytes<G>(0, rows, nsets, pl.ncta));
     // a phase of 256 MiB of pieces is about 16 ms of work; always at least
     // four rows
     size_t room = std::max((size_t)256 << 20, (size_t)4 * (nsets + pl.ncta) * 3 * G::kSet * 4);
     if (max_bytes) {
-        if (rows <= kMaxPairRows && all + tsum <= max_bytes)
+        if (rows <= pl.max_rows && all + tsum <= max_bytes)
             room = std::min(room, max_bytes - tsum);
         else if (max_bytes > tsum + carry)
             room = std::min(room, (max_bytes - tsum - carry) & ~(size_t)255);
         else
             return false;
     }
-    const bool one = rows <= kMaxPairRows && all <= room;
-    if (!one)
-        pl.parts = 0;
-    if (!one && phase_end<G>(0, rows, nsets, pl.ncta, room) == 0)
-        return false;
+    const bool one = rows <= pl.max_rows && all <= room;
+    if (!one && (pl.parts || phase_end<G>(0, rows, nsets, pl.ncta, pl.max_rows, room) == 0))
+        return false;  // (parts are at most `slots` pieces, always one phase)
     pl.react_bytes = one ? all : room;
     pl.off_react = 0;
     pl.off_tsum = align256(pl.react_bytes);
@@ -519,7 +526,7 @@ static int launch_geometry(const PairPlan &pl, float4 *force, const float4 *posM
     R.fi = fi ? *fi : FusedIntegrate{};
     R.fi.js = nullptr;
     for (P.row0 = 0; P.row0 < rows; P.row0 = P.row1) {
-        P.row1 = phase_end<G>(P.row0, rows, nsets, pl.ncta, pl.react_bytes);
+        P.row1 = phase_end<G>(P.row0, rows, nsets, pl.ncta, pl.max_rows, pl.react_bytes);
         if (P.row1 == P.row0)
             return NBGB_ERR_WORKSPACE;
         const long long total =
@@ -544,7 +551,7 @@ static int launches_geometry(const PairPlan &pl) {
     const int nsets = pair::sets_of<G>(pl.n), rows = pair::rows_of<G>(pl.n);
     int k = 0;
     for (int row = 0; row < rows; k++) {
-        const int end = phase_end<G>(row, rows, nsets, pl.ncta, pl.react_bytes);
+        const int end = phase_end<G>(row, rows, nsets, pl.ncta, pl.max_rows, pl.react_bytes);
         if (end == row)
             break;
         row = end;

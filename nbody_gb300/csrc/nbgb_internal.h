@@ -27,6 +27,7 @@ struct PairPlan {
     int lone = 0;             // one CTA an SM
     int groups8 = 0;          // eight reduction threads a body (else four)
     int each = 1;             // bodies of a reduction thread
+    int max_rows = 0;         // rows of one phase, at most
     size_t react_bytes = 0;   // reaction pieces of one phase, at most
     size_t off_react = 0, off_tsum = 0, off_carry = 0;
     size_t workspace_bytes = 0;

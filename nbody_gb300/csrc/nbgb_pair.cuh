@@ -172,7 +172,8 @@ __device__ __forceinline__ void store_source(float *buf, int j, float4 v) {
 // needed: pm(), n(), eps2(), short_ok() (eps2 in the short forms' range),
 // status() (not null: refuse masses < 0), react(s) (the piece of step s's
 // meeting, not asked for one-sided ones), tsum() (the targets' piece, 3 x
-// kRow).  SHARE: the last row may fill only some warps' targets; it meets only
+// kRow), remainder() (whether what rounding the piece to one float leaves out
+// follows it; a stretch with a single fold leaves nothing).  SHARE: the last row may fill only some warps' targets; it meets only
 // its own sets, one-sided, and warps without targets of their own then take a
 // share of the others' steps (one or two full warps: 4 or 2 shares).
 template <class G, bool SHARE, class Io>
@@ -355,7 +356,12 @@ __device__ __forceinline__ void row_stretch(const Io &io, float *smem, int b, in
                     comp_add(hi, lo, hl[(6 * k + c) * NT + tid + 32 * full * q]);
                     lo += hl[(6 * k + 3 + c) * NT + tid + 32 * full * q];
                 }
-                out[c * G::kRow + tile * 32 * KI + lane + 32 * k] = hi + lo;
+                float sum, rest;
+                two_sum(hi, lo, sum, rest);
+                float *o = out + c * G::kRow + tile * 32 * KI + lane + 32 * k;
+                o[0] = sum;
+                if (io.remainder())
+                    o[3 * G::kRow] = rest;
             }
     }
     // the next row's staging reuses buffers others may still be reading

@@ -40,7 +40,7 @@ constexpr int kMinSteps = 16;  // of a CTA; with 8, 4,096 bodies take longer (mo
 
 struct PotParams {
     const float4 *__restrict__ pm;
-    float *__restrict__ tsum;  // [row + CTA][kRow]
+    float *__restrict__ tsum;  // [row + CTA][sums, remainders][kRow]
     int n, nsets, rows, ncta, slots;
     // The first `slots` CTAs take the first `early` steps, the late ones the
     // rest: q[] steps each, one more for the first r[] of them
@@ -162,10 +162,14 @@ __global__ void __launch_bounds__(PG::kThreads, PG::kCtas)
             set++;
             buf ^= 1;
         }
-        float *out = P.tsum + ((size_t)b + cta) * PG::kRow + warp * 32 * KI + lane;
+        float *out = P.tsum + ((size_t)b + cta) * 2 * PG::kRow + warp * 32 * KI + lane;
 #pragma unroll
-        for (int k = 0; k < KI; k++)
-            out[32 * k] = hi[k] + lo[k];
+        for (int k = 0; k < KI; k++) {
+            float sum, rest;
+            two_sum(hi[k], lo[k], sum, rest);
+            out[32 * k] = sum;
+            out[PG::kRow + 32 * k] = rest;
+        }
     }
 }
 
@@ -180,10 +184,10 @@ __global__ void __launch_bounds__(256)
     const unsigned a = (unsigned)(pair::meetings_before<PG>(b, P.nsets) << 5);
     const unsigned e = (unsigned)(pair::meetings_before<PG>(b + 1, P.nsets) << 5);
     const int c0 = holder(P, a), c1 = holder(P, e - 1);
-    const float *piece = P.tsum + ((size_t)b + c0) * PG::kRow + (i - b * PG::kRow);
+    const float *piece = P.tsum + ((size_t)b + c0) * 2 * PG::kRow + (i - b * PG::kRow);
     float hi = 0.f, lo = 0.f;
 #pragma unroll 8
-    for (int c = c0; c <= c1; c++, piece += PG::kRow)
+    for (int c = 2 * c0; c <= 2 * c1 + 1; c++, piece += PG::kRow)
         comp_add(hi, lo, *piece);
     // the self pair as the loop evaluates it
     comp_add(hi, lo, -0.5f * (P.pm[i].w * rsqrt_mufu(P.eps2)));
@@ -216,7 +220,7 @@ PotParams params(size_t n, int sms) {
 
 size_t potential_workspace_bytes(size_t n, int sms) {
     const PotParams P = params(n, sms);
-    return (size_t)(P.rows + P.ncta) * PG::kRow * 4;
+    return (size_t)(P.rows + P.ncta) * 2 * PG::kRow * 4;
 }
 
 int launch_potential(size_t n, int sms, const float4 *posMass, float eps2, void *workspace,

@@ -93,3 +93,18 @@ def test_groups_beyond_the_scratch_arena(cuda):
         err = np.linalg.norm(a[idx, :3] - f, axis=1) / np.linalg.norm(f, axis=1)
         assert err.max() <= TOL_VS_FP64
     e.close()
+
+
+@pytest.mark.parametrize("n", [1500, 20000, 70000])
+def test_partial_sums_keep_their_remainders(cuda, n):
+    from test_pair_gpu import cancelling
+    pm, _, want = cancelling(n, 512 if n < 8192 else 1024)
+    e = nb.Ensemble(n, 1, 1e-20, tuning=None)
+    p = pm[:, :3].astype(np.float64)
+    slot = e.add(p, np.zeros_like(p), pm[:, 3].copy(), 0.01, 3)
+    e.tick(1)
+    e.synchronize()
+    a = e.get_state(slot)[2][:512]
+    assert np.all(np.abs(a[:, 0] - want) <= 2.0 ** -23 * want), a[:, 0] - want
+    assert np.all(a[:, 1:] == 0)
+    e.close()

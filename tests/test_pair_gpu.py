@@ -152,3 +152,30 @@ def test_negative_masses_stay_refused_by_the_stream_ordered_force(cuda):
 def test_whole_row_slice_is_the_default_force(cuda, n):
     pm, _ = nb.ic_uniform_ball(n, 8, 1.0, 0.5, 1.5)
     assert np.array_equal(_run(nb.force_rows, pm, 1e-4, 0, n), _run(nb.force, pm, 1e-4))
+
+
+def cancelling(n, row):
+    """n bodies whose forces on the first `row` (massless, at the origin) are
+    exact in every partial sum that keeps its remainder: sources at x = 2 and
+    then at x = -2, eps2 lost in r^2 = 4, so every term is mass / 4, and masses
+    of 16 bits that cancel but for one.  128 terms of a chain and the two
+    halves of a fold fit 24 bits; a stretch's sum does not.  Returns posMass,
+    eps2 and the exact force."""
+    rng = np.random.default_rng(n)
+    h = (n - row - 1) // 2
+    k = rng.integers(1 << 15, 1 << 16, h)
+    pm = np.zeros((n, 4), np.float32)
+    pm[row:row + h, 0], pm[row:row + h, 3] = 2.0, k
+    pm[row + h:row + 2 * h, 0], pm[row + h:row + 2 * h, 3] = -2.0, k[::-1]
+    pm[row + 2 * h, 0], pm[row + 2 * h, 3] = 2.0, 12345.0
+    pm[:, 3] *= 2.0 ** -16
+    return pm, 1e-20, 12345.0 * 2.0 ** -18
+
+
+@pytest.mark.parametrize("n", [8192, 12799, 16384, 40000, 300000])
+def test_partial_sums_keep_their_remainders(cuda, n):
+    pm, eps2, want = cancelling(n, 512 if n < 12800 else 1024)
+    for fn in (nb.force, nb.force_newton3):
+        out = _run(fn, pm, eps2)[:512]
+        assert np.all(np.abs(out[:, 0] - want) <= 2.0 ** -23 * want), out[:, 0] - want
+        assert np.all(out[:, 1:] == 0)
