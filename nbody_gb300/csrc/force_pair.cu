@@ -453,14 +453,22 @@ static bool plan_geometry(size_t n, int sms, size_t max_bytes, PairPlan &pl) {
     // more shared memory than two can have keeps them from sharing an SM when
     // there is one for each
     pl.lone = pl.ncta <= sms;
-    // eight reduction threads a body where it has many pieces (N = 6,000, 31:
-    // 16.5 us against 17.5 with four), four where their smaller blocks fit
-    // beside the pair kernel's CTAs and start early (8,192, 27: 26.6 / 27.5)
-    pl.groups8 = pl.ncta / rows + rows / 2 >= 28 && rows <= 16;
-    // two bodies a thread where the blocks of one would not be resident
-    // together (12,800 bodies: 57.0 -> 53.1 us, 32,768: 294.7 -> 290.5; with
-    // fewer blocks one is as fast or faster: 6,000 16.3 and 16.7)
-    pl.each = (long long)nsets * (G::kSet / 32) > sms * (pl.groups8 ? 2LL : 5LL) ? 2 : 1;
+    if (pl.parts) {
+        // eight reduction threads a body where it has many pieces (N = 6,000,
+        // 31: 16.5 us against 17.5 with four); two bodies a thread where the
+        // blocks of one would not be resident together
+        pl.groups8 = pl.ncta / rows + rows / 2 >= 28 && rows <= 16;
+        pl.each = (long long)nsets * (G::kSet / 32) > sms * (pl.groups8 ? 2LL : 5LL) ? 2 : 1;
+    } else {
+        // with remainders to add, two bodies a thread throughout, and eight
+        // threads for them where few rows share the CTAs' pieces.  us a call,
+        // eight and four threads: N = 5,000 15.5, 16.2; 8,192 27.0, 27.5; 9,000
+        // 31.4, 31.8; 10,007 (20 rows) 37.5, 37.4; 16,384 81.2, 81.5; 18,000
+        // 95.8, 96.2; 20,000 (20 rows) 119.5, 116.8; one body a thread: 16,384
+        // 81.2, 82.4, 10,007 37.5, 37.7
+        pl.groups8 = rows <= 18;
+        pl.each = 2;
+    }
     pl.slots = pl.ncta;
     if (!max_bytes && cost >= (long long)slots * pair::kLateSteps * pair::kCostBoth)
         pl.ncta = std::min(2 * slots, kMaxPairCtas);
