@@ -553,8 +553,9 @@ __device__ __forceinline__ long long row_piece(int row, int nsets, int ch) {
 struct Item {
     const float4 *pm_;
     float *react_, *tsum_;
-    int n_, row, set, nset, pieces, kind;    // kind: the system's Desc::pair, or 3: tasks from `row` on
+    int n_, row, set, nset, kind;    // kind: the system's Desc::pair, or 3: tasks from `row` on
     float eps2_;
+    int pieces;  // (last: where it stood before eps2_ the wide rows took 2 % longer)
     __device__ __forceinline__ const float4 *pm() const { return pm_; }
     __device__ __forceinline__ int n() const { return n_; }
     __device__ __forceinline__ float eps2() const { return eps2_; }
@@ -860,11 +861,13 @@ inline int sub_eff(const HostSys &h) {
 // Items of a pair system are whole source sets of one row: few enough that an
 // item's start-up (2-3 us) is small beside its steps (11 us a set with narrow
 // rows, 30 us with wide ones), many enough that one system alone fills the
-// GPU.  Depends on n only, as does the geometry: rows of 512 targets below
+// GPU.  Up to two sets the targets' sums need no remainders: with four below
+// 2,048 bodies 200 systems of 1,100 take 142 us a tick instead of 131, 249 of
+// 1,497 256 instead of 244, one system 39 instead of 25.  Depends on n only, as does the geometry: rows of 512 targets below
 // 8,192 bodies (more, smaller items, less padding), 1,024 above.
 int sets_per_item(size_t n) {
     if (n < 8192)
-        return n < 2048 ? 4 : 2;
+        return 2;
     int ch = 1;
     for (size_t m = 16384; m <= n && ch < 32; m *= 2)
         ch *= 2;
@@ -878,8 +881,8 @@ void pair_shape(size_t n, HostSys &h) {
     h.ch = sets_per_item(n);
     const size_t meetings = (size_t)nbgb::pair::meetings_before<G>(h.rows, h.nsets);
     h.react_len = meetings * 3 * G::kSet;
-    // an item of one set is a single fold, which leaves no remainder
-    h.target_pieces = h.ch > 1 ? 2 : 1;
+    // up to 256 sources are one float here as in the one-sided queue
+    h.target_pieces = h.ch * G::kSet > 256 ? 2 : 1;
     h.scratch_len = h.react_len +
                     (meetings / h.ch + h.rows) * h.target_pieces * 3 * G::kRow;  // row_piece
 }

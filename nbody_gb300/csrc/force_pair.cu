@@ -40,8 +40,8 @@
 // is more work, as many short late ones (stretch_cost).  A stretch may begin and end inside a set or a row.
 // Pieces: the reactions of one stretch's part of one (row, set) meeting
 // (kSet x 3 floats, slot = meeting index + CTA index) and the targets' sums
-// of its part of one row (kRow x 3 floats and as many for what rounding them
-// leaves out, slot = row + CTA index); both
+// of its part of one row (kRow x 3 floats, and as many for what rounding them
+// leaves out where stretches exceed 256 sources, slot = row + CTA index); both
 // numberings grow strictly along the line, so no two pieces share a slot.
 // The reduce kernel adds each body's pieces in a fixed order with compensated
 // FP32 sums and writes the force (and integrates, when asked).  Both kernels
@@ -84,13 +84,11 @@ struct Source {
 struct Params {
     Source src;
     float *__restrict__ react;  // [slot][3][kSet]
-    float *__restrict__ tsum;   // [slot][3 kPieces][kRow]
+    float *__restrict__ tsum;   // [slot][3 pieces][kRow]
     int nsets, row0, row1;      // rows of this phase
     int ncta, parts;                // parts > 0: stretches are parts of meetings
+    int pieces;                     // the targets' sums of a stretch; 2: and remainders
     unsigned step[kMaxPairCtas + 1];  // first step of each CTA's stretch
-    // the targets' sums of a stretch and their remainders; a part of a meeting
-    // is one fold and has none
-    __host__ __device__ int target_pieces() const { return parts ? 1 : 2; }
 };
 
 // Row b's part of this CTA's stretch (row_stretch asks for it).
@@ -108,9 +106,9 @@ struct StretchIo {
     }
     __device__ __forceinline__ float *tsum() const {
         return P.tsum +
-               ((size_t)(b - P.row0) + blockIdx.x) * P.target_pieces() * 3 * G::kRow;
+               ((size_t)(b - P.row0) + blockIdx.x) * P.pieces * 3 * G::kRow;
     }
-    __device__ __forceinline__ bool remainder() const { return P.target_pieces() > 1; }
+    __device__ __forceinline__ bool remainder() const { return P.pieces > 1; }
 };
 
 template <class G>
@@ -242,7 +240,7 @@ __global__ void __launch_bounds__(3 * 32 * kGroups)
                      (unsigned)((meetings_before<G>(b + 1, P.nsets) - g0) << 5), tf, tl);
             n_list = base;
             t_first = tf;
-            t_count = (tl - tf + 1) * P.target_pieces();
+            t_count = (tl - tf + 1) * P.pieces;
         }
     }
     __syncthreads();
@@ -252,7 +250,7 @@ __global__ void __launch_bounds__(3 * 32 * kGroups)
     const float *react = P.react + (size_t)comp * kSet + sub * kB + j;
     const int i = set * kSet + sub * kB + j;
     const float *tsum = P.tsum + (size_t)comp * G::kRow + (i - b * G::kRow) +
-                        (size_t)(b - P.row0 + tf) * P.target_pieces() * 3 * G::kRow;
+                        (size_t)(b - P.row0 + tf) * P.pieces * 3 * G::kRow;
     auto piece = [&](int q) {
         return q < nr ? react + (size_t)list[q] * 3 * kSet
                       : tsum + (size_t)(q - nr) * 3 * G::kRow;
@@ -332,6 +330,7 @@ __global__ void __launch_bounds__(3 * 32 * kGroups)
 // at least kMinCost (no stretch is empty, and few pieces at small N), a part
 // of a meeting at least kMinPartSteps steps.
 constexpr int kCostBoth = 4, kCostOne = 3, kMinCost = 32, kMinPartSteps = 4;
+constexpr int kShortSteps = 64;  // 256 sources
 constexpr size_t kLoneSmem = 120 * 1024;  // one CTA an SM
 
 template <class G>
@@ -472,11 +471,13 @@ static bool plan_geometry(size_t n, int sms, size_t max_bytes, PairPlan &pl) {
     pl.slots = pl.ncta;
     if (!max_bytes && cost >= (long long)slots * pair::kLateSteps * pair::kCostBoth)
         pl.ncta = std::min(2 * slots, kMaxPairCtas);
+    // stretches of one-sided steps only hold most of them
+    pl.pieces = pl.parts || cost <= (long long)pl.ncta * pair::kShortSteps * pair::kCostOne ? 1 : 2;
     // (a small workspace holds few rows' pieces at a time, which need few
     // places for the targets' sums)
     pl.max_rows = max_bytes ? 64 : kMaxPairRows;
     const size_t tsum = align256((size_t)(std::min(rows, pl.max_rows) + pl.ncta) *
-                                 (pl.parts ? 3 : 6) * G::kRow * 4);
+                                 (3 * pl.pieces) * G::kRow * 4);
     const size_t carry = align256((size_t)nsets * G::kSet * 6 * 4);
     const size_t all = align256(react_bytes<G>(0, rows, nsets, pl.ncta));
     // a phase of 256 MiB of pieces is about 16 ms of work; always at least
@@ -491,8 +492,8 @@ static bool plan_geometry(size_t n, int sms, size_t max_bytes, PairPlan &pl) {
             return false;
     }
     const bool one = rows <= pl.max_rows && all <= room;
-    if (!one && (pl.parts || phase_end<G>(0, rows, nsets, pl.ncta, pl.max_rows, room) == 0))
-        return false;  // (parts are at most `slots` pieces, always one phase)
+    if (!one && (pl.pieces == 1 || phase_end<G>(0, rows, nsets, pl.ncta, pl.max_rows, room) == 0))
+        return false;  // (short stretches are few pieces, always one phase)
     pl.react_bytes = one ? all : room;
     pl.off_react = 0;
     pl.off_tsum = align256(pl.react_bytes);
@@ -542,6 +543,7 @@ static int launch_geometry(const PairPlan &pl, float4 *force, const float4 *posM
         const bool late = total >= (long long)pl.slots * pair::kLateSteps * pair::kCostBoth;
         P.ncta = (int)std::min<long long>(late ? pl.ncta : pl.slots, total / pair::kMinCost);
         P.parts = pl.parts;
+        P.pieces = pl.pieces;
         if (pl.parts)
             P.ncta = pl.ncta;
         pair::cut_steps<G>(P.row0, P.row1, nsets, P.ncta, pl.slots, pl.parts, P.step);

@@ -28,6 +28,7 @@ struct PairPlan {
     int groups8 = 0;          // eight reduction threads a body (else four)
     int each = 1;             // bodies of a reduction thread
     int max_rows = 0;         // rows of one phase, at most
+    int pieces = 2;           // 1: the targets' sums of a stretch have no remainders
     size_t react_bytes = 0;   // reaction pieces of one phase, at most
     size_t off_react = 0, off_tsum = 0, off_carry = 0;
     size_t workspace_bytes = 0;

@@ -173,7 +173,8 @@ __device__ __forceinline__ void store_source(float *buf, int j, float4 v) {
 // status() (not null: refuse masses < 0), react(s) (the piece of step s's
 // meeting, not asked for one-sided ones), tsum() (the targets' piece, 3 x
 // kRow), remainder() (whether what rounding the piece to one float leaves out
-// follows it; a stretch with a single fold leaves nothing).  SHARE: the last row may fill only some warps' targets; it meets only
+// follows it; not asked for where a stretch is 256 sources at most, which the
+// one-sided kernel too adds up in one float).  SHARE: the last row may fill only some warps' targets; it meets only
 // its own sets, one-sided, and warps without targets of their own then take a
 // share of the others' steps (one or two full warps: 4 or 2 shares).
 template <class G, bool SHARE, class Io>
@@ -345,24 +346,36 @@ __device__ __forceinline__ void row_stretch(const Io &io, float *smem, int b, in
         fold();
     if (SHARE && shares > 1)
         __syncthreads();
-    float *out = io.tsum();
+    float *out = io.tsum() + tile * 32 * KI + lane;
+    auto total = [&](int k, int c, float &hi, float &lo) {
+        hi = hl[(6 * k + c) * NT + tid];
+        lo = hl[(6 * k + 3 + c) * NT + tid];
+        for (int q = 1; q < shares; q++) {
+            comp_add(hi, lo, hl[(6 * k + c) * NT + tid + 32 * full * q]);
+            lo += hl[(6 * k + 3 + c) * NT + tid + 32 * full * q];
+        }
+    };
     if (share == 0) {
 #pragma unroll
         for (int k = 0; k < KI; k++)
 #pragma unroll
             for (int c = 0; c < 3; c++) {
-                float hi = hl[(6 * k + c) * NT + tid], lo = hl[(6 * k + 3 + c) * NT + tid];
-                for (int q = 1; q < shares; q++) {
-                    comp_add(hi, lo, hl[(6 * k + c) * NT + tid + 32 * full * q]);
-                    lo += hl[(6 * k + 3 + c) * NT + tid + 32 * full * q];
-                }
-                float sum, rest;
-                two_sum(hi, lo, sum, rest);
-                float *o = out + c * G::kRow + tile * 32 * KI + lane + 32 * k;
-                o[0] = sum;
-                if (io.remainder())
-                    o[3 * G::kRow] = rest;
+                float hi, lo;
+                total(k, c, hi, lo);
+                out[c * G::kRow + 32 * k] = __fadd_rn(hi, lo);
             }
+        // (a loop of its own: a condition on each store cost all rows 4 %)
+        if (io.remainder()) {
+#pragma unroll
+            for (int k = 0; k < KI; k++)
+#pragma unroll
+                for (int c = 0; c < 3; c++) {
+                    float hi, lo, sum, rest;
+                    total(k, c, hi, lo);
+                    two_sum(hi, lo, sum, rest);
+                    out[(3 + c) * G::kRow + 32 * k] = rest;
+                }
+        }
     }
     // the next row's staging reuses buffers others may still be reading
     __syncthreads();
