@@ -451,8 +451,8 @@ constexpr int kBodyBlock = 64;  // bodies of one entry of the block map, two a r
 
 struct PairParams {
     const Desc *desc;
-    const int4 *items;  // {system, row, chunk, 0} or {-1, first task, 0, 0}
-    const int2 *tasks;  // {system, tile}, four to an item ({-1, 0}: none)
+    const int4 *items;  // {system, row, chunk, 0} or {-1, first task, warps a task, 0}
+    const int2 *tasks;  // {system, tile}, 4 / warps to an item ({-1, 0}: none)
     int n_items, pass;
     unsigned *head;                  // zeroed by ens_drift
     const float4 *pm;
@@ -467,19 +467,32 @@ __device__ __forceinline__ bool takes_part(const Desc &d, int pass) {
     return (d.flags & kInForce) && (pass == 0 || ((d.flags & kMove) && d.sub > pass));
 }
 
-// Bodies 128 tile .. 128 tile + 127 of a small system by one warp: forces from
-// all its sources, acceleration and closing half kick.  buf: the warp's part
-// of the CTA's shared memory.  A system of up to kTaskBelow - 1 bodies is too
+// Bodies 128 tile .. 128 tile + 127 of a small system by one warp, or by two or
+// four of a CTA that share its sets out: forces from
+// all its sources, acceleration and closing half kick.  smem: the CTA's shared
+// memory.  A system of up to kTaskBelow - 1 bodies is too
 // small for rows: most of a row's targets would be padding and its items
 // short (1,024 systems a tick, GB300, against rows and the one-sided queue:
-// see kTaskBelow).
+// see kTaskBelow).  The sets' sums are added in set order either way, so the
+// result does not depend on which it is.
 constexpr int kTaskBodies = 32 * Narrow::KI;
+constexpr int kTaskSets = 8;  // of a system, at most
+static_assert((4 * Narrow::kSource + 2 * kTaskSets * 3 * kTaskBodies) * 4 <= kPairSmem,
+              "sources of four warps and the sums of two tasks");
 
+template <int WARPS>
 __device__ __forceinline__ void warp_task(const PairParams &P, const Desc &d, int tile,
-                                          float *buf) {
+                                          float *smem) {
     constexpr int KI = Narrow::KI, kSet = Narrow::kSet;
     static_assert(kSet == kTaskBodies, "a lane stages as many sources as it has targets");
-    const int lane = threadIdx.x & 31;
+    static_assert(KI % WARPS == 0, "a warp finishes 32 KI / WARPS bodies");
+    const int lane = threadIdx.x & 31, share = (threadIdx.x >> 5) % WARPS;
+    float *buf = smem + (threadIdx.x >> 5) * Narrow::kSource;
+    // WARPS > 1: the task's sums, [set][3][KI][32]
+    float *part = smem + 4 * Narrow::kSource +
+                  (threadIdx.x >> 5) / WARPS * (kTaskSets * 3 * KI * 32);
+    const int each = (d.nsets + WARPS - 1) / WARPS;
+    const int set0 = share * each, set1 = min(set0 + each, d.nsets);
     const float4 *pm = P.pm + d.body_off;
     const f2 eps2p = f2_pack(d.eps2, d.eps2), zero2 = f2_pack(0.f, 0.f);
     f2 nx[KI], ny[KI], nz[KI], nm[KI], ax[KI], ay[KI], az[KI];
@@ -487,7 +500,7 @@ __device__ __forceinline__ void warp_task(const PairParams &P, const Desc &d, in
     float4 next[KI];
 #pragma unroll
     for (int k = 0; k < KI; k++) {
-        const int i = tile * kTaskBodies + lane + 32 * k, j = lane + 32 * k;
+        const int i = tile * kTaskBodies + lane + 32 * k, j = set0 * kSet + lane + 32 * k;
         const float4 v = i < d.n ? pm[i] : make_float4(0.f, 0.f, 0.f, 0.f);
         next[k] = j < d.n ? pm[j] : make_float4(0.f, 0.f, 0.f, 0.f);
         nx[k] = f2_pack(-v.x, -v.x);
@@ -499,7 +512,7 @@ __device__ __forceinline__ void warp_task(const PairParams &P, const Desc &d, in
         for (int c = 0; c < 3; c++)
             hi[c][k] = lo[c][k] = 0.f;
     }
-    for (int set = 0; set < d.nsets; set++) {
+    for (int set = set0; set < set1; set++) {
         __syncwarp();
 #pragma unroll
         for (int k = 0; k < KI; k++) {
@@ -513,20 +526,37 @@ __device__ __forceinline__ void warp_task(const PairParams &P, const Desc &d, in
                                             1.f);
 #pragma unroll
         for (int k = 0; k < KI; k++) {
-            float l, h;
-            f2_unpack(ax[k], l, h);
-            comp_add(hi[0][k], lo[0][k], l + h);
-            f2_unpack(ay[k], l, h);
-            comp_add(hi[1][k], lo[1][k], l + h);
-            f2_unpack(az[k], l, h);
-            comp_add(hi[2][k], lo[2][k], l + h);
+            const f2 a[3] = {ax[k], ay[k], az[k]};
+#pragma unroll
+            for (int c = 0; c < 3; c++) {
+                float l, h;
+                f2_unpack(a[c], l, h);
+                if (WARPS > 1)
+                    part[((set * 3 + c) * KI + k) * 32 + lane] = l + h;
+                else
+                    comp_add(hi[c][k], lo[c][k], l + h);
+            }
             ax[k] = ay[k] = az[k] = zero2;
         }
     }
+    constexpr int kMine = KI / WARPS;  // body groups this warp finishes
+    if (WARPS > 1) {
+        if (WARPS == 4 || threadIdx.x < 32 * WARPS)  // the task's warps only
+            asm volatile("bar.sync 1, %0;" ::"n"(32 * WARPS) : "memory");
+        else
+            asm volatile("bar.sync 2, %0;" ::"n"(32 * WARPS) : "memory");
+        for (int set = 0; set < d.nsets; set++)
+#pragma unroll
+            for (int k = 0; k < kMine; k++)
+#pragma unroll
+                for (int c = 0; c < 3; c++)
+                    comp_add(hi[c][k], lo[c][k],
+                             part[((set * 3 + c) * KI + share * kMine + k) * 32 + lane]);
+    }
     const double kdt = 0.5 * d.dt;
 #pragma unroll
-    for (int k = 0; k < KI; k++) {
-        const int b = tile * kTaskBodies + lane + 32 * k;
+    for (int k = 0; k < kMine; k++) {
+        const int b = tile * kTaskBodies + lane + 32 * (share * kMine + k);
         if (b >= d.n)
             continue;
         const size_t i = (size_t)d.body_off + b;
@@ -553,7 +583,8 @@ __device__ __forceinline__ long long row_piece(int row, int nsets, int ch) {
 struct Item {
     const float4 *pm_;
     float *react_, *tsum_;
-    int n_, row, set, nset, kind;    // kind: the system's Desc::pair, or 3: tasks from `row` on
+    int n_, row, set, nset, kind;
+    // kind: the system's Desc::pair, or 3: tasks from `row` on, `set` warps each
     float eps2_;
     int pieces;  // (last: where it stood before eps2_ the wide rows took 2 % longer)
     __device__ __forceinline__ const float4 *pm() const { return pm_; }
@@ -599,6 +630,7 @@ __global__ void __launch_bounds__(kPairCtaThreads, 2) ens_pair_kernel(PairParams
             if (v.x < 0) {
                 item.kind = 3;
                 item.row = v.y;
+                item.set = v.z;
             } else if (P.desc[v.x].pair == 1) {
                 set_item<Narrow>(item, P, P.desc[v.x], v.y, v.z);
             } else {
@@ -608,10 +640,16 @@ __global__ void __launch_bounds__(kPairCtaThreads, 2) ens_pair_kernel(PairParams
         }
         __syncthreads();
         if (item.kind == 3) {
-            const int warp = threadIdx.x >> 5;
-            const int2 t = P.tasks[item.row + warp];
-            if (t.x >= 0 && takes_part(P.desc[t.x], P.pass))
-                warp_task(P, P.desc[t.x], t.y, smem_f + warp * Narrow::kSource);
+            const int warps = item.set;
+            const int2 t = P.tasks[item.row + (int)(threadIdx.x >> 5) / warps];
+            if (t.x >= 0 && takes_part(P.desc[t.x], P.pass)) {
+                if (warps == 1)
+                    warp_task<1>(P, P.desc[t.x], t.y, smem_f);
+                else if (warps == 2)
+                    warp_task<2>(P, P.desc[t.x], t.y, smem_f);
+                else
+                    warp_task<4>(P, P.desc[t.x], t.y, smem_f);
+            }
             __syncthreads();
         } else if (item.kind == 1) {
             pair::row_stretch<Narrow, true>(item, smem_f, item.row, item.set, 0u,
@@ -894,6 +932,39 @@ void pair_shape(size_t n, HostSys &h) {
 // 1,010 (53 / 40 / 106), and of 953 systems of 1,448 1,011 / 882 / 925.
 constexpr size_t kTaskBelow = 1024;
 
+// Warp tasks (longest first) that take a warp each, out of `tasks` with `warps`
+// resident; the others share their sets out among several warps (task_warps),
+// for between a tenth of the GPU's CTA slots and a few rounds it is the last
+// tasks that decide: one warp alone takes 47 us for the eight sets of 1,000
+// bodies, 77 beside another CTA's.  Where the sets divide evenly (four and eight
+// by four warps, six by two) sharing costs nothing: all but whole rounds less
+// one.  Where they do not, idle warps cost more than a nearly full round does:
+// all but whole rounds, and not the rest either from three quarters of a round
+// on.  `sets`: of the longest task after whole rounds.  Microseconds a tick, a
+// warp a task / as here / the one-sided queue's tuned plan: 32 systems of 1,000
+// bodies 76 / 26 / 50, 128 79 / 71 / 83, 512 264 / 240 / 253, 1,024 472 / 466 /
+// 488; of 800 160 71 / 73 / 100, 200 128 / 91 / 116, 1,024 362 / 369 / 464; of
+// 700 64 61 / 37 / 44, 128 63 / 55 / 56, 256 114 / 85 / 93; of 512 64 45 / 18 /
+// 37, 384 84 / 63 / 72; of 300 24 26 / 14 / 42, 384 41 / 41 / 56.
+size_t alone_tasks(size_t tasks, size_t warps, int sets) {
+    const size_t full = tasks / warps * warps;
+    if (sets % 4 == 0 || sets == 6)
+        return full > 0 ? full - warps : 0;
+    return 4 * (tasks - full) > 3 * warps ? tasks : full;
+}
+// Two warps where four would wait for the one with two sets of five or six,
+// unless what is left after whole rounds of them are few enough tasks for a CTA
+// each.
+size_t late_tasks(size_t tasks, size_t ctas) {
+    const size_t rest = tasks % (2 * ctas);
+    return rest <= ctas ? rest : 0;
+}
+int task_warps(int nsets, bool late) {
+    if (nsets <= 2)
+        return 1;
+    return !late && (nsets == 5 || nsets == 6) ? 2 : 4;
+}
+
 // The pair plan of n bodies if its scratch is at most max_floats.
 bool pair_plan(size_t n, size_t max_floats, HostSys &h) {
     HostSys t;
@@ -1105,8 +1176,8 @@ int rebuild_pairs(nbgb_ensemble *e) {
             e->h_blocks[e->n_blocks++] = make_int2(s, k);
         return true;
     };
-    // warp tasks, four of one sub and like length to an item, in the first
-    // group; their bodies need no reduction
+    // warp tasks, four of one sub and like length to an item, or fewer that
+    // have several warps, in the first group; their bodies need no reduction
     std::vector<It> tasks;
     for (int s = 0; s < e->max_systems; s++) {
         const HostSys &h = e->sys[s];
@@ -1125,15 +1196,31 @@ int rebuild_pairs(nbgb_ensemble *e) {
         e->groups.emplace_back();
         e->groups.back().block0 = e->n_blocks;
     }
+    size_t alone_end = 0;
+    size_t late = 0;
     for (size_t k = 0; k < tasks.size();) {
-        if ((size_t)e->n_tasks + 4 > e->tasks_cap)
-            return NBGB_ERR_NO_MEMORY;
         const int sub = tasks[k].sub;
+        if (k == 0 || sub != tasks[k - 1].sub) {
+            size_t end = k;
+            while (end < tasks.size() && tasks[end].sub == sub)
+                end++;
+            const size_t slots = 4 * (size_t)e->grid;
+            const size_t rest = std::min(k + (end - k) / slots * slots, end - 1);
+            alone_end = k + alone_tasks(end - k, slots, tasks[rest].cost);
+            late = end - late_tasks(end - alone_end, (size_t)e->grid);
+        }
+        auto warps_of = [&](size_t t) {
+            return t < alone_end ? 1 : task_warps(tasks[t].cost, t >= late);
+        };
+        const int warps = warps_of(k);
+        if ((size_t)e->n_tasks + 4 / warps > e->tasks_cap)
+            return NBGB_ERR_NO_MEMORY;
         // a one-sided step of four warps costs three quarters of one of a row
-        items.push_back(It{make_int4(-1, e->n_tasks, 0, 0),
-                           (tasks[k].cost * nbgb::ens::Narrow::KI * 3 + 3) / 4, sub});
-        for (int q = 0; q < 4; q++, e->n_tasks++) {
-            const bool have = k < tasks.size() && tasks[k].sub == sub;
+        const int sets = (tasks[k].cost + warps - 1) / warps;
+        items.push_back(It{make_int4(-1, e->n_tasks, warps, 0),
+                           (sets * nbgb::ens::Narrow::KI * 3 + 3) / 4, sub});
+        for (int q = 0; q < 4 / warps; q++, e->n_tasks++) {
+            const bool have = k < tasks.size() && tasks[k].sub == sub && warps_of(k) == warps;
             e->h_tasks[e->n_tasks] =
                 have ? make_int2(tasks[k].v.x, tasks[k].v.y) : make_int2(-1, 0);
             k += have;

@@ -108,3 +108,24 @@ def test_partial_sums_keep_their_remainders(cuda, n):
     assert np.all(np.abs(a[:, 0] - want) <= 2.0 ** -23 * want), a[:, 0] - want
     assert np.all(a[:, 1:] == 0)
     e.close()
+
+
+def test_warps_of_a_task_do_not_change_results(cuda):
+    """One system's tiles are shared among four warps, those of hundreds taken
+    by a warp or two each: the bits are the same (systems of 1 to 8 sets)."""
+    sizes = [100, 200, 384, 500, 640, 768, 800, 1000]
+    got = []
+    for copies in (1, 200):
+        e = nb.Ensemble(copies * sum(sizes), copies * len(sizes), EPS2, tuning=None)
+        slots = {}
+        for k in range(copies):
+            for n in sizes:
+                p, v, m, _ = _ball(n, 700 + n)
+                slots[n, k] = e.add(p, v, m, 0.002, 6)
+        e.tick(4)
+        e.synchronize()
+        got.append({n: e.get_state(slots[n, copies - 1]) for n in sizes})
+        e.close()
+    for n in sizes:
+        for a, b in zip(got[0][n], got[1][n]):
+            assert np.array_equal(a, b), n
