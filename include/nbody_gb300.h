@@ -295,12 +295,21 @@ typedef struct nbgb_ensemble nbgb_ensemble;
 NBGB_API nbgb_ensemble *nbgb_ensemble_create(size_t max_bodies, int max_systems,
                                              float softeningSquared);
 NBGB_API void nbgb_ensemble_destroy(nbgb_ensemble *ens);
+/* How the default plan evaluates a system of N bodies (newton3 != 0: one that
+   nbgb_ensemble_set_newton3_min covers), which depends on N alone: *kind 3
+   tasks of single warps (small systems), 1 and 2 rows of 512 and 1,024 bodies
+   with each pair evaluated once, 0 neither (the one-sided queue; with newton3
+   block pairs).  *sets_per_item source sets of 128 bodies are a unit of work
+   and *scratch_bytes the system's share of the scratch arena (0 for the other
+   kinds).  Any pointer may be NULL; needs no GPU. */
+NBGB_API int nbgb_ensemble_kind(size_t N, int newton3, int *kind, int *sets_per_item,
+                                size_t *scratch_bytes);
 NBGB_API size_t nbgb_ensemble_device_bytes(nbgb_ensemble *ens);
 /* Plan for N in [2^bucket, 2^(bucket+1)): variant 0..3 = (targets per
    thread, unroll) (1,8) (2,4) (1,4) (2,8); tile a power of two in 16..1024
    bodies; j-split 1..4; variant -1 = the default rule: each pair of bodies
    evaluated once (nbgb_ensemble_slot_info then reports variant -1, tile 0),
-   for systems of up to about 290,000 bodies. */
+   for systems of up to 283,008 bodies (nbgb_ensemble_kind). */
 NBGB_API int nbgb_ensemble_set_bucket_plan(nbgb_ensemble *ens, int bucket, int variant, int jt,
                                            int nsplit);
 /* Admit a system (HOST double[n][3] x, v; float m[n]); NBGB_ERR_NO_MEMORY if
@@ -333,8 +342,8 @@ NBGB_API int nbgb_ensemble_max_grid(nbgb_ensemble *ens);
 /* Systems admitted afterwards with N >= nmin are evaluated with each pair
    once, as by the default plan, whatever their bucket's plan; they move one
    step per tick.  0 = none (the default).  The first nonzero call grows the
-   scratch arena (to 1 GiB at most).  Systems too large for it (above about
-   410,000 bodies) take block pairs with FP64 sums instead, whose results repeat
+   scratch arena (to 1 GiB at most).  Systems too large for it (above
+   401,152 bodies) take block pairs with FP64 sums instead, whose results repeat
    to FP64 rounding order rather than bit for bit (arena of 24 B per body of
    capacity, allocated when such a system could be admitted). */
 NBGB_API int nbgb_ensemble_set_newton3_min(nbgb_ensemble *ens, size_t nmin);

@@ -497,6 +497,18 @@ class Ensemble:
         return int(self.lib.nbgb_ensemble_active(self.h))
 
 
+def ensemble_kind(N: int, newton3: bool = False):
+    """(kind, source sets per unit of work, scratch bytes) of a system of N
+    bodies under an ensemble's default plan (newton3: one that set_newton3_min
+    covers): "tasks" (small systems), "pairs" (each pair of bodies once),
+    "onesided" or "blockpairs" (too large for the scratch arena)."""
+    k, c, b = ctypes.c_int(), ctypes.c_int(), ctypes.c_size_t()
+    check(load().nbgb_ensemble_kind(N, int(newton3), ctypes.byref(k), ctypes.byref(c),
+                                    ctypes.byref(b)), "nbgb_ensemble_kind")
+    names = ("blockpairs" if newton3 else "onesided", "pairs", "pairs", "tasks")
+    return names[k.value], c.value, b.value
+
+
 # ---------------------------------------------------------------------------
 # Initial conditions, metrics (host)
 # ---------------------------------------------------------------------------

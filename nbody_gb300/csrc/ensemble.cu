@@ -913,10 +913,10 @@ int sets_per_item(size_t n) {
 }
 
 template <class G>
-void pair_shape(size_t n, HostSys &h) {
+void pair_shape(size_t n, int ch, HostSys &h) {
     h.nsets = (int)((n + G::kSet - 1) / G::kSet);
     h.rows = (int)((n + G::kRow - 1) / G::kRow);
-    h.ch = sets_per_item(n);
+    h.ch = ch;
     const size_t meetings = (size_t)nbgb::pair::meetings_before<G>(h.rows, h.nsets);
     h.react_len = meetings * 3 * G::kSet;
     // up to 256 sources are one float here as in the one-sided queue
@@ -965,7 +965,18 @@ int task_warps(int nsets, bool late) {
     return !late && (nsets == 5 || nsets == 6) ? 2 : 4;
 }
 
-// The pair plan of n bodies if its scratch is at most max_floats.
+// The pair plan of n bodies if its scratch is at most max_floats.  Where it
+// would be more, items of up to kMaxItemSets sets: the places for the
+// targets' sums are one to every item, and those for the reactions, 6 N^2 /
+// 1,024 bytes, then set the limit.  (With 32 sets at most, systems of 250,000
+// bodies did not fit and those of 265,000 did.)
+constexpr int kMaxItemSets = 128;
+void pair_shape(size_t n, int ch, HostSys &h) {
+    if (n < 8192)
+        pair_shape<nbgb::ens::Narrow>(n, ch, h);
+    else
+        pair_shape<nbgb::ens::Wide>(n, ch, h);
+}
 bool pair_plan(size_t n, size_t max_floats, HostSys &h) {
     HostSys t;
     if (n < kTaskBelow) {
@@ -973,10 +984,10 @@ bool pair_plan(size_t n, size_t max_floats, HostSys &h) {
         h.nsets = (int)((n + nbgb::ens::Narrow::kSet - 1) / nbgb::ens::Narrow::kSet);
         return true;
     }
-    if (n < 8192)
-        pair_shape<nbgb::ens::Narrow>(n, t);
-    else
-        pair_shape<nbgb::ens::Wide>(n, t);
+    int ch = sets_per_item(n);
+    pair_shape(n, ch, t);
+    while (t.scratch_len > max_floats && ch < kMaxItemSets)
+        pair_shape(n, ch *= 2, t);
     if (t.scratch_len > max_floats)
         return false;
     h.pair = n < 8192 ? 1 : 2;
@@ -989,19 +1000,22 @@ bool pair_plan(size_t n, size_t max_floats, HostSys &h) {
     return true;
 }
 
-// Scratch arena (floats): what the largest pair system of max_bodies needs,
-// at most `limit`.  Systems that need more than the limit are not pair
+// Scratch arena (floats): what the largest pair system of max_bodies needs with
+// sets_per_item's items, at most `limit` (larger items fit into it).  Systems
+// that need more than the limit are not pair
 // systems: a rule on n alone.
-constexpr size_t kPairScratch = ((size_t)512 << 20) / 4;     // to about 290,000 bodies
-constexpr size_t kPairScratchN3 = ((size_t)1 << 30) / 4;     // Newton-3: to about 410,000
+constexpr size_t kPairScratch = ((size_t)512 << 20) / 4;     // to 283,008 bodies
+constexpr size_t kPairScratchN3 = ((size_t)1 << 30) / 4;     // Newton-3: to 401,152
 size_t scratch_for(size_t max_bodies, size_t limit) {
     size_t most = 0;
     for (size_t n : {(size_t)8191, (size_t)16383, (size_t)32767, (size_t)65535,
                      (size_t)131071, (size_t)262143, max_bodies}) {
         HostSys h;
         n = std::min(n, max_bodies);
-        if (pair_plan(n, ~(size_t)0, h))
+        if (n >= kTaskBelow) {
+            pair_shape(n, sets_per_item(n), h);
             most = std::max(most, h.scratch_len);
+        }
     }
     return std::min(most, limit);
 }
@@ -1486,6 +1500,25 @@ void free_ens(nbgb_ensemble *e) {
 
 extern "C" {
 
+// How a system of N bodies is evaluated by the default plan (newton3: one
+// admitted at or above set_newton3_min's size): kind 3 warp tasks, 1 and 2 rows
+// of pairs (512 and 1,024 bodies), 0 neither (one-sided queue; Newton-3: block
+// pairs); sets_per_item and scratch_bytes of kinds 1 and 2.  No GPU needed.
+NBGB_API int nbgb_ensemble_kind(size_t N, int newton3, int *kind, int *sets_per_item,
+                                size_t *scratch_bytes) {
+    if (N == 0 || N > nbgb::kMaxBodies)
+        return NBGB_ERR_INVALID_ARGUMENT;
+    HostSys h;
+    pair_plan(N, newton3 ? kPairScratchN3 : kPairScratch, h);
+    if (kind)
+        *kind = h.pair;
+    if (sets_per_item)
+        *sets_per_item = h.ch;
+    if (scratch_bytes)
+        *scratch_bytes = h.scratch_len * 4;
+    return NBGB_OK;
+}
+
 // Capacity: max_bodies bodies in total, max_systems concurrent systems.  The
 // device arena is allocated once here (about 250 B per body of capacity plus
 // the pair systems' scratch, up to 512 MiB,
@@ -1510,8 +1543,8 @@ NBGB_API nbgb_ensemble *nbgb_ensemble_create(size_t max_bodies, int max_systems,
     e->part_cap = 8 * (max_bodies + (size_t)max_systems * 512);
     e->cnt_cap = max_bodies / 256 + (size_t)max_systems + 1;
     e->items_cap = 4 * (max_bodies / 256 + (size_t)max_systems) + 64;
-    // pair items (at most 0.05 a body, where sets_per_item is about to grow,
-    // and four for the smallest systems) and 32-body blocks
+    // pair items (at most 0.067 a body, where sets_per_item is about to grow,
+    // and four for the smallest systems) and 64-body blocks
     e->scratch_cap = scratch_for(max_bodies, kPairScratch);
     e->pitems_cap = max_bodies / 12 + 4 * (size_t)max_systems + 64;
     e->tasks_cap = max_bodies / nbgb::ens::kTaskBodies + (size_t)max_systems +
