@@ -1,14 +1,13 @@
-// force_sym.cu -- the all-pairs force with Newton's third law: every pair of
-// bodies is evaluated once and applied to both (the idea of the reference's
-// unregistered tiled kernels, src/nbody_GPU_AOS_tiled.cu:93-179, which add
-// every pair's contribution with per-pair warp reductions and float atomics).
+// force_sym.cu -- Newton's third law by block pairs with FP64 sums, for the
+// ensemble's Newton-3 systems that are too large for its scratch arena (above
+// 401,152 bodies; everything else goes through force_pair.cu, which
+// nbgb_force_newton3 below does too).  The idea is that of the reference's
+// unregistered tiled kernels (src/nbody_GPU_AOS_tiled.cu:93-179), which add
+// every pair's contribution with per-pair warp reductions and float atomics.
 //
 // Here the unit of work is a block pair (bi, bj), bi <= bj, of 2048-body
 // blocks, one CTA of 8 warps each (one CTA per SM: up to 255 registers a
-// thread, spent on independent work per warp rather than on more warps;
-// sizes whose pairs would not fill the GPU use 1024-body blocks with 4
-// targets and 4 sources per lane, 2 CTAs per SM -- the same scheme at half
-// the width):
+// thread, spent on independent work per warp rather than on more warps):
 //   * warp w holds 256 targets of block bi in registers (8 per lane, negated
 //     and duplicated into f32x2 pairs, with their masses);
 //   * block bj is visited as 8 source sets of 256 bodies; every lane loads 8
@@ -47,23 +46,14 @@ namespace sym {
 constexpr int kWarps = 8;
 constexpr int kThreads = kWarps * 32;
 
-// Geometry: KI targets and KJ = KI sources per lane.  KI = 8: 2048-body
-// blocks, one CTA per SM (up to 255 registers); KI = 4: 1024-body blocks,
-// two CTAs per SM (128 registers), four times the block pairs for sizes
-// whose 2048-body pairs would not fill the GPU.
-template <int KI_>
 struct Geo {
-    static constexpr int KI = KI_;                  // targets per lane
-    static constexpr int KJ = KI_;                  // sources per lane
+    static constexpr int KI = 8;                    // targets per lane
+    static constexpr int KJ = KI;                   // sources per lane
     static constexpr int NC = KJ / 2;               // f32x2 source pairs per lane
-    static constexpr int kMinBlocks = KI_ >= 8 ? 1 : 2;  // resident CTAs per SM
-    static constexpr int kSet = 32 * KJ;            // sources per set
+    static constexpr int kSet = 32 * KJ;            // sources per set, one fold
     static constexpr int kBlock = kWarps * 32 * KI; // bodies per block
-    static constexpr int kFoldSets = kSet >= 256 ? 1 : 256 / kSet;  // sets per fold
     static_assert(kBlock == kWarps * kSet, "a block is 8 source sets");
-    static_assert(kWarps % kFoldSets == 0, "folds end with the block's last set");
 };
-constexpr int kWideKI = 8, kNarrowKI = 4;
 
 struct Params {
     const float4 *__restrict__ pm;  // AOS posMass (targets), n bodies
@@ -149,11 +139,9 @@ __device__ __forceinline__ void rotate_set(f2 (&sx)[NC], f2 (&sy)[NC], f2 (&sz)[
 }
 
 // One block pair (bi, bj) of one system, by the whole CTA.
-template <int KI_>
 __device__ __forceinline__ void sym_block_pair(const Params &P, int bi, int bj) {
-    using G = Geo<KI_>;
-    constexpr int KI = G::KI, KJ = G::KJ, NC = G::NC, kSet = G::kSet, kBlock = G::kBlock,
-                  kFoldSets = G::kFoldSets;
+    using G = Geo;
+    constexpr int KI = G::KI, KJ = G::KJ, NC = G::NC, kSet = G::kSet, kBlock = G::kBlock;
     __shared__ float red[kWarps][3][kSet];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const bool diag = (bi == bj);
@@ -200,19 +188,17 @@ __device__ __forceinline__ void sym_block_pair(const Params &P, int bi, int bj) 
         else if (mode == 1)
             rotate_set<false, KI>(sx, sy, sz, sm, rx, ry, rz, nx, ny, nz, nm, ax, ay, az, eps2p,
                                   lane);
-        // fold target sums into the compensated sums every 256 sources
-        if ((s + 1) % kFoldSets == 0) {
+        // fold target sums into the compensated sums every set
 #pragma unroll
-            for (int k = 0; k < KI; k++) {
-                float l, h;
-                f2_unpack(ax[k], l, h);
-                comp_add(hx[k], lx[k], l + h);
-                f2_unpack(ay[k], l, h);
-                comp_add(hy[k], ly[k], l + h);
-                f2_unpack(az[k], l, h);
-                comp_add(hz[k], lz[k], l + h);
-                ax[k] = ay[k] = az[k] = zero2;
-            }
+        for (int k = 0; k < KI; k++) {
+            float l, h;
+            f2_unpack(ax[k], l, h);
+            comp_add(hx[k], lx[k], l + h);
+            f2_unpack(ay[k], l, h);
+            comp_add(hy[k], ly[k], l + h);
+            f2_unpack(az[k], l, h);
+            comp_add(hz[k], lz[k], l + h);
+            ax[k] = ay[k] = az[k] = zero2;
         }
         // reactions on set s: stage per warp, add in warp order, FP64 atomics
 #pragma unroll
@@ -256,7 +242,7 @@ __device__ __forceinline__ void sym_block_pair(const Params &P, int bi, int bj) 
 // Many systems in one launch (the ensemble's Newton-3 systems): CTA b takes
 // block pair b - pair_begin[s] of the system s whose range holds b (binary
 // search over the systems' prefix counts).
-__global__ void __launch_bounds__(kThreads, Geo<kWideKI>::kMinBlocks)
+__global__ void __launch_bounds__(kThreads, 1)
     sym_systems_kernel(const SymSystem *__restrict__ tab, int nsys) {
     const long long b = blockIdx.x;
     int lo = 0, hi = nsys - 1;
@@ -278,7 +264,7 @@ __global__ void __launch_bounds__(kThreads, Geo<kWideKI>::kMinBlocks)
     P.eps2 = t.eps2;
     int bi, bj;
     pair_of(b - t.pair_begin, t.nblocks, bi, bj);
-    sym_block_pair<kWideKI>(P, bi, bj);
+    sym_block_pair(P, bi, bj);
 }
 
 // FP64 sums -> FP32 accelerations {ax, ay, az, 0}, and the sums zeroed for
@@ -310,7 +296,7 @@ int launch_sym_systems(const SymSystem *d_tab, const SymSystem *h_tab, int nsys,
     return cudaGetLastError() == cudaSuccess ? NBGB_OK : NBGB_ERR_CUDA;
 }
 
-int sym_block_bodies() { return sym::Geo<sym::kWideKI>::kBlock; }
+int sym_block_bodies() { return sym::Geo::kBlock; }
 
 }  // namespace nbgb
 
