@@ -34,9 +34,10 @@ interaction (src/nbody.cu:1027).
             oracle's CPU_AOS restatements (IEEE and the reference's flags),
             computed outside every timed region
   reference_mode  milliseconds per resident reference-mode step on small
-            plain systems (N = 1,024, 4,096, 16,384): one launch per step
-            (the integrate in the force kernel's epilogue) against force
-            then integrate, both replaying CUDA graphs of 8 steps
+            plain systems (N = 1,024, 4,096, 16,384): the System's loop
+            (the integrate in the force's last launch) against force and
+            integrate called one after the other, both replaying CUDA graphs
+            of 8 steps
 
 --impl reference times the reference's CPU implementation of the path (the
 reference's own compiled CPU_SOA when oracle/_ref was built on this machine,
@@ -477,11 +478,11 @@ def reference_step_ms(n, dev, stream, flush, reps=5):
 def reference_mode_steps(dev, n=16384, steps=400):  # steps: a multiple of 8
     """Milliseconds per reference-mode step on the plain case at N bodies
     (uniform ball, eps2 = 1e-4, dt = 0.01, damping 0.95, contracted drift):
-    the System's resident loop, one launch per step (the integrate runs in
-    the force kernel's epilogue; graph-launched), against the two-launch form
-    (standalone force kernel, then integrateOne), both replaying CUDA graphs
-    of 8 steps.  L2-resident state: this is the launch and tail cost the
-    fusion removes, not an HBM figure."""
+    the System's resident loop (the integrate in the force's last launch, or
+    right behind it for few bodies; graph-launched) against the calls one
+    after the other (force, then integrateOne), both replaying CUDA graphs
+    of 8 steps.  L2-resident state: launch and tail costs, not an HBM
+    figure."""
     import torch
 
     import nbody_gb300 as nb
@@ -521,8 +522,8 @@ def reference_mode_steps(dev, n=16384, steps=400):  # steps: a multiple of 8
     e1.record()
     torch.cuda.synchronize()
     two_ms = e0.elapsed_time(e1) / steps
-    return {"n_bodies": n, "steps": steps, "ms_per_step_one_launch": fused_ms,
-            "ms_per_step_two_launches": two_ms, "speedup": two_ms / fused_ms,
+    return {"n_bodies": n, "steps": steps, "ms_per_step_resident": fused_ms,
+            "ms_per_step_force_then_integrate": two_ms, "speedup": two_ms / fused_ms,
             "state": f"L2-resident (4 arrays x {n * 16 // 1024} KiB)"}
 
 

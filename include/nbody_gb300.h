@@ -69,7 +69,9 @@ NBGB_API void nbgb_release_workspace(void);
 /* ======================================================================== */
 
 /* Workspace bytes nbgb_force needs for N bodies on the current device
-   (0 if N is unsupported). */
+   (0 if N is unsupported).  On a GB300 0.4 MB for 1,000 bodies, 10 MB for
+   16,384, 120 MB for 131,072, 296 MB for 262,144 and 334 MB for 2^20 (the
+   pieces of pairs go through 256 MiB at a time), 648 MB for 2^23. */
 NBGB_API size_t nbgb_force_workspace_bytes(size_t N);
 
 /*
@@ -270,6 +272,9 @@ NBGB_API int nbgb_system_diagnostics(nbgb_system *sys, double *out);
 NBGB_API void *nbgb_system_device_posmass(nbgb_system *sys);
 NBGB_API void *nbgb_system_device_force(nbgb_system *sys);
 NBGB_API void *nbgb_system_stream(nbgb_system *sys);
+/* The one-sided plan of the system: what it runs after nbgb_system_set_plan
+   and above 2^23 bodies; with the default force below that (nbgb_force_kind)
+   what such a plan would be. */
 NBGB_API int nbgb_system_plan(nbgb_system *sys, int *config, int *nsplit);
 /* Force the one-sided kernel and its plan (config / nsplit as for
    nbgb_force_ex; -1, -1 restores nbgb_force's choice for N).  For tuning and tests; the

@@ -2,10 +2,10 @@
 // once and applied to both (Newton's third law), deterministic: no atomics,
 // every partial sum is written once and added in a fixed order.
 //
-// What bounds it: the FP32 (FMA) pipe and the registers that feed it.  A pair
-// costs 16 packed FP32 operations for two interactions (14 when the masses
-// involved are equal), against 11.5-12 for each interaction of the one-sided
-// kernel.  ncu: FMA pipe 82 % busy; the rest are dispatch stalls of
+// What bounds it: the FP32 (FMA) pipe and the registers that feed it.  Two
+// pairs cost 16 packed FP32 operations for their four interactions (14 when
+// the masses involved are equal), against 23 to 24 of the one-sided
+// kernel.  ncu: FMA pipe 79 % busy; the rest are dispatch stalls of
 // three-operand instructions (six of the 16) and the other instructions' issue.
 // GB300, N = 131,072: 4,256 us with mixed masses (4.04e12 interactions/s),
 // 3,884 us with equal ones (4.42e12), against 4,830 us for 8 sources and 8

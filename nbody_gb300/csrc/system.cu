@@ -193,11 +193,13 @@ int timed_force(nbgb_system *s, const nbgb::FusedIntegrate *fi = nullptr) {
     return rc;
 }
 
-// One reference step: force(x) then integrate (writes x' and its j-stream).
-// With the one-sided kernel both happen in one launch: the force kernel's
-// epilogue integrates each body once its force is final and writes the next
-// step's j-stream into the other buffer, which then becomes current.  With
-// the Newton-3 kernel the integrate is its own launch.
+// One reference step: force(x) then integrate.  The default force integrates
+// in its last launch: the pairs' reduction, once a body's force is final, or,
+// for few bodies, a small kernel behind the direct one (whose CTAs read every
+// position to their end).  Under a forced one-sided plan both happen in one
+// launch: the force kernel's epilogue writes the next step's j-stream into the
+// other buffer, which then becomes current.  With the Newton-3 algorithm the
+// integrate is its own launch.
 int ref_step_body(nbgb_system *s) {
     const int fused_drift = s->integrator == NBGB_INTEGRATOR_REFERENCE_FUSED ? 1 : 0;
     if (s->algorithm == 0) {
