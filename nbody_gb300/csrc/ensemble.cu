@@ -560,8 +560,8 @@ __device__ __forceinline__ void warp_task(const PairParams &P, const Desc &d, in
         if (b >= d.n)
             continue;
         const size_t i = (size_t)d.body_off + b;
-        const float a[3] = {round_sum<3>(hi[0][k], lo[0][k]), round_sum<3>(hi[1][k], lo[1][k]),
-                            round_sum<3>(hi[2][k], lo[2][k])};
+        const float a[3] = {round_force(hi[0][k], lo[0][k]), round_force(hi[1][k], lo[1][k]),
+                            round_force(hi[2][k], lo[2][k])};
         P.acc[i] = make_float4(a[0], a[1], a[2], 0.f);
         if (d.flags & kMove)
 #pragma unroll
@@ -766,7 +766,7 @@ __device__ __forceinline__ void reduce_entry(const Desc &d, int blk, const float
             comp_add(hi.y, lo.y, h.y);
             lo.y += l.y;
         }
-        const float2 a = make_float2(round_sum<3>(hi.x, lo.x), round_sum<3>(hi.y, lo.y));
+        const float2 a = make_float2(round_force(hi.x, lo.x), round_force(hi.y, lo.y));
         *(float2 *)&out[comp][j] = a;
         if (kick && i < d.n)
             vel[0] = fma(widen_f32(a.x), 0.5 * d.dt, v0);

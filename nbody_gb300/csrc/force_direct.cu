@@ -117,7 +117,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                 comp_add(hi, lo, red[w][c][j]);
         }
         if (i < P.n)
-            reinterpret_cast<float *>(P.force)[4 * i + c] = round_sum<3>(hi, lo);
+            reinterpret_cast<float *>(P.force)[4 * i + c] = round_force(hi, lo);
     }
 }
 

@@ -309,7 +309,7 @@ __global__ void __launch_bounds__(3 * 32 * kGroups)
         }
 #pragma unroll
         for (int k = 0; k < kEach; k++)
-            out[comp][lane].v[k] = round_sum<3>(hi.v[k], lo.v[k]);
+            out[comp][lane].v[k] = round_force(hi.v[k], lo.v[k]);
     }
     if (!final)
         return;

@@ -275,11 +275,12 @@ __device__ __forceinline__ void comp_add(float &hi, float &lo, float t) {
 // all floats of [1, 4) weighted evenly over their logarithms, so a sum over many
 // distances of m r^-3 d is 1.65e-8 too small, whatever its rounding errors
 // average out to: a step loop's largest force error after a few thousand
-// bodies.  (hi, lo) of a sum of K-th powers, rounded without that part.
-constexpr float kRsqrtMeanError = 5.5e-9f;
-template <int K>
-__device__ __forceinline__ float round_sum(float hi, float lo) {
-    return __fadd_rn(hi, __fmaf_rn(hi, K * kRsqrtMeanError, lo));
+// bodies.  A force's (hi, lo), rounded without that part.  (Energies keep
+// theirs, 5.5e-9: they are compared to the last of 64 bits from version to
+// version.)
+constexpr float kForceMeanError = 3 * 5.5e-9f;
+__device__ __forceinline__ float round_force(float hi, float lo) {
+    return __fadd_rn(hi, __fmaf_rn(hi, kForceMeanError, lo));
 }
 
 // ---------------------------------------------------------------------------

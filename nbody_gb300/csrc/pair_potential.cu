@@ -191,7 +191,7 @@ __global__ void __launch_bounds__(256)
         comp_add(hi, lo, *piece);
     // the self pair as the loop evaluates it
     comp_add(hi, lo, -0.5f * (P.pm[i].w * rsqrt_mufu(P.eps2)));
-    phi[i].w = -2.f * round_sum<1>(hi, lo);
+    phi[i].w = -2.f * (hi + lo);
 }
 
 PotParams params(size_t n, int sms) {

@@ -1,4 +1,4 @@
-"""Forces and energies against FP64 on average: sums over many pairs keep no
+"""Forces against FP64 on average: sums over many pairs keep no
 common relative error (the hardware reciprocal square root's mean error is
 taken out), and their rounding errors stay where the kernels' comments put
 them."""
@@ -69,15 +69,3 @@ def test_ensemble(cuda, n):
     mean, rms = _errors(e.get_state(slot)[2], pm, 0.01)
     e.close()
     assert mean <= MEAN and rms <= RMS, (mean, rms)
-
-
-@pytest.mark.parametrize("n", [3001, 20000])
-def test_potential_energy(cuda, n):
-    pm, vm = nb.ic_reference(n, 9)
-    s = nb.System(n, nb.INTEGRATOR_REFERENCE, 0.01, 0.016, 0.95)
-    s.set_state(pm, vm)
-    got = s.diagnostics()["potential"]
-    s.close()
-    phi = nb.force_f64_host(pm, 0.01, np.arange(n))[1]
-    want = 0.5 * (pm[:, 3].astype(np.float64) * phi).sum()
-    assert abs(got / want - 1) <= 2e-9, got / want - 1  # 5.5e-9 with the mean error
