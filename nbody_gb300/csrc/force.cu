@@ -854,12 +854,12 @@ static int plan_force_among(size_t n, const std::vector<int> &cands, int force_n
 // Evaluate pairs once (force_pair.cu) up to kMaxPairForce bodies: 14-16 FP32
 // operations for two interactions against 23.  Microseconds a call, pairs
 // against the one-sided plan and its pack launch (back to back in a graph,
-// GB300, uniform ball): 5,000 14.8 / 18, 8,192 27 / 37, 10,007 37 / 53, 16,384
-// 81 / 110, 131,072 4,256 / 5,820; equal masses (Plummer) 100,003 2,282 /
-// 3,480, 131,072 3,884 / 5,820, 2^20 246,800 / 369,100.  Few bodies take the
+// GB300, uniform ball): 5,000 14.4 / 18, 8,192 27 / 37, 10,007 37.5 / 53, 16,384
+// 81.5 / 110, 131,072 4,267 / 5,820; equal masses (Plummer) 100,003 2,288 /
+// 3,480, 131,072 3,897 / 5,820, 2^20 247,300 / 369,100.  Few bodies take the
 // single launch of force_direct.cu instead.  Above the line a phase's pieces (12 N
 // bytes a row) take too much workspace.
-// Results of pair plans are closer to 64 bits at every size (3.7e-8 against
+// Results of pair plans are closer to 64 bits at every size (3.1e-8 against
 // 8.5e-8 at 100,003).  A plan that would take log-domain pairs refuses
 // negative masses as that plan does.
 static void use_pair_plan(ForcePlan &pl, const DeviceInfo *d, size_t max_bytes = 0) {

@@ -7,8 +7,8 @@
 // the masses involved are equal), against 23 to 24 of the one-sided
 // kernel.  ncu: FMA pipe 79 % busy; the rest are dispatch stalls of
 // three-operand instructions (six of the 16) and the other instructions' issue.
-// GB300, N = 131,072: 4,256 us with mixed masses (4.04e12 interactions/s),
-// 3,884 us with equal ones (4.42e12), against 4,830 us for 8 sources and 8
+// GB300, N = 131,072: 4,267 us with mixed masses (4.03e12 interactions/s),
+// 3,897 us with equal ones (4.41e12), against 4,830 us for 8 sources and 8
 // targets a lane with all source registers shuffled and FP64 atomics, and
 // 5,820 us one-sided.
 //
@@ -33,7 +33,8 @@
 // Narrow rows (512 bodies, 4 targets a lane) serve n below kNarrowBelow, where
 // rows of 1,024 are too few pieces of work: 12,500 bodies take 52.7 us narrow
 // and 51.2 us wide (equal masses 50.1 and 50.4), 13,000 56.8 and 54.6, 8,192
-// 26.5 and 26.6, 10,007 36.8 and 37.1.
+// 26.5 and 26.6, 10,007 36.8 and 37.1 (before pieces had remainders, which
+// cost both 0.6 to 1 us).
 //
 // Split.  The steps of all (row, set) meetings form one line, and the host
 // cuts it into equal stretches of cost, one per resident CTA, and, where there
