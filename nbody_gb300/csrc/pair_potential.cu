@@ -189,11 +189,8 @@ __global__ void __launch_bounds__(256)
 #pragma unroll 8
     for (int c = 2 * c0; c <= 2 * c1 + 1; c++, piece += PG::kRow)
         comp_add(hi, lo, *piece);
-    // the self pair as the loop evaluates it: the product unrounded (its
-    // rounding is the same for every body of one mass)
-    const float m = P.pm[i].w, r = rsqrt_mufu(P.eps2), p = __fmul_rn(m, r);
-    comp_add(hi, lo, -0.5f * p);
-    lo = __fmaf_rn(-0.5f, __fmaf_rn(m, r, -p), lo);
+    // the self pair as the loop evaluates it
+    comp_add(hi, lo, -0.5f * (P.pm[i].w * rsqrt_mufu(P.eps2)));
     phi[i].w = -2.f * (hi + lo);
 }
 

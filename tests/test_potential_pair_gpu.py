@@ -29,21 +29,3 @@ def test_potential_energy(cuda, n, equal):
     assert abs(d["potential"] - pe) <= 2e-6 * (abs(pe) + self_terms)
     assert s.diagnostics()["potential"] == d["potential"]
     s.close()
-
-
-@pytest.mark.parametrize("n", [836, 1100, 1783, 3001])
-def test_self_pairs_of_equal_masses_leave_no_common_error(cuda, n):
-    """Every body's self pair is the same product; rounded before it is taken
-    out, it shifted all bodies' sums alike.  What stays is the hardware
-    reciprocal square root's mean error, 5.5e-9, and rounding: 3e-8 a body, so
-    1e-9 of the mean of 836, 3e-9 at three of its standard deviations."""
-    err = []
-    for seed in range(4):
-        p, v, pm, _ = nb.ic_plummer(n, 90 + seed)
-        s = nb.System(n, nb.INTEGRATOR_KDK64, 1e-4, 0.002, 1.0)
-        s.set_state64(p, v, pm[:, 3].copy())
-        got = s.diagnostics()["potential"]
-        s.close()
-        phi = nb.force_f64_host(pm, 1e-4, np.arange(n))[1]
-        err.append(got / (0.5 * (pm[:, 3].astype(np.float64) * phi).sum()) - 1)
-    assert abs(np.mean(err)) <= 5.5e-9 + 3e-9, err
