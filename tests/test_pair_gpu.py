@@ -179,3 +179,16 @@ def test_partial_sums_keep_their_remainders(cuda, n):
         out = _run(fn, pm, eps2)[:512]
         assert np.all(np.abs(out[:, 0] - want) <= 2.0 ** -23 * want), out[:, 0] - want
         assert np.all(out[:, 1:] == 0)
+
+
+@pytest.mark.parametrize("n", [65537, 300001, 640003])
+def test_phases_within_a_small_workspace(cuda, n):
+    """The 32 MiB entry point: phases of at most 64 rows, down to one or two."""
+    import torch
+    _, _, pm, _ = nb.ic_plummer(n, 9)
+    t = torch.from_numpy(pm).cuda()
+    out = torch.full_like(t, float("nan"))
+    assert nb.load().nbgb_force_static(out.data_ptr(), t.data_ptr(), 1e-4, n, 0) == 0
+    torch.cuda.synchronize()
+    assert nb.last_status() == 0 and bool(torch.isfinite(out).all())
+    assert _err(out.cpu().numpy(), pm, 1e-4, np.arange(0, n, n // 300)) <= TOL_VS_FP64
