@@ -189,7 +189,9 @@ __global__ void __launch_bounds__(256)
 #pragma unroll 8
     for (int c = 2 * c0; c <= 2 * c1 + 1; c++, piece += PG::kRow)
         comp_add(hi, lo, *piece);
-    // the self pair as the loop evaluates it
+    // the self pair, its product rounded (the loop adds it unrounded): an error
+    // common to bodies of one mass, up to 5e-9 of the energy of 836 of them and
+    // below 1e-9 from a few thousand on
     comp_add(hi, lo, -0.5f * (P.pm[i].w * rsqrt_mufu(P.eps2)));
     phi[i].w = -2.f * (hi + lo);
 }
