@@ -14,6 +14,8 @@
 // from the one-sided force-and-potential kernel, 8.0 ms from here (4.3e12
 // pairs/s; the MUFU pipe alone allows 4.7e12); 65,536: 1,780 and 570 us;
 // 20,000: 288 and 119; 8,192: 128 and 117; 4,096: 108 and 106; 1,000: 104 and 97.
+// A stretch's sums carry the remainders of their rounding, which equal masses
+// have in common: without them 165,639 bodies are 7.2e-9 off, not 5.5e-9.
 // Against 64 bits both are off by 5.5e-9 of the energy at 262,144 (the MUFU
 // rsqrt's mean error), and where the self pair weighs (eps2 = 0.01, N = 20,000)
 // 2.8e-8 there and 5e-9 here.
